@@ -163,6 +163,65 @@ __device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, 
   z1 = r * sn;
 }
 
+// The pair of philox_normal2 to about 1e-10 of its radius, in FP64: what an
+// FP32 result needs to be the FP64 draw rounded once, at a quarter of the FP64
+// operations of the full-precision functions.
+//   u in (0, 1) is built from its 52 bits (exact); u = m 2^e with m in
+//   [1/sqrt 2, sqrt 2), -ln u = -(e ln 2 + 2 atanh s), s = (m - 1)/(m + 1), by
+//   the odd series to s^11 (|s| < 0.1716: what is left out is below 5e-11 of
+//   it); the quotient and the square root by one Newton step from FP32
+//   approximations (1e-14); the angle's quarter turns come off exactly and
+//   sine and cosine of the rest, within pi/4, are Taylor sums to a^11 and a^12
+//   (below 1e-11).
+template <typename Key>
+__device__ __forceinline__ void philox_normal2_mid(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, double& z0,
+                                                   double& z1) {
+  uint32_t o[4];
+  philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), key, o);
+  const double u1 = __hiloint2double((int)(0x3ff00000u | (o[0] >> 12)), (int)((o[0] << 20) | (o[1] >> 12))) -
+                    (1.0 - 0x1p-53);
+  const double u2 = __hiloint2double((int)(0x3ff00000u | (o[2] >> 12)), (int)((o[2] << 20) | (o[3] >> 12))) -
+                    (1.0 - 0x1p-53);
+  const int hi = __double2hiint(u1);
+  int e = (hi >> 20) - 1023;
+  double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(u1));
+  if (m > 1.4142135623730951) {
+    m *= 0.5;
+    e += 1;
+  }
+  const double mp = m + 1.0;
+  double q = (double)__frcp_rn((float)mp);
+  q = fma(q, fma(-mp, q, 1.0), q);
+  const double s = (m - 1.0) * q, s2 = s * s;
+  double p = 1.0 / 11.0;
+  p = fma(p, s2, 1.0 / 9.0);
+  p = fma(p, s2, 1.0 / 7.0);
+  p = fma(p, s2, 1.0 / 5.0);
+  p = fma(p, s2, 1.0 / 3.0);
+  p = fma(p, s2, 1.0);
+  const double y = -2.0 * fma((double)e, 0.69314718055994531, 2.0 * s * p);  // -2 ln u1 > 0
+  const double g = (double)rsqrtf((float)y), h = y * g;
+  const double r = fma(fma(-h, h, y), 0.5 * g, h);
+  const double w = 4.0 * u2, big = w + 6755399441055744.0;  // 1.5 2^52: rounds w to an integer
+  const int n = __double2loint(big);
+  const double a = (w - (big - 6755399441055744.0)) * 1.5707963267948966, a2 = a * a;
+  double sn = -1.0 / 39916800.0, cs = 1.0 / 479001600.0;
+  sn = fma(sn, a2, 1.0 / 362880.0);
+  cs = fma(cs, a2, -1.0 / 3628800.0);
+  sn = fma(sn, a2, -1.0 / 5040.0);
+  cs = fma(cs, a2, 1.0 / 40320.0);
+  sn = fma(sn, a2, 1.0 / 120.0);
+  cs = fma(cs, a2, -1.0 / 720.0);
+  sn = fma(sn, a2, -1.0 / 6.0);
+  cs = fma(cs, a2, 1.0 / 24.0);
+  cs = fma(cs, a2, -0.5);
+  sn = fma(sn * a2, a, a);
+  cs = fma(cs, a2, 1.0);
+  const double c = (n & 1) ? sn : cs, d = (n & 1) ? cs : sn;
+  z0 = r * (((n + 1) & 2) ? -c : c);  // cos of n quarter turns plus a
+  z1 = r * ((n & 2) ? -d : d);        // sin
+}
+
 // ---------------------------------------------------------------- Peskin
 // phi(r) of cuda/SELM_Kernel.cu:391-395 for r = |distance| (grid units)
 template <typename T> __device__ __forceinline__ T peskin4(T r) {

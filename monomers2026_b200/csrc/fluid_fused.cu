@@ -34,6 +34,7 @@
 #include <cudaTypedefs.h>
 
 #include "common.cuh"
+#include "fluid_any.h"
 #include "fluid_fused_fast.cuh"
 #include "selm_engine.h"
 #include "selm_kernels.h"
@@ -564,6 +565,8 @@ struct FusedState {
   bool ready_node[2] = {false, false};
   bool body_ready = false;  // set by the step body just issued
   bool fast = false;  // compile-time four-step kernels for this grid size
+  bool any = false;   // run-time factor kernels (fluid_any.cuh), where not fast
+  AnyPlan aplan{};
   // tuning knobs (SELM_TUNE_*): four-step split, blocks per SM of the z kernel
   int tune_split = 0;
   int tune_z_blocks = kZDefaultBlocksPerSm;
@@ -685,11 +688,14 @@ template <typename T> static int fused_alloc_t(selm_sim* s, FusedState* z) {
   z->plan = plan_for<T>(s->nx, s->ny, s->nz);
   z->fast = fast_size(s->nx) && s->nx == s->ny && s->nx == s->nz;
   if (z->fast) CUF(fast_attrs_for<T>(s->nx));
+  z->any = !z->fast && any_plan<T>(s->nx, &z->aplan);
+  if (z->any) CUF(any_attrs());
   if (z->fast && sizeof(T) == 4 && s->nx == 128 && !slab)
     z->zmap_ok = encode_zmap(&z->zmap, z->work, (long)s->ny * (s->nx / 2 + 1), s->nz, ZShape<float, 128>::WB);
   const int prec = (int)(8 * sizeof(T));
   z->tune_split = tune_default_of(s->nx, prec, SELM_TUNE_FFT_SPLIT, 0);
   z->tune_z_blocks = tune_default_of(s->nx, prec, SELM_TUNE_Z_BLOCKS, z_default_blocks(s->nx, prec));
+  if (z->fast || z->any) return SELM_OK;
   CUF(cudaFuncSetAttribute((const void*)k_xy_forward<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)z->plan.smem_xy));
   CUF(cudaFuncSetAttribute((const void*)k_xy_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -782,6 +788,19 @@ template <typename T> static int fused_fluid_t(selm_sim* s) {
     fast_dispatch<T>(s->nx, z->tune_split, z->tune_z_blocks, (const T*)z->fp, (C*)z->work, (C*)z->uhat, (T*)z->u,
                      zg, tb, z->symx, z->symy, z->symz, s->ny, s->nz, s->st, s, z->zmap_ok ? &z->zmap : nullptr);
     CUF(cudaGetLastError());
+    return SELM_OK;
+  }
+  if (z->any) {
+    const AnyPlan& A = z->aplan;
+    prof_mark(s, "xy_forward", true);
+    CUF(any_xy_forward<T>(A, (const T*)z->fp, (C*)z->work, tb, 3 * s->nz, s->st));
+    prof_mark(s, "xy_forward", false);
+    prof_mark(s, "z_update", true);
+    CUF(any_z_update<T>(A, (C*)z->work, (C*)z->uhat, zgeom_of(s, g), tb, z->symx, z->symy, z->symz, s->st));
+    prof_mark(s, "z_update", false);
+    prof_mark(s, "xy_inverse", true);
+    CUF(any_xy_inverse<T>(A, (const C*)z->work, (T*)z->u, tb, 3 * s->nz, T(1), z->d_step, s->st));
+    prof_mark(s, "xy_inverse", false);
     return SELM_OK;
   }
   prof_mark(s, "xy_forward", true);

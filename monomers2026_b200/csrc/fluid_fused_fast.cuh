@@ -190,22 +190,6 @@ __global__ void __launch_bounds__(512) k_xy_inverse_fast(const cpx<T>* __restric
 }
 
 // ---------------------------------------------------------------- z pencils + update
-struct ZGeom {
-  int ny, nxh, nx;
-  double dx, mu, rho, dt, noise_amp;
-  double idx2;  // 1/dx^2
-  int qs;       // quasi-steady: u_hat = P (F_hat + noise) / (mu lambda_h), no state
-  int stochastic, noise_mode;
-  uint64_t seed;
-  const uint64_t* step;
-  PhiloxKeys rk;  // round keys of seed
-  // a decomposed instance's block of columns: work and uhat hold the columns
-  // c0 .. c0 + ncol - 1 of the flattened (y, x) half spectrum, ncol apart
-  // from one z plane to the next (ncol == 0: all ny * nxh columns)
-  long c0 = 0, ncol = 0;
-  uint32_t* err = nullptr;  // status word (a TMA copy that timed out)
-};
-
 // reference noise draw of a half-spectrum mode (cuda/SELM_Kernel.cu:56-79); the
 // amplitude sqrt(lambda_h) comes from the symbol tables (cm = cos - 1).  The
 // FP64 forms draw FP64 normals (same stream as the plain form) and scale them
@@ -214,11 +198,12 @@ struct ZGeom {
 // FP64 normals to FP32 precision) and scales them by the whole per-mode
 // amplitude noise_amp sqrt(lambda_h) (times 1/sqrt 2 for a complex draw),
 // which is formed in FP64 and rounded to FP32 once: the noise-variance
-// prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).
-template <typename T, int N>
-__device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int i, int j, int k, double cmx,
+// prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).  MID (FP32): the
+// normals to 1e-10 instead (philox_normal2_mid), scaled in FP64 and rounded once.
+template <typename T, bool MID>
+__device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int nz, int i, int j, int k, double cmx,
                                                 double cmy, double cmz, cpx<T> out[3]) {
-  const int k1 = (k == 0) ? 0 : N - k, j1 = (j == 0) ? 0 : g.ny - j, i1 = (i == 0) ? 0 : g.nx - i;
+  const int k1 = (k == 0) ? 0 : nz - k, j1 = (j == 0) ? 0 : g.ny - j, i1 = (i == 0) ? 0 : g.nx - i;
   const bool selfc = (k1 == k && j1 == j && i1 == i);
   const uint32_t q = (uint32_t)(((long)k * g.ny + j) * g.nxh + i);
   if constexpr (sizeof(T) == 8) {
@@ -235,14 +220,130 @@ __device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, i
   } else {
     const double lam = -2.0 * (cmx + cmy + cmz) * g.idx2;
     const double amp = g.noise_amp * sqrt(fmax(lam, 0.0));
-    const float re = (float)(selfc ? amp : amp * 0.7071067811865476);
-    const float im = selfc ? 0.0f : re;
+    if constexpr (MID) {
+      const double re = selfc ? amp : amp * 0.7071067811865476, im = selfc ? 0.0 : re;
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      float z0, z1;
-      philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
-      out[d] = make_float2(z0 * re, z1 * im);
+      for (int d = 0; d < 3; d++) {
+        double z0, z1;
+        philox_normal2_mid(g.rk, q, (uint32_t)d, step, z0, z1);
+        out[d] = make_float2((float)(z0 * re), (float)(z1 * im));
+      }
+    } else {
+      const float re = (float)(selfc ? amp : amp * 0.7071067811865476);
+      const float im = selfc ? 0.0f : re;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        float z0, z1;
+        philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
+        out[d] = make_float2(z0 * re, z1 * im);
+      }
     }
+  }
+}
+
+// constants of the spectral update
+template <typename T> struct ModeConsts {
+  uint64_t step;
+  double idx2;
+  T invN, idx1, irho;
+};
+template <typename T> __device__ __forceinline__ ModeConsts<T> mode_consts(const ZGeom& g, int nz) {
+  return ModeConsts<T>{*g.step, 1.0 / (g.dx * g.dx), (T)(1.0 / ((double)g.nx * g.ny * nz)), (T)(1.0 / g.dx),
+                       (T)(1.0 / g.rho)};
+}
+
+// The spectral update of mode (i, j, k), all three components: the
+// transformed forcing at a[c astep] is replaced by the new velocity over N,
+// u_hat (component c at uh[c cplane]) by the new velocity.  MID: the
+// FP32 form's normals to 1e-10 (noise_draw_fast).
+template <typename T, bool MID = false>
+__device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>& mc, int nz, int i, int j, int k,
+                                            const double* __restrict__ symx, const double* __restrict__ symy,
+                                            const double* __restrict__ symz, cpx<T>* __restrict__ uh, long cplane,
+                                            cpx<T>* a, int astep) {
+  using C = cpx<T>;
+  const int ny = g.ny;
+  const double idx2 = mc.idx2;
+  const T idx1 = mc.idx1;
+  C X[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) X[c] = a[c * astep];
+  const double cx = symx[2 * i], sx = symx[2 * i + 1];
+  const double cy = symy[2 * j], sy = symy[2 * j + 1];
+  const double cz = symz[2 * k], sz = symz[2 * k + 1];
+  if (g.stochastic) {
+    C Xn[3];
+    noise_draw_fast<T, MID>(g, mc.step, nz, i, j, k, cx, cy, cz, Xn);
+    if (i == 0 || ((g.nx & 1) == 0 && i == g.nx / 2)) {
+      const int jc = (j == 0) ? 0 : ny - j, kc = (k == 0) ? 0 : nz - k;
+      if (jc != j || kc != k) {
+        C Xc[3];
+        noise_draw_fast<T, MID>(g, mc.step, nz, i, jc, kc, cx, symy[2 * jc], symz[2 * kc], Xc);
+        const T s = (g.noise_mode == 1 || g.qs) ? T(0.7071067811865476) : T(0.5);
+#pragma unroll
+        for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<C>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; c++) Xn[c].y = T(0);
+      }
+    }
+    if constexpr (sizeof(T) == 8) {
+      const T amp = (T)g.noise_amp;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        X[c].x += amp * Xn[c].x;
+        X[c].y += amp * Xn[c].y;
+      }
+    } else {  // FP32: the FP64 prefactor is already in the draw
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        X[c].x += Xn[c].x;
+        X[c].y += Xn[c].y;
+      }
+    }
+  }
+  C un[3];
+  if (i == 0 && j == 0 && k == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) un[c] = fftk::mk<C>(T(0), T(0));
+  } else if (g.qs) {
+    // steady Stokes: u_hat = P f_hat / (mu lambda_h), lambda_h = -L_h > 0
+    const double Lk = 2.0 * (cx + cy + cz) * idx2;
+    const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
+                    fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
+    C s = cmul(D[0], X[0]);
+    s = cadd(s, cmul(D[1], X[1]));
+    s = cadd(s, cmul(D[2], X[2]));
+    const T iL = (T)(1.0 / Lk), imuL = (T)(-1.0 / (g.mu * Lk));
+    s = fftk::mk<C>(s.x * iL, s.y * iL);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const C pf = csub(X[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
+      un[c] = fftk::mk<C>(pf.x * imuL, pf.y * imuL);
+    }
+  } else {
+    const double Lk = 2.0 * (cx + cy + cz) * idx2;
+    const T visc = (T)(1.0 + g.mu * g.dt * Lk / g.rho);
+    C us[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const C q = uh[c * cplane];
+      us[c] = fftk::mk<C>(q.x * visc + X[c].x * mc.irho, q.y * visc + X[c].y * mc.irho);
+    }
+    const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
+                    fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
+    C s = cmul(D[0], us[0]);
+    s = cadd(s, cmul(D[1], us[1]));
+    s = cadd(s, cmul(D[2], us[2]));
+    const T iL = (T)(1.0 / Lk);
+    s = fftk::mk<C>(s.x * iL, s.y * iL);
+#pragma unroll
+    for (int c = 0; c < 3; c++) un[c] = csub(us[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    if (!g.qs) uh[c * cplane] = un[c];
+    a[c * astep] = fftk::mk<C>(un[c].x * mc.invN, un[c].y * mc.invN);
   }
 }
 
@@ -373,99 +474,13 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   }
   __syncthreads();
   // spectral update: thread (w, k) for all three components, u_hat read and written in place
-  const uint64_t step = *g.step;
-  const T invN = (T)(1.0 / ((double)g.nx * ny * N));
-  const double idx2 = 1.0 / (g.dx * g.dx);
-  const T idx1 = (T)(1.0 / g.dx);
-  const T irho = (T)(1.0 / g.rho);
-  const long cplane = (long)N * plane;
+  const ModeConsts<T> mc = mode_consts<T>(g, N);
 #pragma unroll 1
   for (int u = threadIdx.x; u < WB * N; u += blockDim.x) {
     const int w = u % WB, k = u / WB;
     if (w >= wn) continue;
-    const int i = coli[w], j = colj[w];
-    const long gk = (long)k * plane + col0 + w;
-    const int pa = dpos<N1, N2>(k) * NL + w;
-    C X[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) X[c] = A[pa + c * WB];
-    const double cx = symx[2 * i], sx = symx[2 * i + 1];
-    const double cy = symy[2 * j], sy = symy[2 * j + 1];
-    const double cz = symz[2 * k], sz = symz[2 * k + 1];
-    if (g.stochastic) {
-      C Xn[3];
-      noise_draw_fast<T, N>(g, step, i, j, k, cx, cy, cz, Xn);
-      if (i == 0 || ((g.nx & 1) == 0 && i == g.nx / 2)) {
-        const int jc = (j == 0) ? 0 : ny - j, kc = (k == 0) ? 0 : N - k;
-        if (jc != j || kc != k) {
-          C Xc[3];
-          noise_draw_fast<T, N>(g, step, i, jc, kc, cx, symy[2 * jc], symz[2 * kc], Xc);
-          const T s = (g.noise_mode == 1 || g.qs) ? T(0.7071067811865476) : T(0.5);
-#pragma unroll
-          for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<C>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; c++) Xn[c].y = T(0);
-        }
-      }
-      if constexpr (sizeof(T) == 8) {
-        const T amp = (T)g.noise_amp;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          X[c].x += amp * Xn[c].x;
-          X[c].y += amp * Xn[c].y;
-        }
-      } else {  // FP32: the FP64 prefactor is already in the draw
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          X[c].x += Xn[c].x;
-          X[c].y += Xn[c].y;
-        }
-      }
-    }
-    C un[3];
-    if (i == 0 && j == 0 && k == 0) {
-#pragma unroll
-      for (int c = 0; c < 3; c++) un[c] = fftk::mk<C>(T(0), T(0));
-    } else if (g.qs) {
-      // steady Stokes: u_hat = P f_hat / (mu lambda_h), lambda_h = -L_h > 0
-      const double Lk = 2.0 * (cx + cy + cz) * idx2;
-      const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
-                      fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
-      C s = cmul(D[0], X[0]);
-      s = cadd(s, cmul(D[1], X[1]));
-      s = cadd(s, cmul(D[2], X[2]));
-      const T iL = (T)(1.0 / Lk), imuL = (T)(-1.0 / (g.mu * Lk));
-      s = fftk::mk<C>(s.x * iL, s.y * iL);
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const C pf = csub(X[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
-        un[c] = fftk::mk<C>(pf.x * imuL, pf.y * imuL);
-      }
-    } else {
-      const double Lk = 2.0 * (cx + cy + cz) * idx2;
-      const T visc = (T)(1.0 + g.mu * g.dt * Lk / g.rho);
-      C us[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const C uh = uhat[gk + c * cplane];
-        us[c] = fftk::mk<C>(uh.x * visc + X[c].x * irho, uh.y * visc + X[c].y * irho);
-      }
-      const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
-                      fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
-      C s = cmul(D[0], us[0]);
-      s = cadd(s, cmul(D[1], us[1]));
-      s = cadd(s, cmul(D[2], us[2]));
-      const T iL = (T)(1.0 / Lk);
-      s = fftk::mk<C>(s.x * iL, s.y * iL);
-#pragma unroll
-      for (int c = 0; c < 3; c++) un[c] = csub(us[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      if (!g.qs) uhat[gk + c * cplane] = un[c];
-      A[pa + c * WB] = fftk::mk<C>(un[c].x * invN, un[c].y * invN);
-    }
+    mode_update<T>(g, mc, N, coli[w], colj[w], k, symx, symy, symz, uhat + (long)k * plane + col0 + w,
+                   (long)N * plane, A + dpos<N1, N2>(k) * NL + w, WB);
   }
   __syncthreads();
   // pass B inverse in place: thread (line, k1)

@@ -35,6 +35,23 @@ template <typename T>
 cudaError_t fft3_c2r(cpx<T>* in, T* out, int nx, int ny, int nz, int ncomp, T scale, const FftTables<T>& tb,
                      cudaStream_t st);
 
+// the z kernels' geometry and constants (fused forms)
+struct ZGeom {
+  int ny, nxh, nx;
+  double dx, mu, rho, dt, noise_amp;
+  double idx2;  // 1/dx^2
+  int qs;       // quasi-steady: u_hat = P (F_hat + noise) / (mu lambda_h), no state
+  int stochastic, noise_mode;
+  uint64_t seed;
+  const uint64_t* step;
+  PhiloxKeys rk;  // round keys of seed
+  // a decomposed instance's block of columns: work and uhat hold the columns
+  // c0 .. c0 + ncol - 1 of the flattened (y, x) half spectrum, ncol apart
+  // from one z plane to the next (ncol == 0: all ny * nxh columns)
+  long c0 = 0, ncol = 0;
+  uint32_t* err = nullptr;  // status word (a TMA copy that timed out)
+};
+
 // ---- binning (counting sort of monomers into buckets, deterministic order)
 struct BinSpec {
   int mode;      // 0: grid tiles (cell = floor((x-lo)/dx), bucket = cell / tile), 1: cells of size L/nc,
