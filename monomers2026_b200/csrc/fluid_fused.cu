@@ -35,7 +35,7 @@
 
 #include "common.cuh"
 #include "fluid_any.h"
-#include "fluid_fused_fast.cuh"
+#include "fluid_fast.h"
 #include "selm_engine.h"
 #include "selm_kernels.h"
 
@@ -369,181 +369,12 @@ template <typename T> static FusedPlan plan_for(int nx, int ny, int nz) {
   return p;
 }
 
-// ---------------------------------------------------------------- fast-path dispatch
-// Row pairs per x-pass chunk of the plane kernels: the largest divisor RP of
-// N/2 (halving from N/2) at which two blocks share an SM, else the largest
-// at which one block fits.
-template <typename T, int N> constexpr size_t smem_xy_for(int rp) {
-  // plane P, x-pass rows Ax (padded by up to 16 slots in the inverse), twiddles
-  return sizeof(cpx<T>) * ((size_t)N * (N / 2 + 1) + (size_t)N * (rp + 1) + 16 + N);
-}
-template <typename T, int N> constexpr int rows_per_chunk_fast() {
-  constexpr size_t kSm = 227 * 1024;
-  int rp = N / 2;
-  while (2 * smem_xy_for<T, N>(rp) > kSm && rp % 2 == 0 && rp > 8) rp /= 2;
-  if (2 * smem_xy_for<T, N>(rp) <= kSm) return rp;
-  rp = N / 2;
-  while (smem_xy_for<T, N>(rp) > kSm && rp % 2 == 0) rp /= 2;
-  return rp;
-}
-template <typename T, int N> constexpr size_t smem_xy_fast() { return smem_xy_for<T, N>(rows_per_chunk_fast<T, N>()); }
-// grid sizes with compile-time four-step kernels
-#define SELM_FAST_SIZES(X) X(16) X(24) X(30) X(32) X(48) X(64) X(96) X(128)
-
-// Shape of a z-kernel block: WB columns, TPB threads, at least MINB blocks
-// per SM (register bound), and the default cap on blocks per SM (0: none).
-// The 128^3 FP32 kernel takes 20 columns in blocks held to three per SM's
-// registers: its 416 blocks then all fit at once, where 16 columns left a
-// second wave of 76 blocks (measured 64 us against 78 with 19 columns; 20
-// makes the block's columns a whole number of 16-byte units, which its
-// tensor copies need: kTma).
-template <typename T, int N> struct ZShape {
-  static constexpr bool kWide = sizeof(T) == 4 && N == 128;
-  static constexpr bool kTma = kWide;
-  static constexpr int WB = sizeof(T) == 8 ? 8 : (kWide ? 20 : 16);
-  static constexpr int TPB = 256;
-  static constexpr int MINB = kWide ? 3 : (sizeof(T) == 8 ? 2 : 1);
-  static constexpr int CAP = 3;
-};
-template <typename T, int N> constexpr int wb_fast() { return ZShape<T, N>::WB; }
-// Shared memory of the z kernel: what its lines need, or more when the
-// blocks per SM are capped (the request then leaves room for no more).  By
-// default at most three blocks share an SM: with the 128^3 FP32 kernel, four
-// resident blocks per SM measured slower than three.
-template <typename T, int N> constexpr size_t smem_z_need() {
-  // the TMA form places its columns at a 128-byte boundary: up to 128 bytes more
-  return sizeof(cpx<T>) * ((size_t)N * 3 * wb_fast<T, N>() + N) + (ZShape<T, N>::kTma ? 128 : 0);
-}
-constexpr int kZDefaultBlocksPerSm = 3;
-// the default cap of a size (ZShape<T, N>::CAP)
-static int z_default_blocks(int n, int precision) {
-  switch (n) {
-#define SELM_CASE(N) \
-  case N:            \
-    return precision == 32 ? ZShape<float, N>::CAP : ZShape<double, N>::CAP;
-    SELM_FAST_SIZES(SELM_CASE)
-#undef SELM_CASE
-    default:
-      return kZDefaultBlocksPerSm;
-  }
-}
-static size_t smem_z_request(size_t need, int blocks_per_sm) {
-  if (blocks_per_sm <= 0) return need;
-  const size_t cap = 228 * 1024 / (size_t)(blocks_per_sm + 1) + 1024;  // blocks_per_sm + 1 do not fit
-  return need < cap ? cap : need;
-}
-constexpr size_t kZSmemMax = 228 * 1024 / 3 + 1024;  // the largest request (two blocks per SM)
-
-template <typename T, int N, int N1> static cudaError_t fast_attrs_split() {
-  cudaError_t e;
-  constexpr int RP = rows_per_chunk_fast<T, N>();
-  if ((e = cudaFuncSetAttribute((const void*)k_xy_forward_fast<T, N, N1, RP>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_xy_fast<T, N>())))
-    return e;
-  if ((e = cudaFuncSetAttribute((const void*)k_xy_inverse_fast<T, N, N1, RP>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_xy_fast<T, N>())))
-    return e;
-  const size_t zmax = smem_z_need<T, N>() > kZSmemMax ? smem_z_need<T, N>() : kZSmemMax;
-  using Z = ZShape<T, N>;
-  if constexpr (Z::kTma) {
-    if ((e = cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zmax)))
-      return e;
-  }
-  return cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zmax);
-}
-template <typename T, int N> static cudaError_t fast_attrs() {
-  cudaError_t e = fast_attrs_split<T, N, fftk::Split<N>::N1>();
-  if (e != cudaSuccess) return e;
-  return fast_attrs_split<T, N, fftk::SplitBalanced<N>::N1>();
-}
-
-template <typename T, int N, int N1>
-static void fast_launch(const T* fp, cpx<T>* work, cpx<T>* uhat, T* u, const ZGeom& zg, const FftTables<T>& tb,
-                        const double* symx, const double* symy, const double* symz, int ny, int nz, cudaStream_t st,
-                        selm_sim* s, int z_blocks_per_sm, const CUtensorMap* zmap) {
-  constexpr int RP = rows_per_chunk_fast<T, N>();
-  using Z = ZShape<T, N>;
-  const unsigned planes = (unsigned)(3 * nz);
-  prof_mark(s, "xy_forward", true);
-  k_xy_forward_fast<T, N, N1, RP><<<planes, 512, smem_xy_fast<T, N>(), st>>>(fp, work, tb.wx_f);
-  count_launches(1);
-  prof_mark(s, "xy_forward", false);
-  prof_mark(s, "z_update", true);
-  const unsigned zb = (unsigned)z_blocks<Z::WB>(zg.nxh, ny);
-  const size_t zs = smem_z_request(smem_z_need<T, N>(), z_blocks_per_sm);
-  bool tma = false;
-  if constexpr (Z::kTma) {
-    if (zmap) {  // the block's columns by tensor copies (the map covers work)
-      k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true><<<zb, Z::TPB, zs, st>>>(work, uhat, zg, tb.wz_f, symx,
-                                                                                       symy, symz, *zmap);
-      tma = true;
-    }
-  }
-  if (!tma)
-    k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB><<<zb, Z::TPB, zs, st>>>(work, uhat, zg, tb.wz_f, symx, symy,
-                                                                              symz, CUtensorMap{});
-  count_launches(1);
-  prof_mark(s, "z_update", false);
-  prof_mark(s, "xy_inverse", true);
-  k_xy_inverse_fast<T, N, N1, RP><<<planes, 512, smem_xy_fast<T, N>(), st>>>(work, u, tb.wx_f, (uint64_t*)zg.step);
-  count_launches(1);
-  prof_mark(s, "xy_inverse", false);
-}
-
-static bool fast_size(int n) {
-  switch (n) {
-#define SELM_CASE(N) case N:
-    SELM_FAST_SIZES(SELM_CASE)
-#undef SELM_CASE
-    return true;
-    default:
-      return false;
-  }
-}
-
-template <typename T> static cudaError_t fast_attrs_for(int n) {
-  switch (n) {
-#define SELM_CASE(N) \
-  case N:            \
-    return fast_attrs<T, N>();
-    SELM_FAST_SIZES(SELM_CASE)
-#undef SELM_CASE
-    default:
-      return cudaErrorInvalidValue;
-  }
-}
-
-// split 0: the default four-step split of N; 1: the most balanced one
-template <typename T>
-static void fast_dispatch(int n, int split, int z_blocks_per_sm, const T* fp, cpx<T>* work, cpx<T>* uhat, T* u,
-                          const ZGeom& zg, const FftTables<T>& tb, const double* symx, const double* symy,
-                          const double* symz, int ny, int nz, cudaStream_t st, selm_sim* s,
-                          const CUtensorMap* zmap) {
-  switch (n) {
-#define SELM_CASE(N)                                                                                            \
-  case N:                                                                                                       \
-    if (split == 1)                                                                                             \
-      fast_launch<T, N, fftk::SplitBalanced<N>::N1>(fp, work, uhat, u, zg, tb, symx, symy, symz, ny, nz, st, s, \
-                                                    z_blocks_per_sm, zmap);                                          \
-    else                                                                                                        \
-      fast_launch<T, N, fftk::Split<N>::N1>(fp, work, uhat, u, zg, tb, symx, symy, symz, ny, nz, st, s,         \
-                                            z_blocks_per_sm, zmap);                                                  \
-    break;
-    SELM_FAST_SIZES(SELM_CASE)
-#undef SELM_CASE
-    default:
-      break;
-  }
-}
-
 }  // namespace selm
 
 using namespace selm;
 
 // grid sizes with compile-time four-step FFT kernels
-bool fused_fast_size(int n) { return fast_size(n); }
+bool fused_fast_size(int n) { return fast_tuned_size(n); }
 
 struct FusedState {
   bool fp32 = false;
@@ -686,15 +517,15 @@ template <typename T> static int fused_alloc_t(selm_sim* s, FusedState* z) {
     CUF(cudaStreamSynchronize(s->st));
   }
   z->plan = plan_for<T>(s->nx, s->ny, s->nz);
-  z->fast = fast_size(s->nx) && s->nx == s->ny && s->nx == s->nz;
+  z->fast = fast_size(s->nx, (int)(8 * sizeof(T))) && s->nx == s->ny && s->nx == s->nz;
   if (z->fast) CUF(fast_attrs_for<T>(s->nx));
   z->any = !z->fast && any_plan<T>(s->nx, &z->aplan);
   if (z->any) CUF(any_attrs());
-  if (z->fast && sizeof(T) == 4 && s->nx == 128 && !slab)
-    z->zmap_ok = encode_zmap(&z->zmap, z->work, (long)s->ny * (s->nx / 2 + 1), s->nz, ZShape<float, 128>::WB);
+  if (z->fast && sizeof(T) == 4 && s->nx == kZTmaSize && !slab)
+    z->zmap_ok = encode_zmap(&z->zmap, z->work, (long)s->ny * (s->nx / 2 + 1), s->nz, kZTmaColumns);
   const int prec = (int)(8 * sizeof(T));
   z->tune_split = tune_default_of(s->nx, prec, SELM_TUNE_FFT_SPLIT, 0);
-  z->tune_z_blocks = tune_default_of(s->nx, prec, SELM_TUNE_Z_BLOCKS, z_default_blocks(s->nx, prec));
+  z->tune_z_blocks = tune_default_of(s->nx, prec, SELM_TUNE_Z_BLOCKS, kZDefaultBlocksPerSm);
   if (z->fast || z->any) return SELM_OK;
   CUF(cudaFuncSetAttribute((const void*)k_xy_forward<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)z->plan.smem_xy));
@@ -785,9 +616,14 @@ template <typename T> static int fused_fluid_t(selm_sim* s) {
   const unsigned planes = (unsigned)(3 * s->nz);
   if (z->fast) {
     const ZGeom zg = zgeom_of(s, g);
-    fast_dispatch<T>(s->nx, z->tune_split, z->tune_z_blocks, (const T*)z->fp, (C*)z->work, (C*)z->uhat, (T*)z->u,
-                     zg, tb, z->symx, z->symy, z->symz, s->ny, s->nz, s->st, s, z->zmap_ok ? &z->zmap : nullptr);
-    CUF(cudaGetLastError());
+    const FastBufs<T> b{(const T*)z->fp, (C*)z->work, (C*)z->uhat, (T*)z->u};
+    const char* names[3] = {"xy_forward", "z_update", "xy_inverse"};
+    for (int stage = kStageXyForward; stage <= kStageXyInverse; stage++) {
+      prof_mark(s, names[stage], true);
+      CUF(fast_stage<T>(stage, s->nx, z->tune_split, z->tune_z_blocks, b, zg, tb, z->symx, z->symy, z->symz, 3 * s->nz,
+                        (long)s->ny * zg.nxh, z->zmap_ok ? &z->zmap : nullptr, s->st));
+      prof_mark(s, names[stage], false);
+    }
     return SELM_OK;
   }
   if (z->any) {
@@ -1098,50 +934,17 @@ int fused_set_field(selm_sim* s, int which, const double* in) {
 // slab's tiles, the FFTs of its planes and the z pass of its columns give
 // the same values as in a single instance; only the interpolation is summed
 // in another order (slab by slab).
-enum SlabStage { kSlabXyForward = 0, kSlabZ = 1, kSlabXyInverse = 2 };
-
-template <typename T, int N, int N1>
-static void slab_launch(int stage, selm_sim* s, const ZGeom& zg, const FftTables<T>& tb) {
-  using C = cpx<T>;
-  using Z = ZShape<T, N>;
-  constexpr int RP = rows_per_chunk_fast<T, N>();
-  FusedState* z = s->fz;
-  const unsigned planes = (unsigned)(3 * s->slab.nzl);
-  if (stage == kSlabXyForward) {
-    k_xy_forward_fast<T, N, N1, RP><<<planes, 512, smem_xy_fast<T, N>(), s->st>>>((const T*)z->fp, (C*)z->work,
-                                                                                  tb.wx_f);
-  } else if (stage == kSlabZ) {
-    const unsigned nb = (unsigned)((s->slab.ncl + Z::WB - 1) / Z::WB);
-    k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB>
-        <<<nb, Z::TPB, smem_z_request(smem_z_need<T, N>(), z->tune_z_blocks), s->st>>>(
-            (C*)s->slab.cols, (C*)z->uhat, zg, tb.wz_f, z->symx, z->symy, z->symz, CUtensorMap{});
-  } else {
-    k_xy_inverse_fast<T, N, N1, RP><<<planes, 512, smem_xy_fast<T, N>(), s->st>>>((const C*)z->work, (T*)z->u,
-                                                                                  tb.wx_f, (uint64_t*)zg.step);
-  }
-  count_launches(1);
-}
-
 template <typename T> static int slab_fluid(int stage, selm_sim* s) {
   const FftTables<T>& tb = *reinterpret_cast<const FftTables<T>*>(s->fz->fp32 ? (const void*)&s->tb32
                                                                                  : (const void*)&s->tb64);
+  FusedState* z = s->fz;
   ZGeom zg = zgeom_of(s, geom_of(s));
   zg.c0 = s->slab.c0;
   zg.ncol = s->slab.ncl;
-  switch (s->nx) {
-#define SELM_CASE(N)                                                        \
-  case N:                                                                   \
-    if (s->fz->tune_split == 1)                                             \
-      slab_launch<T, N, fftk::SplitBalanced<N>::N1>(stage, s, zg, tb);      \
-    else                                                                    \
-      slab_launch<T, N, fftk::Split<N>::N1>(stage, s, zg, tb);              \
-    break;
-    SELM_FAST_SIZES(SELM_CASE)
-#undef SELM_CASE
-    default:
-      return selm_fail(SELM_ERR_STATE, "a slab needs a grid size of the compile-time FFT kernels");
-  }
-  CUF(cudaGetLastError());
+  using C = cpx<T>;
+  const FastBufs<T> b{(const T*)z->fp, (C*)(stage == kStageZ ? s->slab.cols : z->work), (C*)z->uhat, (T*)z->u};
+  CUF(fast_stage<T>(stage, s->nx, z->tune_split, z->tune_z_blocks, b, zg, tb, z->symx, z->symy, z->symz,
+                    3 * s->slab.nzl, s->slab.ncl, nullptr, s->st));
   return SELM_OK;
 }
 
@@ -1172,7 +975,7 @@ template <typename T> static int slab_advance_t(selm_sim* s) {
   } else {
     CUF(cudaMemsetAsync(z->fp, 0, sizeof(T) * 3 * (size_t)s->slab.nzl * s->ny * s->nx, s->st));
   }
-  return slab_fluid<T>(kSlabXyForward, s);
+  return slab_fluid<T>(kStageXyForward, s);
 }
 
 static int slab_ready(selm_sim* s) {
@@ -1197,13 +1000,13 @@ extern "C" int selm_slab_advance(selm_sim* s) {
 extern "C" int selm_slab_solve(selm_sim* s) {
   int rc = slab_ready(s);
   if (rc) return rc;
-  return s->fz->fp32 ? slab_fluid<float>(kSlabZ, s) : slab_fluid<double>(kSlabZ, s);
+  return s->fz->fp32 ? slab_fluid<float>(kStageZ, s) : slab_fluid<double>(kStageZ, s);
 }
 
 extern "C" int selm_slab_finish(selm_sim* s) {
   int rc = slab_ready(s);
   if (rc) return rc;
-  rc = s->fz->fp32 ? slab_fluid<float>(kSlabXyInverse, s) : slab_fluid<double>(kSlabXyInverse, s);
+  rc = s->fz->fp32 ? slab_fluid<float>(kStageXyInverse, s) : slab_fluid<double>(kStageXyInverse, s);
   if (rc) return rc;
   fused_step_taken(s);  // step count, positions x^{n+1}
   return engine_forces(s);

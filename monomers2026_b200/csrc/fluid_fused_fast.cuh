@@ -1,14 +1,13 @@
-// fluid_fused_fast.cuh - the fused spectral kernels for compile-time grid
-// sizes N = N1*N2 (N1, N2 <= 16), built on the four-step FFT of fft_fast.cuh.
-// Same arithmetic contract as the generic kernels of fluid_fused.cu:
-//   k_xy_forward_fast : per (component, z) plane, x r2c (two rows per complex
-//                       line) and y FFT -> half spectrum [c][z][y][x];
+// fluid_fused_fast.cuh - the fused z kernel for compile-time grid sizes
+// N = N1*N2 (N1, N2 <= 16), built on the four-step FFT of fft_fast.cuh, and the
+// spectral update that the run-time sizes share.  Same arithmetic contract as
+// the generic kernels of fluid_fused.cu:
 //   k_z_update_fast   : per block of Wb consecutive (x, y) columns of the
 //                       half spectrum, three components each: z FFT, the spectral update
 //                       (viscous factor, projection, Philox noise, zero mode)
 //                       with u_hat read and written in place, inverse z FFT
-//                       with the 1/N normalisation;
-//   k_xy_inverse_fast : inverse y FFT and x c2r, writing u.
+//                       with the 1/N normalisation.
+// The plane kernels before and after it are in fluid_plane.cuh.
 // Shared-memory lines are stored line-fastest (element t of line l at
 // t*stride + l), so threads of consecutive lines touch consecutive words.
 #pragma once
@@ -16,178 +15,13 @@
 
 #include "common.cuh"
 #include "fft_fast.cuh"
+#include "selm_kernels.h"
 
 namespace selm {
 
 // ---------------------------------------------------------------- helpers
-template <int N1, int N2, typename C>
-__device__ __forceinline__ void pass_a(C* s, int stride, int l, int n2, const C* tw, bool inverse_twiddle,
-                                       int gpad = 0) {
-  // in place: reads x[N2 n1 + n2], writes Y at N2 k1 + n2; element x of line l
-  // at x stride + (x / N2) gpad + l
-  C v[N1];
-#pragma unroll
-  for (int n1 = 0; n1 < N1; n1++) v[n1] = s[(N2 * n1 + n2) * stride + n1 * gpad + l];
-  if (!inverse_twiddle) fftk::dft<N1, -1>(v);
-  else fftk::dft<N1, +1>(v);
-#pragma unroll
-  for (int k1 = 1; k1 < N1; k1++) {
-    C w = tw[n2 * k1];
-    if (inverse_twiddle) w.y = -w.y;
-    v[k1] = cmul(v[k1], w);
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < N1; k1++) s[(N2 * k1 + n2) * stride + k1 * gpad + l] = v[k1];
-}
-
 // position of natural index k after pass A + pass B (in place): N2 (k mod N1) + k / N1
 template <int N1, int N2> __device__ __forceinline__ int dpos(int k) { return N2 * (k % N1) + k / N1; }
-
-// ---------------------------------------------------------------- x/y plane kernels
-template <typename T, int N, int N1_, int RP>
-__global__ void __launch_bounds__(512) k_xy_forward_fast(const T* __restrict__ in, cpx<T>* __restrict__ out,
-                                                         const cpx<T>* __restrict__ twx) {
-  using C = cpx<T>;
-  constexpr int N1 = N1_, N2 = N / N1_;
-  static_assert(N1 * N2 == N && N1 <= 16 && N2 <= 16, "four-step split");
-  constexpr int NH = N / 2 + 1, NLP = NH, RPP = RP + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* P = reinterpret_cast<C*>(smem_raw);  // [N rows y][NLP] : element y of line m at y*NLP + m
-  C* Ax = P + N * NLP;                    // [N][RPP]        : element x of row pair lr at x*RPP + lr
-  C* tw = Ax + N * RPP;                   // W_N^t
-  const long plane = blockIdx.x;
-  const T* src = in + plane * (long)N * N;
-  C* dst = out + plane * (long)N * NH;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) tw[t] = twx[t];
-  for (int y0 = 0; y0 < N / 2; y0 += RP) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < RP * N; idx += blockDim.x) {
-      const int lr = idx / N, x = idx % N;
-      const int ya = y0 + lr;
-      Ax[x * RPP + lr] = fftk::mk<C>(src[(long)ya * N + x], src[(long)(ya + N / 2) * N + x]);
-    }
-    __syncthreads();
-    for (int u = threadIdx.x; u < RP * N2; u += blockDim.x) pass_a<N1, N2>(Ax, RPP, u % RP, u / RP, tw, false);
-    __syncthreads();
-    for (int u = threadIdx.x; u < RP * N1; u += blockDim.x) {
-      const int lr = u % RP, k1 = u / RP;
-      C v[N2];
-#pragma unroll
-      for (int n2 = 0; n2 < N2; n2++) v[n2] = Ax[(N2 * k1 + n2) * RPP + lr];
-      fftk::dft<N2, -1>(v);
-#pragma unroll
-      for (int k2 = 0; k2 < N2; k2++) Ax[(N2 * k1 + k2) * RPP + lr] = v[k2];
-    }
-    __syncthreads();
-    // unpack two real rows: A = (Z[m] + conj Z[-m])/2, B = (Z[m] - conj Z[-m])/(2i).
-    // The pair is rows y and y + N/2, so the lanes of a warp (consecutive
-    // pairs) store to consecutive rows of P, whose odd pitch NH spreads them
-    // over the banks (rows y, y + 1 put them two rows apart: 4-way conflicts)
-    for (int u = threadIdx.x; u < RP * NH; u += blockDim.x) {
-      const int lr = u % RP, m = u / RP;
-      const C z = Ax[dpos<N1, N2>(m) * RPP + lr];
-      const C zr = Ax[dpos<N1, N2>((N - m) % N) * RPP + lr];
-      const T sx = z.x + zr.x, sy = z.y - zr.y, dx_ = z.x - zr.x, dy = z.y + zr.y;
-      const int ya = y0 + lr;
-      P[ya * NLP + m] = fftk::mk<C>(sx * T(0.5), sy * T(0.5));
-      P[(ya + N / 2) * NLP + m] = fftk::mk<C>(dy * T(0.5), -dx_ * T(0.5));
-    }
-  }
-  __syncthreads();
-  for (int u = threadIdx.x; u < NH * N2; u += blockDim.x) pass_a<N1, N2>(P, NLP, u % NH, u / NH, tw, false);
-  __syncthreads();
-  for (int u = threadIdx.x; u < NH * N1; u += blockDim.x) {
-    const int m = u % NH, k1 = u / NH;
-    C v[N2];
-#pragma unroll
-    for (int n2 = 0; n2 < N2; n2++) v[n2] = P[(N2 * k1 + n2) * NLP + m];
-    fftk::dft<N2, -1>(v);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; k2++) dst[(long)(k1 + N1 * k2) * NH + m] = v[k2];
-  }
-}
-
-template <typename T, int N, int N1_, int RP>
-__global__ void __launch_bounds__(512) k_xy_inverse_fast(const cpx<T>* __restrict__ in, T* __restrict__ out,
-                                                         const cpx<T>* __restrict__ twx, uint64_t* step) {
-  using C = cpx<T>;
-  constexpr int N1 = N1_, N2 = N / N1_;
-  static_assert(N1 * N2 == N && N1 <= 16 && N2 <= 16, "four-step split");
-  constexpr int NH = N / 2 + 1, NLP = NH, RPP = RP + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* P = reinterpret_cast<C*>(smem_raw);
-  C* Ax = P + N * NLP;
-  // Ax: element x of row pair lr at x RPP + x / N2 + lr.  The slot added every
-  // N2 rows makes the x pass B, whose lanes read rows N2 apart, hit distinct
-  // banks (N2 RPP alone is a multiple of 8 words)
-  C* tw = Ax + N * RPP + N1;
-  const long plane = blockIdx.x;
-  const C* src = in + plane * (long)N * NH;
-  T* dst = out + plane * (long)N * N;
-  // the last kernel of the step's fluid solve advances the device step counter
-  // (the step's noise has been drawn; nothing later in the step reads it)
-  if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
-  for (int t = threadIdx.x; t < N; t += blockDim.x) tw[t] = twx[t];
-  for (int idx = threadIdx.x; idx < N * NH; idx += blockDim.x) {
-    const int ky = idx / NH, m = idx % NH;
-    P[ky * NLP + m] = src[idx];
-  }
-  __syncthreads();
-  // inverse y FFT, in place: row y ends at position dpos(y)
-  for (int u = threadIdx.x; u < NH * N2; u += blockDim.x) pass_a<N1, N2>(P, NLP, u % NH, u / NH, tw, true);
-  __syncthreads();
-  for (int u = threadIdx.x; u < NH * N1; u += blockDim.x) {
-    const int m = u % NH, k1 = u / NH;
-    C v[N2];
-#pragma unroll
-    for (int n2 = 0; n2 < N2; n2++) v[n2] = P[(N2 * k1 + n2) * NLP + m];
-    fftk::dft<N2, +1>(v);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; k2++) P[(N2 * k1 + k2) * NLP + m] = v[k2];
-  }
-  // x c2r, two rows per complex line; imaginary parts of m = 0 and m = N/2 drop out
-  for (int y0 = 0; y0 < N / 2; y0 += RP) {
-    __syncthreads();
-    // thread (m, row pair), m fastest: P is read along a row (consecutive
-    // words) and Ax written at the odd stride RPP (no bank conflicts); row
-    // pairs fastest would read rows 2 N2 apart, all on one bank
-    for (int idx = threadIdx.x; idx < RP * N; idx += blockDim.x) {
-      const int m = idx % N, lr = idx / N;
-      const int pa = dpos<N1, N2>(y0 + lr), pb = dpos<N1, N2>(y0 + lr + N / 2);
-      C a, b;
-      if (m < NH) {
-        a = P[pa * NLP + m];
-        b = P[pb * NLP + m];
-      } else {
-        const C ha = P[pa * NLP + (N - m)], hb = P[pb * NLP + (N - m)];
-        a = fftk::mk<C>(ha.x, -ha.y);
-        b = fftk::mk<C>(hb.x, -hb.y);
-      }
-      if (m == 0 || ((N & 1) == 0 && m == N / 2)) {
-        a.y = T(0);
-        b.y = T(0);
-      }
-      Ax[m * RPP + m / N2 + lr] = fftk::mk<C>(a.x - b.y, a.y + b.x);
-    }
-    __syncthreads();
-    for (int u = threadIdx.x; u < RP * N2; u += blockDim.x) pass_a<N1, N2>(Ax, RPP, u % RP, u / RP, tw, true, 1);
-    __syncthreads();
-    for (int u = threadIdx.x; u < RP * N1; u += blockDim.x) {
-      const int k1 = u % N1, lr = u / N1;
-      C v[N2];
-#pragma unroll
-      for (int n2 = 0; n2 < N2; n2++) v[n2] = Ax[(N2 * k1 + n2) * RPP + k1 + lr];
-      fftk::dft<N2, +1>(v);
-      const int ya = y0 + lr;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; k2++) {
-        const int xx = k1 + N1 * k2;
-        dst[(long)ya * N + xx] = v[k2].x;
-        dst[(long)(ya + N / 2) * N + xx] = v[k2].y;
-      }
-    }
-  }
-}
 
 // ---------------------------------------------------------------- z pencils + update
 // reference noise draw of a half-spectrum mode (cuda/SELM_Kernel.cu:56-79); the
@@ -399,7 +233,7 @@ template <int WB> __host__ __device__ __forceinline__ int z_blocks(int nxh, int 
 // TMA: the block's columns of work come into shared memory and go back by
 // tensor copies (tmap: work as [plane][component][column], 3-D, box WB x 3
 // x N), instead of the passes' own global loads and stores.
-template <typename T, int N, int N1_, int WB, int TPB, int MINB, bool TMA = false>
+template <typename T, int N, int N1_, int WB, int TPB, int MINB, bool TMA, bool MID>
 __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict__ work, cpx<T>* __restrict__ uhat, ZGeom g,
                                                        const cpx<T>* __restrict__ twz,
                                                        const double* __restrict__ symx,
@@ -479,7 +313,7 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   for (int u = threadIdx.x; u < WB * N; u += blockDim.x) {
     const int w = u % WB, k = u / WB;
     if (w >= wn) continue;
-    mode_update<T>(g, mc, N, coli[w], colj[w], k, symx, symy, symz, uhat + (long)k * plane + col0 + w,
+    mode_update<T, MID>(g, mc, N, coli[w], colj[w], k, symx, symy, symz, uhat + (long)k * plane + col0 + w,
                    (long)N * plane, A + dpos<N1, N2>(k) * NL + w, WB);
   }
   __syncthreads();

@@ -1,6 +1,7 @@
 """The fused forms at grid sizes of the run-time factor kernels (one, two and
-three factors, odd sizes, an odd number of row pairs), thermal noise on,
-against the oracle.  Tolerances: a step's rounding is about 1e-15 (FP64) and
+three factors, odd sizes, an odd number of row pairs) and of the compile-time
+even sizes (second factors 5 to 9, odd and even), thermal noise on, against the
+oracle.  Tolerances: a step's rounding is about 1e-15 (FP64) and
 3e-7 (FP32) of the field's maximum; 1e-11 and 1e-5 as for the other sizes."""
 import numpy as np
 import pytest
@@ -15,7 +16,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,integrator,noise", [(7, "inertial", "ref_compat"), (13, "quasi_steady", "exact"),
                                                (20, "inertial", "exact"), (25, "inertial", "ref_compat"),
                                                (33, "quasi_steady", "ref_compat"), (42, "inertial", "ref_compat"),
-                                               (125, "inertial", "exact")])
+                                               (125, "inertial", "exact"), (36, "inertial", "ref_compat"),
+                                               (50, "inertial", "exact"), (54, "quasi_steady", "ref_compat"),
+                                               (70, "inertial", "ref_compat"), (98, "inertial", "exact")])
 def test_run_time_sizes_match_the_oracle(oracle, n, integrator, noise, form, tol):
     wl = W.config(1, kT=1.0, grid=n, length=6, form=form)
     p = wl.params
