@@ -7,6 +7,8 @@
 
 #include "fft_any.cuh"
 #include "fluid_fused_fast.cuh"
+#include "fluid_plane.cuh"
+#include "fluid_plain.cuh"
 
 namespace selm {
 
@@ -83,11 +85,11 @@ __device__ __forceinline__ void xy_forward_any(const PlaneGeom& g, const cpx<T>*
   });
 }
 
-// x c2r and y inverse FFT of one plane, times scale
+// y inverse FFT and x c2r of one plane
 template <typename T>
 __device__ __forceinline__ void xy_inverse_any(const PlaneGeom& g, const cpx<T>* __restrict__ twx,
                                                const cpx<T>* __restrict__ twy, const cpx<T>* __restrict__ src,
-                                               T* __restrict__ dst, T scale, unsigned char* raw) {
+                                               T* __restrict__ dst, unsigned char* raw) {
   using C = cpx<T>;
   const PlaneSmem<T> s = plane_smem<T>(g, raw);
   const int nx = g.x.n, ny = g.y.n, nh = g.nh, rp = g.rp, rpp = rp + 1;
@@ -167,37 +169,36 @@ __device__ __forceinline__ void xy_inverse_any(const PlaneGeom& g, const cpx<T>*
         fftk::dft<R, +1>(v);
         T* d = dst + ya * nx + q;
 #pragma unroll
-        for (int j = 0; j < R; j++) d[j * nb] = v[j].x * scale;
+        for (int j = 0; j < R; j++) d[j * nb] = v[j].x;
         if (yb < ny) {
           d = dst + yb * nx + q;
 #pragma unroll
-          for (int j = 0; j < R; j++) d[j * nb] = v[j].y * scale;
+          for (int j = 0; j < R; j++) d[j * nb] = v[j].y;
         }
       }
     });
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_forward_any(const T* __restrict__ in, cpx<T>* __restrict__ out,
-                                                                         PlaneGeom g, const cpx<T>* __restrict__ twx,
+template <typename T, typename In>
+__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_forward_any(In in, cpx<T>* __restrict__ out, PlaneGeom g,
+                                                                         const cpx<T>* __restrict__ twx,
                                                                          const cpx<T>* __restrict__ twy) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long plane = blockIdx.x;
-  const T* src = in + plane * g.x.n * g.y.n;
-  xy_forward_any<T>(g, twx, twy, out + plane * g.y.n * g.nh, smem_raw,
-                    [&](int y, int x) { return src[y * g.x.n + x]; });
+  const auto src = in.plane(blockIdx.x, g.x.n);
+  xy_forward_any<T>(g, twx, twy, out + (long)blockIdx.x * g.y.n * g.nh, smem_raw,
+                    [&](int y, int x) { return src.at(y, x, g.x.n); });
 }
 
 template <typename T>
 __global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_inverse_any(const cpx<T>* __restrict__ in, T* __restrict__ out,
                                                                          PlaneGeom g, const cpx<T>* __restrict__ twx,
-                                                                         const cpx<T>* __restrict__ twy, T scale,
+                                                                         const cpx<T>* __restrict__ twy,
                                                                          uint64_t* step) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;  // as k_xy_inverse_fast
   const long plane = blockIdx.x;
-  xy_inverse_any<T>(g, twx, twy, in + plane * g.y.n * g.nh, out + plane * g.x.n * g.y.n, scale, smem_raw);
+  xy_inverse_any<T>(g, twx, twy, in + plane * g.y.n * g.nh, out + plane * g.x.n * g.y.n, smem_raw);
 }
 
 // ---------------------------------------------------------------- z pencils
@@ -308,10 +309,102 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
   z_inverse_store<T>(p, work, plane, col0, wn, tw, A);
 }
 
+// ---------------------------------------------------------------- the reference-structured form's z passes (FP64)
+// z FFT, Poisson solve and inverse z FFT of one component
+__global__ void __launch_bounds__(256, 2) k_z_poisson_any(double2* __restrict__ work, int nh, PencilGeom p,
+                                                          const double2* __restrict__ twz,
+                                                          const double* __restrict__ sym, double dxsq) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nz = p.z.n, wb = p.wb;
+  double2* A = reinterpret_cast<double2*>(smem_raw);
+  double2* tw = A + nz * p.nl;
+  int* pos = reinterpret_cast<int*>(tw + nz);
+  const long plane = (long)nz * nh, col0 = (long)blockIdx.x * wb;
+  const int wn = (int)min((long)wb, plane - col0);
+  for (int t = threadIdx.x; t < nz; t += blockDim.x) {
+    tw[t] = twz[t];
+    pos[t] = mode_pos(p.z, t);
+  }
+  __syncthreads();
+  z_load_forward<double>(p, work, plane, col0, wn, tw, A);
+  __syncthreads();
+  for (int u = threadIdx.x; u < wb * nz; u += blockDim.x) {
+    const int k = div_by(p.dwb, u), w = u - k * wb;
+    if (w >= wn) continue;
+    const int col = (int)col0 + w, j = col / nh, i = col - j * nh;
+    A[pos[k] * p.nl + w] = poisson_mode(A[pos[k] * p.nl + w], sym, i, j, k, dxsq);
+  }
+  __syncthreads();
+  z_inverse_store<double>(p, work, plane, col0, wn, tw, A);
+}
+
+// the thermal forcing's spectrum (three components), drawn and inverse transformed along z
+__global__ void __launch_bounds__(256, 2) k_z_noise_any(double2* __restrict__ work, int nh, PencilGeom p,
+                                                        const double2* __restrict__ twz, const double* __restrict__ sym,
+                                                        NoiseArgs na) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nz = p.z.n, wb = p.wb;
+  double2* A = reinterpret_cast<double2*>(smem_raw);
+  double2* tw = A + nz * p.nl;
+  int* pos = reinterpret_cast<int*>(tw + nz);
+  const long plane = (long)nz * nh, col0 = (long)blockIdx.x * wb;
+  const int wn = (int)min((long)wb, plane - col0);
+  for (int t = threadIdx.x; t < nz; t += blockDim.x) {
+    tw[t] = twz[t];
+    pos[t] = mode_pos(p.z, t);
+  }
+  __syncthreads();
+  const uint64_t step = *na.step + 1;
+#pragma unroll 1
+  for (int u = threadIdx.x; u < wb * nz; u += blockDim.x) {
+    const int k = div_by(p.dwb, u), w = u - k * wb;
+    if (w >= wn) continue;
+    const int col = (int)col0 + w, j = col / nh, i = col - j * nh;
+    noise_mode_draw(na, step, sym, nz, nh, i, j, k, A + pos[k] * p.nl + w, wb);
+  }
+  __syncthreads();
+  z_inverse_store<double>(p, work, plane, col0, wn, tw, A);
+}
+
 // ---------------------------------------------------------------- launchers
+cudaError_t any_plain_stage(int stage, const AnyPlan& p, const PlainBufs& b, const FftTables<double>& tb,
+                            cudaStream_t st) {
+  const int n = p.xy.x.n, nh = p.xy.nh;
+  // one component: its lines only, in blocks of three times the columns
+  PencilGeom one = p.z;
+  one.wb = one.nl;
+  one.dwb = one.dnl;
+  const unsigned nz1 = (unsigned)(((long)n * nh + one.wb - 1) / one.wb);
+  const unsigned nz3 = (unsigned)(((long)n * nh + p.z.wb - 1) / p.z.wb);
+  switch (stage) {
+    case kPlainForward:
+      k_xy_forward_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(DivergencePlanes{b.u, b.dx}, b.work, p.xy,
+                                                                             tb.wx_f, tb.wy_f);
+      break;
+    case kPlainPoisson:
+      k_z_poisson_any<<<nz1, 256, p.smem_z, st>>>(b.work, nh, one, tb.wz_f, b.sym, b.dx * b.dx);
+      break;
+    case kPlainInverse:
+      k_xy_inverse_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(b.work, b.p, p.xy, tb.wx_f, tb.wy_f,
+                                                                             nullptr);
+      break;
+    case kPlainNoise:
+      k_z_noise_any<<<nz3, 256, p.smem_z, st>>>(b.nwork, nh, p.z, tb.wz_f, b.sym, b.noise);
+      break;
+    default:
+      k_xy_inverse_any<double><<<(unsigned)(3 * n), p.threads_xy, p.smem_xy, st>>>(b.nwork, b.f, p.xy, tb.wx_f,
+                                                                                   tb.wy_f, (uint64_t*)b.noise.step);
+  }
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t any_attrs() {
   cudaError_t e = cudaSuccess;
-  for (const void* k : {(const void*)k_xy_forward_any<float>, (const void*)k_xy_forward_any<double>,
+  for (const void* k : {(const void*)k_xy_forward_any<float, ArrayPlanes<float>>,
+                        (const void*)k_xy_forward_any<double, ArrayPlanes<double>>,
+                        (const void*)k_xy_forward_any<double, DivergencePlanes>, (const void*)k_z_poisson_any,
+                        (const void*)k_z_noise_any,
                         (const void*)k_xy_inverse_any<float>, (const void*)k_xy_inverse_any<double>,
                         (const void*)k_z_update_any<float>, (const void*)k_z_update_any<double>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmBytes);
@@ -321,15 +414,16 @@ cudaError_t any_attrs() {
 template <typename T>
 cudaError_t any_xy_forward(const AnyPlan& p, const T* in, cpx<T>* out, const FftTables<T>& tb, int planes,
                            cudaStream_t st) {
-  k_xy_forward_any<T><<<(unsigned)planes, p.threads_xy, p.smem_xy, st>>>(in, out, p.xy, tb.wx_f, tb.wy_f);
+  k_xy_forward_any<T><<<(unsigned)planes, p.threads_xy, p.smem_xy, st>>>(ArrayPlanes<T>{in}, out, p.xy, tb.wx_f,
+                                                                         tb.wy_f);
   count_launches(1);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t any_xy_inverse(const AnyPlan& p, const cpx<T>* in, T* out, const FftTables<T>& tb, int planes, T scale,
+cudaError_t any_xy_inverse(const AnyPlan& p, const cpx<T>* in, T* out, const FftTables<T>& tb, int planes,
                            uint64_t* step, cudaStream_t st) {
-  k_xy_inverse_any<T><<<(unsigned)planes, p.threads_xy, p.smem_xy, st>>>(in, out, p.xy, tb.wx_f, tb.wy_f, scale, step);
+  k_xy_inverse_any<T><<<(unsigned)planes, p.threads_xy, p.smem_xy, st>>>(in, out, p.xy, tb.wx_f, tb.wy_f, step);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -346,7 +440,7 @@ cudaError_t any_z_update(const AnyPlan& p, cpx<T>* work, cpx<T>* uhat, const ZGe
 
 #define SELM_ANY(T)                                                                                                   \
   template cudaError_t any_xy_forward<T>(const AnyPlan&, const T*, cpx<T>*, const FftTables<T>&, int, cudaStream_t);    \
-  template cudaError_t any_xy_inverse<T>(const AnyPlan&, const cpx<T>*, T*, const FftTables<T>&, int, T, uint64_t*,      \
+  template cudaError_t any_xy_inverse<T>(const AnyPlan&, const cpx<T>*, T*, const FftTables<T>&, int, uint64_t*,         \
                                          cudaStream_t);                                                                 \
   template cudaError_t any_z_update<T>(const AnyPlan&, cpx<T>*, cpx<T>*, const ZGeom&, const FftTables<T>&,              \
                                        const double*, const double*, const double*, cudaStream_t);

@@ -166,10 +166,14 @@ template <typename T>
 cudaError_t any_xy_forward(const AnyPlan& p, const T* in, cpx<T>* out, const FftTables<T>& tb, int planes,
                            cudaStream_t st);
 template <typename T>
-cudaError_t any_xy_inverse(const AnyPlan& p, const cpx<T>* in, T* out, const FftTables<T>& tb, int planes, T scale,
+cudaError_t any_xy_inverse(const AnyPlan& p, const cpx<T>* in, T* out, const FftTables<T>& tb, int planes,
                            uint64_t* step, cudaStream_t st);
 template <typename T>
 cudaError_t any_z_update(const AnyPlan& p, cpx<T>* work, cpx<T>* uhat, const ZGeom& g, const FftTables<T>& tb,
                          const double* symx, const double* symy, const double* symz, cudaStream_t st);
+
+// a stage (PlainStage) of the reference-structured form
+cudaError_t any_plain_stage(int stage, const AnyPlan& p, const PlainBufs& b, const FftTables<double>& tb,
+                            cudaStream_t st);
 
 }  // namespace selm

@@ -46,4 +46,8 @@ cudaError_t fast_stage(int stage, int n, int split, int z_blocks_per_sm, const F
                        const FftTables<T>& tb, const double* symx, const double* symy, const double* symz, int planes,
                        long ncol, const CUtensorMap* zmap, cudaStream_t st);
 
+// the reference-structured FP64 form's stages (PlainStage), fast_size(n, 64)
+cudaError_t plain_fast_attrs(int n);
+cudaError_t plain_fast_stage(int stage, int n, const PlainBufs& b, const FftTables<double>& tb, cudaStream_t st);
+
 }  // namespace selm

@@ -84,7 +84,7 @@ template <typename T, int N> constexpr size_t smem_z_need() {
   // the TMA form places its columns at a 128-byte boundary: up to 128 bytes more
   return sizeof(cpx<T>) * ((size_t)N * 3 * ZShape<T, N>::WB + N) + (ZShape<T, N>::kTma ? 128 : 0);
 }
-static size_t smem_z_request(size_t need, int blocks_per_sm) {
+inline size_t smem_z_request(size_t need, int blocks_per_sm) {
   if (blocks_per_sm <= 0) return need;
   const size_t cap = 228 * 1024 / (size_t)(blocks_per_sm + 1) + 1024;  // blocks_per_sm + 1 do not fit
   return need < cap ? cap : need;
@@ -98,7 +98,7 @@ template <typename T, int N, int N1, int NP> struct FastKernels {
 
   static cudaError_t attrs() {
     cudaError_t e;
-    for (const void* k : {(const void*)k_xy_forward_fast<T, N, NP>, (const void*)k_xy_inverse_fast<T, N, NP>})
+    for (const void* k : {(const void*)k_xy_forward_fast<T, N, NP, ArrayPlanes<T>>, (const void*)k_xy_inverse_fast<T, N, NP>})
       if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem))) return e;
     const size_t zmax = smem_z_need<T, N>() > kZSmemMax ? smem_z_need<T, N>() : kZSmemMax;
     if constexpr (Z::kTma) {
@@ -115,7 +115,7 @@ template <typename T, int N, int N1, int NP> struct FastKernels {
                          const CUtensorMap* zmap, cudaStream_t st) {
     count_launches(1);
     if (stage == kStageXyForward) {
-      k_xy_forward_fast<T, N, NP><<<(unsigned)planes, P::TPB, P::smem, st>>>(b.fp, b.work, tb.wx_f);
+      k_xy_forward_fast<T, N, NP><<<(unsigned)planes, P::TPB, P::smem, st>>>(ArrayPlanes<T>{b.fp}, b.work, tb.wx_f);
     } else if (stage == kStageXyInverse) {
       k_xy_inverse_fast<T, N, NP><<<(unsigned)planes, P::TPB, P::smem, st>>>(b.work, b.u, tb.wx_f, (uint64_t*)zg.step);
     } else {

@@ -507,12 +507,7 @@ template <typename T> static int fused_alloc_t(selm_sim* s, FusedState* z) {
   const int nn[3] = {s->nx, s->ny, s->nz};
   double* tabs[3] = {z->symx, z->symy, z->symz};
   for (int a = 0; a < 3; a++) {
-    std::vector<double> h(2 * nn[a]);
-    for (int t = 0; t < nn[a]; t++) {
-      const double sh = sin(M_PI * t / nn[a]);
-      h[2 * t] = -2.0 * sh * sh;                 // cos(theta) - 1
-      h[2 * t + 1] = sin(2.0 * M_PI * t / nn[a]);  // sin(theta)
-    }
+    const std::vector<double> h = symbol_table(nn[a]);
     CUF(cudaMemcpyAsync(tabs[a], h.data(), sizeof(double) * 2 * nn[a], cudaMemcpyHostToDevice, s->st));
     CUF(cudaStreamSynchronize(s->st));
   }
@@ -635,7 +630,7 @@ template <typename T> static int fused_fluid_t(selm_sim* s) {
     CUF(any_z_update<T>(A, (C*)z->work, (C*)z->uhat, zgeom_of(s, g), tb, z->symx, z->symy, z->symz, s->st));
     prof_mark(s, "z_update", false);
     prof_mark(s, "xy_inverse", true);
-    CUF(any_xy_inverse<T>(A, (const C*)z->work, (T*)z->u, tb, 3 * s->nz, T(1), z->d_step, s->st));
+    CUF(any_xy_inverse<T>(A, (const C*)z->work, (T*)z->u, tb, 3 * s->nz, z->d_step, s->st));
     prof_mark(s, "xy_inverse", false);
     return SELM_OK;
   }

@@ -1,12 +1,21 @@
 // fluid_plain.cu - the reference-structured FP64 fluid step (drop-in form).
 //
-// One kernel per reference kernel of cuda/SELM_Kernel.cu, same arithmetic and
-// operation order, with the library FFTs (cuFFT D2Z/Z2D,
-// cuda/SELM_Eulerian_Period.cu:26-30,113,117,146) replaced by this project's
-// Stockham passes (x r2c/c2r, y, z) and the CUB sums
-// (cuda/SELM_Eulerian_Period.cu:121-123) by a fixed-tree reduction.
+// The steps of the reference's kernels (cuda/SELM_Kernel.cu) in its order, in
+// real space: u*, divergence, Poisson solve, gradient correction, mean removal
+// and the next thermal forcing.  The library FFTs (cuFFT D2Z/Z2D,
+// cuda/SELM_Eulerian_Period.cu:26-30,113,117,146) are this project's: plane
+// and pencil kernels (fluid_plain_fast.cuh, fluid_any.cu) that take the
+// divergence as they load and divide or draw in the z pass; sizes with prime
+// factors above 13, or whose planes do not fit in shared memory, keep
+// Stockham passes per axis.  The CUB sums
+// (cuda/SELM_Eulerian_Period.cu:121-123) are a fixed-tree reduction.
 // Layout: planar [3][Nz][Ny][Nx] doubles; half spectrum [Nz][Ny][Nx/2+1].
+#include <algorithm>
+
 #include "common.cuh"
+#include "fluid_any.h"
+#include "fluid_fast.h"
+#include "fluid_plain.cuh"
 #include "selm_kernels.h"
 
 namespace selm {
@@ -53,124 +62,95 @@ __global__ void k_div(const double* __restrict__ in, double* __restrict__ out, i
   out[n] = (a[n + i1] - a[n] + b[n + j1] - b[n] + c[n + k1] - c[n]) / dx;
 }
 
-// p_hat /= sum_d 2(cos(2 pi i_d/N_d) - 1)/dx^2, zero mode -> 0
-// (cuda/SELM_Kernel.cu:3-34)
-__global__ void k_poisson(double2* in, int Nx, int Ny, int Nz, double dx) {
+// the Poisson solve in the half spectrum (sizes of the axis passes)
+__global__ void k_poisson(double2* in, int Nx, int Ny, int Nz, const double* __restrict__ sym, double dxsq) {
   const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int Nxh = Nx / 2 + 1;
   const long N2 = (long)Nxh * Ny * Nz;
   if (n >= N2) return;
   const long Nyx = (long)Ny * Nxh;
   const int k = (int)(n / Nyx), j = (int)(n % Nyx / Nxh), i = (int)(n % Nxh);
-  const double dxsq = dx * dx;
-  const double coef =
-      (2 * (cos(2 * kPi * i / Nx) - 1) + 2 * (cos(2 * kPi * j / Ny) - 1) + 2 * (cos(2 * kPi * k / Nz) - 1)) / dxsq;
-  double2 v = in[n];
-  if (n != 0) {
-    v.x /= coef;
-    v.y /= coef;
-  } else {
-    v.x = 0.0;
-    v.y = 0.0;
-  }
-  in[n] = v;
+  in[n] = poisson_mode(in[n], sym, i, j, k, dxsq);
 }
 
-// u = u* - (p[n] - p[n - e_d])/(dx*N)   (cuda/SELM_Kernel.cu:119-152)
-__global__ void k_grad(const double* __restrict__ p, double* __restrict__ u, int Nx, int Ny, int Nz, double dx) {
-  const long N = (long)Nx * Ny * Nz;
-  const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const long Nyx = (long)Ny * Nx;
-  const long o0 = (n % Nx != 0) ? -1 : Nx - 1;
-  const long o1 = (n % Nyx / Nx != 0) ? -(long)Nx : (long)(Ny - 1) * Nx;
-  const long o2 = (n / Nyx != 0) ? -Nyx : (long)(Nz - 1) * Nyx;
-  const double pn = p[n];
-  u[n] -= (pn - p[n + o0]) / (dx * N);
-  u[N + n] -= (pn - p[n + o1]) / (dx * N);
-  u[2 * N + n] -= (pn - p[n + o2]) / (dx * N);
-}
-
-// ---------------------------------------------------------------- mean removal
-// Fixed-tree sums (deterministic): stage 1 writes one partial per block and
-// component, stage 2 reduces the partials in one block.
-constexpr int kSumThreads = 256;
-__global__ void k_sum_partial(const double* __restrict__ u, long N, double* __restrict__ partial) {
-  __shared__ double sh[kSumThreads];
-  const int d = blockIdx.y;
-  const double* ud = u + d * N;
-  double s = 0.0;
-  for (long n = (long)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (long)gridDim.x * blockDim.x) s += ud[n];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[d * gridDim.x + blockIdx.x] = sh[0];
-}
-
-__global__ void k_sum_final(const double* __restrict__ partial, int nparts, double* __restrict__ sum) {
-  __shared__ double sh[kSumThreads];
-  const int d = blockIdx.x;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += partial[d * nparts + i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = kSumThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) sum[d] = sh[0];
-}
-
-// u -= sum/N  (cuda/SELM_Kernel.cu:197-207)
-__global__ void k_subtract_mean(double* __restrict__ u, const double* __restrict__ sum, long N) {
-  const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
+// ---------------------------------------------------------------- gradient and mean removal
+// u = u* - (p[n] - p[n - e_d])/(dx*N) (cuda/SELM_Kernel.cu:119-152), with the
+// sums of the new components: one partial per block and component, in a fixed
+// order.  At 128^3 the separate passes read the velocity three times and wrote
+// it twice; the sums' own pass is gone.
+constexpr int kGradThreads = 512;
+__device__ __forceinline__ double block_total(double v, double* sh) {
 #pragma unroll
-  for (int d = 0; d < 3; d++) u[d * N + n] -= sum[d] / N;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[w] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int i = 0; i < nw; i++) s += sh[i];
+  return s;
+}
+__global__ void __launch_bounds__(kGradThreads) k_grad_sum(const double* __restrict__ p, double* __restrict__ u, int Nx,
+                                                           int Ny, int Nz, double dx, double* __restrict__ partial) {
+  __shared__ double sh[kGradThreads / 32];
+  const long N = (long)Nx * Ny * Nz, Nyx = (long)Ny * Nx;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+  for (long n = (long)blockIdx.x * kGradThreads + threadIdx.x; n < N; n += (long)gridDim.x * kGradThreads) {
+    const long row = n / Nx;
+    const int i = (int)(n - row * Nx), k = (int)(row / Ny), j = (int)(row - (long)k * Ny);
+    const long o0 = (i != 0) ? -1 : Nx - 1;
+    const long o1 = (j != 0) ? -(long)Nx : (long)(Ny - 1) * Nx;
+    const long o2 = (k != 0) ? -Nyx : (long)(Nz - 1) * Nyx;
+    const double pn = p[n];
+    const double a = u[n] - (pn - p[n + o0]) / (dx * N);
+    const double b = u[N + n] - (pn - p[n + o1]) / (dx * N);
+    const double c = u[2 * N + n] - (pn - p[n + o2]) / (dx * N);
+    u[n] = a;
+    u[N + n] = b;
+    u[2 * N + n] = c;
+    s0 += a;
+    s1 += b;
+    s2 += c;
+  }
+  s0 = block_total(s0, sh);
+  s1 = block_total(s1, sh);
+  s2 = block_total(s2, sh);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = s0;
+    partial[gridDim.x + blockIdx.x] = s1;
+    partial[2 * gridDim.x + blockIdx.x] = s2;
+  }
+}
+
+// u -= sum/N (cuda/SELM_Kernel.cu:197-207); every block adds the partials of
+// its component itself, in the same order
+__global__ void __launch_bounds__(kGradThreads) k_subtract_mean(double* __restrict__ u,
+                                                                const double* __restrict__ partial, int nparts, long N) {
+  __shared__ double sh[kGradThreads / 32];
+  const int d = blockIdx.y;
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += kGradThreads) s += partial[d * nparts + i];
+  const double mean = block_total(s, sh) / N;
+  double* ud = u + d * N;
+  for (long n = (long)blockIdx.x * kGradThreads + threadIdx.x; n < N; n += (long)gridDim.x * kGradThreads) ud[n] -= mean;
 }
 
 // ---------------------------------------------------------------- thermal noise
-// Half-spectrum draw of cuda/SELM_Kernel.cu:37-85 with Philox instead of a
-// per-mode XORWOW state: amplitude sqrt(lambda_h)/sqrt(2) on re and im, or
-// (sqrt(lambda_h), 0) on self-conjugate modes.  noise_mode 1 (exact) scales
-// the non-self-conjugate modes of the x=0 / x=Nx/2 planes by sqrt(2) so the
-// Hermitian average the c2r takes keeps the full variance.
-__global__ void k_noise_generate(double2* __restrict__ out, int Nx, int Ny, int Nz, double dx, uint64_t seed,
-                                 uint64_t step, int noise_mode) {
+// the forcing's half spectrum (sizes of the axis passes)
+__global__ void k_noise_generate(double2* __restrict__ out, int Nx, int Ny, int Nz, const double* __restrict__ sym,
+                                 NoiseArgs na) {
   const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int Nxh = Nx / 2 + 1;
   const long N2 = (long)Nxh * Ny * Nz;
   if (n >= N2) return;
   const long Nyx = (long)Ny * Nxh;
   const int k = (int)(n / Nyx), j = (int)(n % Nyx / Nxh), i = (int)(n % Nxh);
-  const double dxsq = dx * dx;
-  double coef =
-      (2 * (1 - cos(2 * kPi * i / Nx)) + 2 * (1 - cos(2 * kPi * j / Ny)) + 2 * (1 - cos(2 * kPi * k / Nz))) / dxsq;
-  coef = sqrt(coef);
-  const int k1 = (Nz - k) % Nz, j1 = (Ny - j) % Ny, i1 = (Nx - i) % Nx;
-  const bool selfc = !(k1 != k || j1 != j || i1 != i);
-  double re, im;
-  if (!selfc) {
-    re = coef / sqrt(2.0);
-    im = re;
-  } else {
-    re = coef;
-    im = 0.0;
-  }
-  if (noise_mode == 1 && !selfc && (i == 0 || ((Nx & 1) == 0 && i == Nx / 2))) {
-    re *= sqrt(2.0);
-    im *= sqrt(2.0);
-  }
+  double2 z[3];
+  noise_mode_draw(na, *na.step + 1, sym, Nx, Nxh, i, j, k, z, 1);
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    double z0, z1;
-    philox_normal2(seed, (uint32_t)n, (uint32_t)d, step, z0, z1);
-    out[d * N2 + n] = make_double2(z0 * re, z1 * im);
-  }
+  for (int d = 0; d < 3; d++) out[d * N2 + n] = z[d];
 }
+__global__ void k_step_advance(uint64_t* step) { *step += 1; }
 
 // ---------------------------------------------------------------- FFT passes
 // Complex FFT along a strided axis.  Line (o, i), i < ni: element t at
@@ -350,49 +330,61 @@ template cudaError_t fft3_r2c<float>(const float*, float2*, int, int, int, int, 
 template cudaError_t fft3_c2r<float>(float2*, float*, int, int, int, int, float, const FftTables<float>&,
                                      cudaStream_t);
 
+static cudaError_t plain_stage(int stage, const PlainPlan& pp, const PlainBufs& b, int n, const FftTables<double>& tb,
+                               cudaStream_t st) {
+  return pp.fast ? plain_fast_stage(stage, n, b, tb, st) : any_plain_stage(stage, *pp.any, b, tb, st);
+}
+
 // One fluid step of the reference structure (cuda/SELM_Eulerian_Period.cu:96-126):
 // u_new = P(u_old + (mu dt lap u_old + f)/rho) - mean.
-cudaError_t plain_fluid_run(const double* u_old, double* u_new, const double* f, double* p, double2* work,
-                            double* partial, double* sum, int nx, int ny, int nz, double dx, double dt, double mu,
-                            double rho, const FftTables<double>& tb, cudaStream_t st) {
+cudaError_t plain_fluid_run(const double* u_old, double* u_new, const PlainPlan& pp, const PlainBufs& b,
+                            double* partial, int nx, int ny, int nz, double dt, double mu, double rho,
+                            const FftTables<double>& tb, cudaStream_t st) {
   const long N = (long)nx * ny * nz;
   const long N2 = (long)(nx / 2 + 1) * ny * nz;
   const int bs = 128;
   const unsigned g1 = (unsigned)((N + bs - 1) / bs), g2 = (unsigned)((N2 + bs - 1) / bs);
-  k_u2uAsterisk<<<g1, bs, 0, st>>>(u_old, f, u_new, dx, dt, mu, rho, nx, ny, nz);
+  k_u2uAsterisk<<<g1, bs, 0, st>>>(u_old, b.f, u_new, b.dx, dt, mu, rho, nx, ny, nz);
   count_launches(1);
-  k_div<<<g1, bs, 0, st>>>(u_new, p, nx, ny, nz, dx);
-  count_launches(1);
-  cudaError_t e = fft3_r2c<double>(p, work, nx, ny, nz, 1, tb, st);
-  if (e != cudaSuccess) return e;
-  k_poisson<<<g2, bs, 0, st>>>(work, nx, ny, nz, dx);
-  count_launches(1);
-  e = fft3_c2r<double>(work, p, nx, ny, nz, 1, 1.0, tb, st);
-  if (e != cudaSuccess) return e;
-  k_grad<<<g1, bs, 0, st>>>(p, u_new, nx, ny, nz, dx);
-  count_launches(1);
-  const int nparts = kSumParts;
-  k_sum_partial<<<dim3(nparts, 3), kSumThreads, 0, st>>>(u_new, N, partial);
-  count_launches(1);
-  k_sum_final<<<3, kSumThreads, 0, st>>>(partial, nparts, sum);
-  count_launches(1);
-  k_subtract_mean<<<g1, bs, 0, st>>>(u_new, sum, N);
-  count_launches(1);
+  cudaError_t e = cudaGetLastError();
+  if (pp.fast || pp.any) {
+    for (int stage : {kPlainForward, kPlainPoisson, kPlainInverse})
+      if (e == cudaSuccess) e = plain_stage(stage, pp, b, nx, tb, st);
+    if (e != cudaSuccess) return e;
+  } else {
+    k_div<<<g1, bs, 0, st>>>(u_new, b.p, nx, ny, nz, b.dx);
+    count_launches(1);
+    if ((e = fft3_r2c<double>(b.p, b.work, nx, ny, nz, 1, tb, st)) != cudaSuccess) return e;
+    k_poisson<<<g2, bs, 0, st>>>(b.work, nx, ny, nz, b.sym, b.dx * b.dx);
+    count_launches(1);
+    if ((e = fft3_c2r<double>(b.work, b.p, nx, ny, nz, 1, 1.0, tb, st)) != cudaSuccess) return e;
+  }
+  const unsigned parts = (unsigned)std::min<long>(kSumParts, (N + kGradThreads - 1) / kGradThreads);
+  k_grad_sum<<<parts, kGradThreads, 0, st>>>(b.p, u_new, nx, ny, nz, b.dx, partial);
+  k_subtract_mean<<<dim3(parts, 3), kGradThreads, 0, st>>>(u_new, partial, (int)parts, N);
+  count_launches(2);
   return cudaGetLastError();
 }
 
-// Thermal forcing of cuda/SELM_Eulerian_Period.cu:128-153:
+// Thermal forcing of cuda/SELM_Eulerian_Period.cu:128-153 for the step after
+// the device counter's, which it advances:
 // f = sqrt(2 kB T dt mu / N) * c2r(noise half spectrum), or f = 0.
-cudaError_t plain_compute_f(double* f, double2* work, int nx, int ny, int nz, double dx, double kB, double T,
-                            double dt, double mu, bool stochastic, uint64_t seed, uint64_t step, int noise_mode,
-                            const FftTables<double>& tb, cudaStream_t st) {
+cudaError_t plain_forcing(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                          const FftTables<double>& tb, cudaStream_t st) {
   const long N = (long)nx * ny * nz;
-  if (!stochastic) return cudaMemsetAsync(f, 0, sizeof(double) * 3 * N, st);
+  if (!stochastic) return cudaMemsetAsync(b.f, 0, sizeof(double) * 3 * N, st);
+  if (pp.fast || pp.any) {
+    const cudaError_t e = plain_stage(kPlainNoise, pp, b, nx, tb, st);
+    return e ? e : plain_stage(kPlainNoiseInverse, pp, b, nx, tb, st);
+  }
   const long N2 = (long)(nx / 2 + 1) * ny * nz;
-  const double scale = sqrt(2 * kB * T * dt * mu / N);
-  k_noise_generate<<<(unsigned)((N2 + 127) / 128), 128, 0, st>>>(work, nx, ny, nz, dx, seed, step, noise_mode);
+  k_noise_generate<<<(unsigned)((N2 + 127) / 128), 128, 0, st>>>(b.nwork, nx, ny, nz, b.sym, b.noise);
   count_launches(1);
-  return fft3_c2r<double>(work, f, nx, ny, nz, 3, scale, tb, st);
+  cudaError_t e = fft3_c2r<double>(b.nwork, b.f, nx, ny, nz, 3, 1.0, tb, st);
+  if (e != cudaSuccess) return e;
+  k_step_advance<<<1, 1, 0, st>>>((uint64_t*)b.noise.step);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 }  // namespace selm

@@ -72,9 +72,38 @@ template <int R, int S, typename C> __device__ __forceinline__ void twiddle_row(
   }
 }
 
-template <typename T, int N, int N1>
+// What the forward kernel transforms: the planes of an array, or the
+// divergence of a velocity (forward differences, cuda/SELM_Kernel.cu:100-116).
+template <typename T> struct ArrayPlanes {
+  const T* __restrict__ in;
+  struct Plane {
+    const T* src;
+    __device__ __forceinline__ T at(int y, int x, int n) const { return src[y * n + x]; }
+  };
+  __device__ __forceinline__ Plane plane(int p, int n) const { return Plane{in + (long)p * (n * n)}; }
+};
+struct DivergencePlanes {
+  const double* __restrict__ u;
+  double dx;
+  struct Plane {
+    const double *a, *b, *c, *cn;  // the three components, the third's next plane
+    double dx;
+    __device__ __forceinline__ double at(int y, int x, int n) const {
+      const int q = y * n + x;
+      const int i1 = (x != n - 1) ? 1 : -x, j1 = (y != n - 1) ? n : -y * n;
+      return (a[q + i1] - a[q] + b[q + j1] - b[q] + cn[q] - c[q]) / dx;
+    }
+  };
+  __device__ __forceinline__ Plane plane(int z, int n) const {
+    const long pl = (long)n * n, N = pl * n;
+    const double* c = u + 2 * N + z * pl;
+    return Plane{u + z * pl, u + N + z * pl, c, (z != n - 1) ? c + pl : u + 2 * N, dx};
+  }
+};
+
+template <typename T, int N, int N1, typename In>
 __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1>::NB)
-    k_xy_forward_fast(const T* __restrict__ in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ twx) {
+    k_xy_forward_fast(In in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ twx) {
   using C = cpx<T>;
   using S = PlaneShape<T, N, N1>;
   constexpr int N2 = S::N2, NH = S::NH, HP = S::HP, G = S::GF, PW = S::PW;
@@ -82,17 +111,17 @@ __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* P = reinterpret_cast<C*>(smem_raw);  // [HP][PW]
   C* tw = P + HP * PW;
-  const T* src = in + (long)blockIdx.x * (N * N);
+  const auto src = in.plane(blockIdx.x, N);
   C* dst = out + (long)blockIdx.x * (N * NH);
   for (int t = threadIdx.x; t < N; t += S::TPB) tw[t] = twx[t];
   __syncthreads();
   // x, first factor: thread (row pair, n2), n2 fastest (runs of N2 values of a row)
   for (int u = threadIdx.x; u < HP * N2; u += S::TPB) {
     const int lr = u / N2, n2 = u % N2;
-    const T* a = src + lr * N + n2;
     C v[N1];
 #pragma unroll
-    for (int n1 = 0; n1 < N1; n1++) v[n1] = fftk::mk<C>(a[N2 * n1], a[HP * N + N2 * n1]);
+    for (int n1 = 0; n1 < N1; n1++)
+      v[n1] = fftk::mk<C>(src.at(lr, N2 * n1 + n2, N), src.at(lr + HP, N2 * n1 + n2, N));
     fftk::dft<N1, -1>(v);
     if (N2 > 1) twiddle_row<N1, -1>(v, tw, n2);
     C* p = P + lr * PW + n2;

@@ -17,6 +17,8 @@
 #include <vector>
 
 #include "../../include/selm_b200.h"
+#include "fluid_any.h"
+#include "fluid_fast.h"
 #include "selm_engine.h"
 #include "selm_kernels.h"
 
@@ -316,6 +318,17 @@ extern "C" int selm_slab_layout(const selm_sim* s, int* z0, int* nzl, long long*
   return SELM_OK;
 }
 
+// (cos - 1, sin) of 2 pi t / n, t < n
+std::vector<double> symbol_table(int n) {
+  std::vector<double> h(2 * (size_t)n);
+  for (int t = 0; t < n; t++) {
+    const double sh = sin(M_PI * t / n);
+    h[2 * t] = -2.0 * sh * sh;
+    h[2 * t + 1] = sin(2.0 * M_PI * t / n);
+  }
+  return h;
+}
+
 int engine_allocate_grid(selm_sim* s) {
   int rc;
   const long N = s->N, N2 = s->N2;
@@ -331,7 +344,23 @@ int engine_allocate_grid(selm_sim* s) {
     if ((rc = dalloc(s, &s->p64, N))) return rc;
     if ((rc = dalloc(s, &s->work64, 6 * N2))) return rc;  // 3 components x N2 complex
     if ((rc = dalloc(s, &s->partial, 3 * kSumParts))) return rc;
-    if ((rc = dalloc(s, &s->sum, 3))) return rc;
+    if ((rc = dalloc(s, &s->sym64, 2 * s->nx))) return rc;
+    if ((rc = dalloc(s, &s->step64, 1))) return rc;
+    {
+      const std::vector<double> h = symbol_table(s->nx);
+      CU(cudaMemcpyAsync(s->sym64, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s->st));
+      CU(cudaStreamSynchronize(s->st));
+    }
+    s->plan64.fast = fast_size(s->nx, 64);
+    if (s->plan64.fast) {
+      CU(plain_fast_attrs(s->nx));
+    } else {
+      s->any64 = new AnyPlan();
+      if (any_plan<double>(s->nx, s->any64)) {
+        s->plan64.any = s->any64;
+        CU(any_attrs());
+      }
+    }
     CU(cudaMemsetAsync(s->u64[0], 0, sizeof(double) * 3 * N, s->st));
     CU(cudaMemsetAsync(s->u64[1], 0, sizeof(double) * 3 * N, s->st));
     CU(cudaMemsetAsync(s->fg64, 0, sizeof(double) * 3 * N, s->st));
@@ -841,18 +870,36 @@ static CouplingArgs coupling_args(selm_sim* s, uint64_t step) {
   return a;
 }
 
-static int plain_compute_f_step(selm_sim* s, uint64_t noise_step) {
+static PlainBufs plain_bufs(selm_sim* s, double* u_new) {
+  PlainBufs b{};
+  b.u = u_new;
+  b.p = s->p64;
+  b.f = s->fg64;
+  b.work = (double2*)s->work64;
+  b.nwork = (double2*)s->work64;
+  b.sym = s->sym64;
+  b.dx = s->dx;
+  b.noise.seed = s->prm.seed;
+  b.noise.rk = philox_keys(s->prm.seed);
+  b.noise.step = s->step64;
+  b.noise.scale = sqrt(2 * s->prm.KB * s->prm.T * s->prm.dt * s->prm.mu / s->N);  // cuda/SELM_Eulerian_Period.cu:141
+  b.noise.dxsq = s->dx * s->dx;
+  b.noise.noise_mode = s->prm.noise_mode;
+  return b;
+}
+
+// the forcing of the step after the device counter's, which it advances
+static int plain_forcing_step(selm_sim* s) {
   prof_mark(s, "noise", true);
-  CU(plain_compute_f(s->fg64, (double2*)s->work64, s->nx, s->ny, s->nz, s->dx, s->prm.KB, s->prm.T, s->prm.dt,
-                     s->prm.mu, s->prm.flag_stochastic != 0, s->prm.seed, noise_step, s->prm.noise_mode, s->tb64,
-                     s->st));
+  CU(plain_forcing(s->plan64, plain_bufs(s, nullptr), s->nx, s->ny, s->nz, s->prm.flag_stochastic != 0, s->tb64, s->st));
   prof_mark(s, "noise", false);
   return SELM_OK;
 }
 
 static int plain_step(selm_sim* s) {
   const uint64_t n = ++s->step;
-  const CouplingArgs a = coupling_args(s, n);
+  CouplingArgs a = coupling_args(s, n);
+  a.step_ptr = s->step64;
   double* xo = s->x[s->cx];
   double* xn = s->x[s->cx ^ 1];
   if (s->M > 0) {
@@ -867,11 +914,11 @@ static int plain_step(selm_sim* s) {
     s->cx ^= 1;
   }
   prof_mark(s, "fluid", true);
-  CU(plain_fluid_run(s->u64[s->cu], s->u64[s->cu ^ 1], s->fg64, s->p64, (double2*)s->work64, s->partial, s->sum,
-                     s->nx, s->ny, s->nz, s->dx, s->prm.dt, s->prm.mu, s->prm.rho, s->tb64, s->st));
+  CU(plain_fluid_run(s->u64[s->cu], s->u64[s->cu ^ 1], s->plan64, plain_bufs(s, s->u64[s->cu ^ 1]), s->partial, s->nx,
+                     s->ny, s->nz, s->prm.dt, s->prm.mu, s->prm.rho, s->tb64, s->st));
   prof_mark(s, "fluid", false);
   s->cu ^= 1;
-  int rc = plain_compute_f_step(s, n + 1);
+  int rc = plain_forcing_step(s);
   if (rc) return rc;
   return engine_forces(s);
 }
@@ -886,7 +933,8 @@ extern "C" int selm_initial(selm_sim* s) {
     CU(cudaMemsetAsync(s->u64[0], 0, sizeof(double) * 3 * s->N, s->st));
     CU(cudaMemsetAsync(s->u64[1], 0, sizeof(double) * 3 * s->N, s->st));
     s->cu = 0;
-    rc = plain_compute_f_step(s, 1);
+    CU(cudaMemsetAsync(s->step64, 0, sizeof(uint64_t), s->st));
+    rc = plain_forcing_step(s);
   } else {
     rc = fused_initial(s);
   }
@@ -921,6 +969,7 @@ extern "C" int selm_destroy(selm_sim* s) {
   if (s->st_copy) cudaStreamSynchronize(s->st_copy);
   analysis_detach_all(s);
   fused_release(s);
+  delete s->any64;
   free_all(s->allocs);
   sim_free_all(s);
   if (s->hstage_cnt) cudaFreeHost(s->hstage_cnt);

@@ -56,7 +56,11 @@ struct selm_sim {
   cudaEvent_t ev_committed = nullptr;  // committed (simulation stream): staging free again
   // plain-form grid (Eulerian::d_u[2], d_f, d_p, cuda/SELM_Eulerian.cuh:12-20)
   double* u64[2] = {nullptr, nullptr};
-  double *fg64 = nullptr, *p64 = nullptr, *work64 = nullptr, *partial = nullptr, *sum = nullptr;
+  double *fg64 = nullptr, *p64 = nullptr, *work64 = nullptr, *partial = nullptr;
+  double* sym64 = nullptr;      // (cos - 1, sin) of 2 pi t / n
+  uint64_t* step64 = nullptr;   // device step counter (the step being taken)
+  selm::AnyPlan* any64 = nullptr;  // run-time factor kernels' plan, where plan64.any points at it
+  selm::PlainPlan plan64{};
   int cu = 0;
   uint32_t* err = nullptr;
   selm::FftTables<double> tb64{};
@@ -99,6 +103,7 @@ int selm_fail(int code, const std::string& msg);
 int sim_alloc(selm_sim* s, void** p, size_t bytes);
 void prof_mark(selm_sim* s, const char* name, bool begin);
 int engine_allocate_grid(selm_sim* s);
+std::vector<double> symbol_table(int n);
 int engine_forces(selm_sim* s);
 // the conservative forces at positions x, issued on stream st (device force field only)
 int engine_forces_on(selm_sim* s, double* x, cudaStream_t st);

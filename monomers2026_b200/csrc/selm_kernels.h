@@ -13,7 +13,7 @@ void count_launches(unsigned n);
 void uncount_launches(unsigned long long n);  // launches recorded into a graph capture, not run
 unsigned long long launches_total();
 
-constexpr int kSumParts = 296;  // fixed number of partial sums (2 per SM)
+constexpr int kSumParts = 592;  // at most so many partial sums (4 blocks of 512 threads per SM)
 
 // Twiddle tables of the three axes, forward (sign -1) and backward (+1).
 template <typename T> struct FftTables {
@@ -22,12 +22,39 @@ template <typename T> struct FftTables {
 };
 
 // ---- fluid, reference structure (FP64)
-cudaError_t plain_fluid_run(const double* u_old, double* u_new, const double* f, double* p, double2* work,
-                            double* partial, double* sum, int nx, int ny, int nz, double dx, double dt, double mu,
-                            double rho, const FftTables<double>& tb, cudaStream_t st);
-cudaError_t plain_compute_f(double* f, double2* work, int nx, int ny, int nz, double dx, double kB, double T,
-                            double dt, double mu, bool stochastic, uint64_t seed, uint64_t step, int noise_mode,
+// The thermal forcing's draw: amplitude per mode scale sqrt(lambda_h), the step
+// after the one the device counter holds.
+struct NoiseArgs {
+  uint64_t seed;
+  PhiloxKeys rk;
+  const uint64_t* step;
+  double scale, dxsq;
+  int noise_mode;
+};
+// The spectral stages of the step: divergence and xy FFT, Poisson solve along
+// z, back to the pressure; the forcing drawn along z, back to the grid (which
+// advances the step counter: no later kernel of the step reads it).
+enum PlainStage { kPlainForward = 0, kPlainPoisson, kPlainInverse, kPlainNoise, kPlainNoiseInverse };
+struct PlainBufs {
+  const double* u;         // u*
+  double *p, *f;           // pressure, forcing
+  double2 *work, *nwork;   // half spectra of the pressure and of the forcing's three components
+  const double* sym;       // (cos - 1, sin) of 2 pi t / n, t < n
+  double dx;
+  NoiseArgs noise;
+};
+struct AnyPlan;
+// how a grid size's spectral stages run: compile-time kernels, run-time
+// factors (any), or, with neither, FFT passes per axis
+struct PlainPlan {
+  bool fast = false;
+  const AnyPlan* any = nullptr;
+};
+cudaError_t plain_fluid_run(const double* u_old, double* u_new, const PlainPlan& pp, const PlainBufs& b,
+                            double* partial, int nx, int ny, int nz, double dt, double mu, double rho,
                             const FftTables<double>& tb, cudaStream_t st);
+cudaError_t plain_forcing(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                          const FftTables<double>& tb, cudaStream_t st);
 template <typename T>
 cudaError_t fft3_r2c(const T* in, cpx<T>* out, int nx, int ny, int nz, int ncomp, const FftTables<T>& tb,
                      cudaStream_t st);

@@ -1,4 +1,4 @@
-"""The fused forms at grid sizes of the run-time factor kernels (one, two and
+"""The three forms at grid sizes of the run-time factor kernels (one, two and
 three factors, odd sizes, an odd number of row pairs) and of the compile-time
 even sizes (second factors 5 to 9, odd and even), thermal noise on, against the
 oracle.  Tolerances: a step's rounding is about 1e-15 (FP64) and
@@ -12,7 +12,7 @@ from monomers2026_b200.selm import Selm
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("form,tol", [("fused64", 1e-11), ("fused32", 1e-5)])
+@pytest.mark.parametrize("form,tol", [("fused64", 1e-11), ("fused32", 1e-5), ("plain64", 1e-11)])
 @pytest.mark.parametrize("n,integrator,noise", [(7, "inertial", "ref_compat"), (13, "quasi_steady", "exact"),
                                                (20, "inertial", "exact"), (25, "inertial", "ref_compat"),
                                                (33, "quasi_steady", "ref_compat"), (42, "inertial", "ref_compat"),
@@ -20,6 +20,8 @@ pytestmark = pytest.mark.gpu
                                                (50, "inertial", "exact"), (54, "quasi_steady", "ref_compat"),
                                                (70, "inertial", "ref_compat"), (98, "inertial", "exact")])
 def test_run_time_sizes_match_the_oracle(oracle, n, integrator, noise, form, tol):
+    if form == "plain64" and integrator != "inertial":
+        pytest.skip("the plain form has the inertial integrator only")
     wl = W.config(1, kT=1.0, grid=n, length=6, form=form)
     p = wl.params
     p.integrator, p.noise_mode = integrator, noise
