@@ -337,25 +337,28 @@ static cudaError_t plain_stage(int stage, const PlainPlan& pp, const PlainBufs& 
 
 // One fluid step of the reference structure (cuda/SELM_Eulerian_Period.cu:96-126):
 // u_new = P(u_old + (mu dt lap u_old + f)/rho) - mean.
-cudaError_t plain_fluid_run(const double* u_old, double* u_new, const PlainPlan& pp, const PlainBufs& b,
-                            double* partial, int nx, int ny, int nz, double dt, double mu, double rho,
-                            const FftTables<double>& tb, cudaStream_t st) {
+cudaError_t plain_ustar(const double* u_old, double* u_new, const PlainBufs& b, int nx, int ny, int nz, double dt,
+                        double mu, double rho, cudaStream_t st) {
+  const long N = (long)nx * ny * nz;
+  k_u2uAsterisk<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(u_old, b.f, u_new, b.dx, dt, mu, rho, nx, ny, nz);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t plain_project(double* u_new, const PlainPlan& pp, const PlainBufs& b, double* partial, int nx, int ny,
+                          int nz, const FftTables<double>& tb, cudaStream_t st) {
   const long N = (long)nx * ny * nz;
   const long N2 = (long)(nx / 2 + 1) * ny * nz;
-  const int bs = 128;
-  const unsigned g1 = (unsigned)((N + bs - 1) / bs), g2 = (unsigned)((N2 + bs - 1) / bs);
-  k_u2uAsterisk<<<g1, bs, 0, st>>>(u_old, b.f, u_new, b.dx, dt, mu, rho, nx, ny, nz);
-  count_launches(1);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = cudaSuccess;
   if (pp.fast || pp.any) {
     for (int stage : {kPlainForward, kPlainPoisson, kPlainInverse})
       if (e == cudaSuccess) e = plain_stage(stage, pp, b, nx, tb, st);
     if (e != cudaSuccess) return e;
   } else {
-    k_div<<<g1, bs, 0, st>>>(u_new, b.p, nx, ny, nz, b.dx);
+    k_div<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(u_new, b.p, nx, ny, nz, b.dx);
     count_launches(1);
     if ((e = fft3_r2c<double>(b.p, b.work, nx, ny, nz, 1, tb, st)) != cudaSuccess) return e;
-    k_poisson<<<g2, bs, 0, st>>>(b.work, nx, ny, nz, b.sym, b.dx * b.dx);
+    k_poisson<<<(unsigned)((N2 + 127) / 128), 128, 0, st>>>(b.work, nx, ny, nz, b.sym, b.dx * b.dx);
     count_launches(1);
     if ((e = fft3_c2r<double>(b.work, b.p, nx, ny, nz, 1, 1.0, tb, st)) != cudaSuccess) return e;
   }
@@ -367,20 +370,23 @@ cudaError_t plain_fluid_run(const double* u_old, double* u_new, const PlainPlan&
 }
 
 // Thermal forcing of cuda/SELM_Eulerian_Period.cu:128-153 for the step after
-// the device counter's, which it advances:
+// the device counter's, which the second part advances:
 // f = sqrt(2 kB T dt mu / N) * c2r(noise half spectrum), or f = 0.
-cudaError_t plain_forcing(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
-                          const FftTables<double>& tb, cudaStream_t st) {
-  const long N = (long)nx * ny * nz;
-  if (!stochastic) return cudaMemsetAsync(b.f, 0, sizeof(double) * 3 * N, st);
-  if (pp.fast || pp.any) {
-    const cudaError_t e = plain_stage(kPlainNoise, pp, b, nx, tb, st);
-    return e ? e : plain_stage(kPlainNoiseInverse, pp, b, nx, tb, st);
-  }
+cudaError_t plain_forcing_draw(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                               const FftTables<double>& tb, cudaStream_t st) {
+  if (!stochastic) return cudaSuccess;
+  if (pp.fast || pp.any) return plain_stage(kPlainNoise, pp, b, nx, tb, st);
   const long N2 = (long)(nx / 2 + 1) * ny * nz;
   k_noise_generate<<<(unsigned)((N2 + 127) / 128), 128, 0, st>>>(b.nwork, nx, ny, nz, b.sym, b.noise);
   count_launches(1);
-  cudaError_t e = fft3_c2r<double>(b.nwork, b.f, nx, ny, nz, 3, 1.0, tb, st);
+  return cudaGetLastError();
+}
+
+cudaError_t plain_forcing_finish(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                                 const FftTables<double>& tb, cudaStream_t st) {
+  if (!stochastic) return cudaMemsetAsync(b.f, 0, sizeof(double) * 3L * nx * ny * nz, st);
+  if (pp.fast || pp.any) return plain_stage(kPlainNoiseInverse, pp, b, nx, tb, st);
+  const cudaError_t e = fft3_c2r<double>(b.nwork, b.f, nx, ny, nz, 3, 1.0, tb, st);
   if (e != cudaSuccess) return e;
   k_step_advance<<<1, 1, 0, st>>>((uint64_t*)b.noise.step);
   count_launches(1);

@@ -342,7 +342,8 @@ int engine_allocate_grid(selm_sim* s) {
     if ((rc = dalloc(s, &s->u64[1], 3 * N))) return rc;
     if ((rc = dalloc(s, &s->fg64, 3 * N))) return rc;
     if ((rc = dalloc(s, &s->p64, N))) return rc;
-    if ((rc = dalloc(s, &s->work64, 6 * N2))) return rc;  // 3 components x N2 complex
+    // half spectra: the forcing's 3 components, the pressure
+    if ((rc = dalloc(s, &s->work64, 8 * N2))) return rc;
     if ((rc = dalloc(s, &s->partial, 3 * kSumParts))) return rc;
     if ((rc = dalloc(s, &s->sym64, 2 * s->nx))) return rc;
     if ((rc = dalloc(s, &s->step64, 1))) return rc;
@@ -548,7 +549,7 @@ static int set_particles_host(selm_sim* s, int M, const double* x, const double*
     }
     if ((rc = alloc_slots(s, s->tiles, s->tslots, M))) return rc;
     CU(cudaMemsetAsync(s->f, 0, sizeof(double) * 3 * M, s->st));
-    fused_invalidate_graphs(s);
+    step_graphs_invalidate(s);
   }
   if (M == 0) return SELM_OK;
   // periodic remap as LAMMPS' Domain::pbc at setup (whole box lengths until x is in [lo, hi));
@@ -776,7 +777,7 @@ extern "C" int selm_set_topology(selm_sim* s, const selm_topology* tp) {
   }
   s->have_topo = true;
   s->cb = nullptr;
-  fused_invalidate_graphs(s);
+  step_graphs_invalidate(s);
   return SELM_OK;
 }
 
@@ -785,7 +786,7 @@ extern "C" int selm_set_force_callback(selm_sim* s, selm_force_fn fn, void* user
   s->cb = fn;
   s->cb_user = user;
   if (fn) s->have_topo = false;
-  fused_invalidate_graphs(s);
+  step_graphs_invalidate(s);
   return SELM_OK;
 }
 
@@ -875,8 +876,8 @@ static PlainBufs plain_bufs(selm_sim* s, double* u_new) {
   b.u = u_new;
   b.p = s->p64;
   b.f = s->fg64;
-  b.work = (double2*)s->work64;
   b.nwork = (double2*)s->work64;
+  b.work = b.nwork + 3 * s->N2;
   b.sym = s->sym64;
   b.dx = s->dx;
   b.noise.seed = s->prm.seed;
@@ -891,36 +892,132 @@ static PlainBufs plain_bufs(selm_sim* s, double* u_new) {
 // the forcing of the step after the device counter's, which it advances
 static int plain_forcing_step(selm_sim* s) {
   prof_mark(s, "noise", true);
-  CU(plain_forcing(s->plan64, plain_bufs(s, nullptr), s->nx, s->ny, s->nz, s->prm.flag_stochastic != 0, s->tb64, s->st));
+  const PlainBufs b = plain_bufs(s, nullptr);
+  CU(plain_forcing_draw(s->plan64, b, s->nx, s->ny, s->nz, s->prm.flag_stochastic != 0, s->tb64, s->st));
+  CU(plain_forcing_finish(s->plan64, b, s->nx, s->ny, s->nz, s->prm.flag_stochastic != 0, s->tb64, s->st));
   prof_mark(s, "noise", false);
   return SELM_OK;
 }
 
-static int plain_step(selm_sim* s) {
-  const uint64_t n = ++s->step;
-  CouplingArgs a = coupling_args(s, n);
+// The launches of one step on positions x[cx], velocity u64[cu].  side (in a
+// graph capture): the forces at the new positions and the next forcing's draw
+// run beside the spread and the fluid solve, on st2 and st3.
+static int plain_body(selm_sim* s, bool side) {
+  CouplingArgs a = coupling_args(s, s->step + 1);
   a.step_ptr = s->step64;
   double* xo = s->x[s->cx];
   double* xn = s->x[s->cx ^ 1];
+  const PlainBufs b = plain_bufs(s, s->u64[s->cu ^ 1]);
+  const bool stochastic = s->prm.flag_stochastic != 0;
+  const bool forces = side && s->M > 0 && s->have_topo;
+  if (side) {
+    CU(cudaEventRecord(s->ev_fork3, s->st));
+    CU(cudaStreamWaitEvent(s->st3, s->ev_fork3, 0));
+    CU(plain_forcing_draw(s->plan64, b, s->nx, s->ny, s->nz, stochastic, s->tb64, s->st3));
+  }
   if (s->M > 0) {
     WRec<double>* rec = static_cast<WRec<double>*>(s->wrec);
     prof_mark(s, "interp_update", true);
     CU(interp_update<double>(s->u64[s->cu], xo, xn, s->v, s->f, s->m, s->tf, nullptr, rec, a, s->err, s->st,
                              &s->tslots));
     prof_mark(s, "interp_update", false);
+    if (forces) {
+      CU(cudaEventRecordWithFlags(s->ev_xv, s->st, cudaEventRecordExternal));  // x^{n+1} and v final
+      CU(cudaEventRecord(s->ev_fork, s->st));
+      CU(cudaStreamWaitEvent(s->st2, s->ev_fork, 0));
+      const int rc = engine_forces_on(s, xn, s->st2);
+      if (rc) return rc;
+      CU(cudaEventRecordWithFlags(s->ev_ready, s->st2, cudaEventRecordExternal));  // f too
+      CU(cudaEventRecord(s->ev_join, s->st2));
+    }
     prof_mark(s, "spread", true);
     CU(spread_slots<double>(s->fg64, true, xo, s->tf, s->tslots, a, s->st, rec));
     prof_mark(s, "spread", false);
-    s->cx ^= 1;
   }
   prof_mark(s, "fluid", true);
-  CU(plain_fluid_run(s->u64[s->cu], s->u64[s->cu ^ 1], s->plan64, plain_bufs(s, s->u64[s->cu ^ 1]), s->partial, s->nx,
-                     s->ny, s->nz, s->prm.dt, s->prm.mu, s->prm.rho, s->tb64, s->st));
+  CU(plain_ustar(s->u64[s->cu], s->u64[s->cu ^ 1], b, s->nx, s->ny, s->nz, s->prm.dt, s->prm.mu, s->prm.rho, s->st));
+  if (side) {
+    // u* has read the forcing: the next one may be written (and the step counter advanced)
+    CU(cudaEventRecord(s->ev_ustar, s->st));
+    CU(cudaStreamWaitEvent(s->st3, s->ev_ustar, 0));
+    CU(plain_forcing_finish(s->plan64, b, s->nx, s->ny, s->nz, stochastic, s->tb64, s->st3));
+    CU(cudaEventRecord(s->ev_join3, s->st3));
+  }
+  CU(plain_project(s->u64[s->cu ^ 1], s->plan64, b, s->partial, s->nx, s->ny, s->nz, s->tb64, s->st));
   prof_mark(s, "fluid", false);
-  s->cu ^= 1;
-  int rc = plain_forcing_step(s);
+  if (side) {
+    CU(cudaStreamWaitEvent(s->st, s->ev_join3, 0));
+    if (forces) CU(cudaStreamWaitEvent(s->st, s->ev_join, 0));
+    if (forces || s->M == 0) return SELM_OK;
+  } else {
+    const int rc = plain_forcing_step(s);
+    if (rc) return rc;
+  }
+  s->cx ^= 1;  // the forces at the new positions
+  const int rc = engine_forces(s);
+  s->cx ^= 1;
+  return rc;
+}
+
+static void plain_graphs_drop(selm_sim* s) {
+  for (int q = 0; q < 4; q++) {
+    if (s->pexec[q]) cudaGraphExecDestroy(s->pexec[q]);
+    s->pexec[q] = nullptr;
+    s->pready[q] = false;
+  }
+}
+
+void step_graphs_invalidate(selm_sim* s) {
+  plain_graphs_drop(s);
+  fused_invalidate_graphs(s);
+}
+
+// the step of the current buffers, captured and instantiated once
+static int plain_capture(selm_sim* s, int q) {
+  int rc = engine_side_stream(s);
   if (rc) return rc;
-  return engine_forces(s);
+  if (!s->st3) CU(cudaStreamCreateWithFlags(&s->st3, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&s->ev_fork3, &s->ev_ustar, &s->ev_join3})
+    if (!*e) CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  const unsigned long long l0 = launches_total();
+  CU(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
+  rc = plain_body(s, true);
+  cudaGraph_t g = nullptr;
+  const cudaError_t ec = cudaStreamEndCapture(s->st, &g);
+  s->pkernels[q] = launches_total() - l0;
+  uncount_launches(s->pkernels[q]);  // recorded, not run
+  cudaError_t ei = cudaSuccess;
+  if (!rc && ec == cudaSuccess) ei = cudaGraphInstantiate(&s->pexec[q], g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (rc) return rc;
+  if (ec != cudaSuccess || ei != cudaSuccess) {
+    s->pexec[q] = nullptr;
+    return selm_fail(SELM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec != cudaSuccess ? ec : ei));
+  }
+  s->pready[q] = s->M > 0 && s->have_topo;
+  return SELM_OK;
+}
+
+// One graph launch; launches one by one with a host force provider, per-kernel
+// timing, or the axis passes of the sizes without spectral kernels.
+static int plain_step(selm_sim* s) {
+  if (!s->cb && !s->prof && (s->plan64.fast || s->plan64.any)) {
+    const int q = s->cu + 2 * s->cx;
+    if (!s->pexec[q]) {
+      const int rc = plain_capture(s, q);
+      if (rc) return rc;
+    }
+    count_launches((unsigned)s->pkernels[q]);
+    CU(cudaGraphLaunch(s->pexec[q], s->st));
+    s->ready_early = s->pready[q];
+  } else {
+    const int rc = plain_body(s, false);
+    if (rc) return rc;
+  }
+  ++s->step;
+  s->cu ^= 1;
+  if (s->M > 0) s->cx ^= 1;
+  return SELM_OK;
 }
 
 extern "C" int selm_initial(selm_sim* s) {
@@ -966,9 +1063,11 @@ extern "C" int selm_destroy(selm_sim* s) {
     cudaEventDestroy(ev.b);
   }
   if (s->st2) cudaStreamSynchronize(s->st2);
+  if (s->st3) cudaStreamSynchronize(s->st3);
   if (s->st_copy) cudaStreamSynchronize(s->st_copy);
   analysis_detach_all(s);
   fused_release(s);
+  plain_graphs_drop(s);
   delete s->any64;
   free_all(s->allocs);
   sim_free_all(s);
@@ -976,6 +1075,9 @@ extern "C" int selm_destroy(selm_sim* s) {
   if (s->hcb) cudaFreeHost(s->hcb);
   if (s->own_st && s->st) cudaStreamDestroy(s->st);
   if (s->st2) cudaStreamDestroy(s->st2);
+  if (s->st3) cudaStreamDestroy(s->st3);
+  for (cudaEvent_t e : {s->ev_fork3, s->ev_ustar, s->ev_join3})
+    if (e) cudaEventDestroy(e);
   if (s->ev_fork) cudaEventDestroy(s->ev_fork);
   if (s->ev_join) cudaEventDestroy(s->ev_join);
   if (s->ev_xv) cudaEventDestroy(s->ev_xv);

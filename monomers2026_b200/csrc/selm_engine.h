@@ -62,6 +62,12 @@ struct selm_sim {
   selm::AnyPlan* any64 = nullptr;  // run-time factor kernels' plan, where plan64.any points at it
   selm::PlainPlan plan64{};
   int cu = 0;
+  // the plain form's captured steps, by (velocity buffer, position buffer)
+  cudaGraphExec_t pexec[4] = {};
+  unsigned long long pkernels[4] = {};
+  bool pready[4] = {};          // the graph records ev_xv and ev_ready
+  cudaStream_t st3 = nullptr;   // side stream: the next forcing beside the pressure solve
+  cudaEvent_t ev_fork3 = nullptr, ev_ustar = nullptr, ev_join3 = nullptr;
   uint32_t* err = nullptr;
   selm::FftTables<double> tb64{};
   selm::FftTables<float> tb32{};
@@ -119,6 +125,7 @@ int fused_step(selm_sim* s);
 int fused_get_field(selm_sim* s, int which, double* out);
 int fused_set_field(selm_sim* s, int which, const double* in);
 int fused_stream_changed(selm_sim* s);
+void step_graphs_invalidate(selm_sim* s);  // every form: the captured steps no longer hold
 void fused_invalidate_graphs(selm_sim* s);
 void fused_release(selm_sim* s);
 // the captured step of positions x[par] -> x[par ^ 1] (captured on first use, kept)

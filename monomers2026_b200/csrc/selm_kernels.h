@@ -50,11 +50,16 @@ struct PlainPlan {
   bool fast = false;
   const AnyPlan* any = nullptr;
 };
-cudaError_t plain_fluid_run(const double* u_old, double* u_new, const PlainPlan& pp, const PlainBufs& b,
-                            double* partial, int nx, int ny, int nz, double dt, double mu, double rho,
-                            const FftTables<double>& tb, cudaStream_t st);
-cudaError_t plain_forcing(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
-                          const FftTables<double>& tb, cudaStream_t st);
+// u* from u_old, b.f; then, in place, the projection and the mean removal
+cudaError_t plain_ustar(const double* u_old, double* u_new, const PlainBufs& b, int nx, int ny, int nz, double dt,
+                        double mu, double rho, cudaStream_t st);
+cudaError_t plain_project(double* u_new, const PlainPlan& pp, const PlainBufs& b, double* partial, int nx, int ny,
+                          int nz, const FftTables<double>& tb, cudaStream_t st);
+// the next step's forcing: its spectrum into b.nwork, then b.f (and the step counter advanced)
+cudaError_t plain_forcing_draw(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                               const FftTables<double>& tb, cudaStream_t st);
+cudaError_t plain_forcing_finish(const PlainPlan& pp, const PlainBufs& b, int nx, int ny, int nz, bool stochastic,
+                                 const FftTables<double>& tb, cudaStream_t st);
 template <typename T>
 cudaError_t fft3_r2c(const T* in, cpx<T>* out, int nx, int ny, int nz, int ncomp, const FftTables<T>& tb,
                      cudaStream_t st);
