@@ -337,133 +337,9 @@ __device__ __forceinline__ T interp_one(double rx, double ry, double rz, int Nx,
   return rv;
 }
 
-// Staggered stencil of component d at grid coordinates (gx, gy, gz): bases
-// floor(r) - 1 and the weight factors of each axis (axis d unshifted, the
-// others shifted by -1/2, the MAC face positions).
-template <typename T>
-__device__ __forceinline__ void stencil_of(double gx, double gy, double gz, int d, int base[3], T w[3][4]) {
-  const double r[3] = {d == 0 ? gx : gx - 0.5, d == 1 ? gy : gy - 0.5, d == 2 ? gz : gz - 0.5};
-#pragma unroll
-  for (int ax = 0; ax < 3; ax++) {
-    base[ax] = (int)floor(r[ax]) - 1;
-#pragma unroll
-    for (int i = 0; i < 4; i++) w[ax][i] = ref_weight<T>(fabs(r[ax] - (double)(base[ax] + i)));
-  }
-}
-
-// Gamma_d u: the weighted sum over the 4^3 stencil of component d, in the
-// reference's loop and product order (cuda/SELM_Kernel.cu:375-422).
-// SLAB: ud holds only the planes [z0, z0 + nzl) of the grid (a decomposed
-// instance's slab); points on other planes are left out (the slabs' sums add
-// up to the whole gather)
-template <typename T, bool SLAB = false>
-__device__ __forceinline__ T stencil_gather(const T* __restrict__ ud, const int base[3], const T w[3][4],
-                                            const CouplingArgs& a, int z0 = 0, int nzl = 0) {
-  T val = T(0);
-  // rows of 4 consecutive x-points: 16-byte vector loads over an aligned
-  // window when the rows are 16-byte aligned (nx a multiple of the vector
-  // width), with zero weights outside the stencil (the non-zero terms are
-  // added in the same order as point by point); scalar loads otherwise
-  constexpr int V = 16 / sizeof(T), NV = (4 + V - 1) / V + 1, W = NV * V;
-  using Vec = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  if (a.nx % V == 0) {
-    const int x0 = wrapi(base[0], a.nx);
-    const int a0 = x0 & ~(V - 1), off = x0 - a0;
-    int vs[NV];
-#pragma unroll
-    for (int m = 0; m < NV; m++) {
-      const int q = a0 + m * V;
-      vs[m] = (q >= a.nx) ? q - a.nx : q;
-    }
-    T wsel[W];
-#pragma unroll
-    for (int t = 0; t < W; t++) {
-      const int i = t - off;
-      wsel[t] = (i == 0) ? w[0][0] : (i == 1) ? w[0][1] : (i == 2) ? w[0][2] : (i == 3) ? w[0][3] : T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const T dk = T(1) * w[2][k];
-      const int zk = wrapi(base[2] + k, a.nz);
-      if (SLAB && (unsigned)(zk - z0) >= (unsigned)nzl) continue;
-      const long zoff = (long)(SLAB ? zk - z0 : zk) * a.ny;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const T dj = dk * w[1][j];
-        const T* row = ud + (zoff + wrapi(base[1] + j, a.ny)) * a.nx;
-#pragma unroll
-        for (int m = 0; m < NV; m++) {
-          // the last chunk holds stencil points only when the window is not chunk-aligned
-          Vec q{};
-          if (m < NV - 1 || off > 0) q = __ldg(reinterpret_cast<const Vec*>(row + vs[m]));
-          const T* e = reinterpret_cast<const T*>(&q);
-#pragma unroll
-          for (int t = 0; t < V; t++) val += e[t] * (dj * wsel[m * V + t]);
-        }
-      }
-    }
-  } else {
-    int ix[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) ix[i] = wrapi(base[0] + i, a.nx);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const T dk = T(1) * w[2][k];
-      const int zk = wrapi(base[2] + k, a.nz);
-      if (SLAB && (unsigned)(zk - z0) >= (unsigned)nzl) continue;
-      const long zoff = (long)(SLAB ? zk - z0 : zk) * a.ny;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const T dj = dk * w[1][j];
-        const T* row = ud + (zoff + wrapi(base[1] + j, a.ny)) * a.nx;
-#pragma unroll
-        for (int i = 0; i < 4; i++) val += __ldg(row + ix[i]) * (dj * w[0][i]);
-      }
-    }
-  }
-  return val;
-}
-
-// The stencil parts a thread of component d stores in the monomer's record:
-// axis d unshifted and axis d+1 shifted (static indices keep w in registers).
-template <typename T>
-__device__ __forceinline__ void record_store(WRec<T>& R, int d, const int base[3], const T w[3][4],
-                                             const CouplingArgs& a) {
-  const int nn[3] = {a.nx, a.ny, a.nz};
-  const int a1 = (d + 1) % 3;
-#pragma unroll
-  for (int ax = 0; ax < 3; ax++) {
-    if (ax == d || ax == a1) {
-      const int sh = (ax == d) ? 0 : 1;
-      R.b[ax][sh] = wrapi(base[ax], nn[ax]);
-#pragma unroll
-      for (int i = 0; i < 4; i++) R.w[ax][sh][i] = w[ax][i];
-    }
-  }
-}
-
-// Tiles of one axis that the union stencil (cells c0 .. c0+4, wrapped)
-// reaches: up to three distinct ones (a partial last tile can add a third).
-__device__ __forceinline__ int axis_tile_set(double g, int a, const BinSpec& bs, int& t0, int& t1, int& t2) {
-  const int n = bs.n[a], T = bs.tile[a];
-  const int c0 = wrapi((int)floor(g - 0.5) - 1, n);
-  t0 = c0 / T;
-  t1 = -1;
-  t2 = -1;
-  int cnt = 1;
-#pragma unroll
-  for (int i = 1; i < 5; i++) {
-    int c = c0 + i;
-    if (c >= n) c -= n;
-    const int t = c / T;
-    if (t != t0 && t != t1 && t != t2) {
-      if (t1 < 0) t1 = t;
-      else t2 = t;
-      cnt++;
-    }
-  }
-  return cnt;
-}
+// Spread tiles: kTX x kTY x kTZ cells (see the spread below).
+constexpr int kTX = 16, kTY = 8, kTZ = 16;  // 16 cells in z: fewer candidates straddle two tiles
+static_assert(kTX == kTZ, "tile indices of x and z");
 
 // Home cell of a grid coordinate along one axis: floor(g) wrapped into
 // [0, n), and whether frac(g) < 1/2 (the half-shifted stencil then starts two
@@ -477,221 +353,361 @@ __device__ __forceinline__ int home_cell(double g, int n, bool& low_half) {
   return wrapi((int)fl, n);
 }
 
-// Home mode: the slot, in the home tile's box (the tile plus 2 cells on each
-// side, x fastest), of component d's stencil base, from the thread of that
-// component.  With home cell c (tile origin t0) the unshifted base
-// floor(g) - 1 sits at box coordinate c - t0 + 1, the shifted base
-// floor(g - 1/2) - 1 at c - t0 or c - t0 + 1: always in [0, tile], and the 4
-// stencil points stay inside the box.
-__device__ __forceinline__ void home_slot_store(unsigned short (&hs)[3], int d, double gx, double gy, double gz,
-                                                const BinSpec& bs) {
-  const double g[3] = {gx, gy, gz};
-  int c[3];
-#pragma unroll
-  for (int ax = 0; ax < 3; ax++) {
-    bool low;
-    const int l = home_cell(g[ax], bs.n[ax], low) % bs.tile[ax];
-    c[ax] = (ax == d) ? l + 1 : (low ? l : l + 1);
+// File monomer p under every spread tile its union stencil reaches: tiles
+// t[axis][0 .. n[axis]).  A slot of the tile while it has room, else the
+// overflow list.  Home mode files it under one tile.
+__device__ __forceinline__ void tile_place(const TileSlots& ts, int p, int t, int slot, uint32_t* err) {
+  if (slot < ts.cap) {
+    ts.slots[(long)t * ts.cap + slot] = p;
+  } else {
+    const int q = atomicAdd(ts.ovf_count, 1);
+    if (q < ts.ovf_cap) ts.ovf[q] = make_int2(t, p);
+    else atomicOr(err, ERR_BUCKET_OVERFLOW);
   }
-  hs[d] = (unsigned short)((c[2] * (bs.tile[1] + 4) + c[1]) * (bs.tile[0] + 4) + c[0]);
+}
+__device__ __forceinline__ void tile_append(const TileSlots& ts, int p, const int (*t)[3], uint32_t* err) {
+  const int nbx = ts.bs.nb[0], nby = ts.bs.nb[1];
+  // a slab of a decomposed instance files only under its own tile layers
+  auto zin = [&](int tz) { return ts.tz1 == 0 || (tz >= ts.tz0 && tz < ts.tz1); };
+  if (t[0][2] < 0 && t[1][2] < 0 && t[2][2] < 0) {
+    // at most 2 x 2 x 2 tiles: all counters bumped before any slot is written, so the atomics overlap
+    int tt[8], sl[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const int tx = t[0][c & 1], ty = t[1][(c >> 1) & 1], tz = t[2][c >> 2];
+      const bool ok = tx >= 0 && ty >= 0 && tz >= 0 && zin(tz);
+      tt[c] = ok ? (tz * nby + ty) * nbx + tx : -1;
+      sl[c] = ok ? atomicAdd(&ts.count[tt[c]], 1) : 0;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (tt[c] >= 0) tile_place(ts, p, tt[c], sl[c], err);
+    return;
+  }
+#pragma unroll 1
+  for (int c = 0; c < 27; c++) {
+    const int tx = t[0][c % 3], ty = t[1][(c / 3) % 3], tz = t[2][c / 9];
+    if (tx < 0 || ty < 0 || tz < 0 || !zin(tz)) continue;
+    const int q = (tz * nby + ty) * nbx + tx;
+    tile_place(ts, p, q, atomicAdd(&ts.count[q], 1), err);
+  }
 }
 
-// Home mode: the tile of the monomer's cell.
-__device__ __forceinline__ int home_tile(double gx, double gy, double gz, const BinSpec& bs) {
-  bool lo_half;
-  const int cx = home_cell(gx, bs.n[0], lo_half), cy = home_cell(gy, bs.n[1], lo_half),
-            cz = home_cell(gz, bs.n[2], lo_half);
-  return ((cz / bs.tile[2]) * bs.nb[1] + cy / bs.tile[1]) * bs.nb[0] + cx / bs.tile[0];
+// ================================================================ interpolation and monomer update
+// A block takes mb consecutive monomers (runs of a chain, whose stencils
+// overlap) in three phases:
+//   A  thread (monomer, axis): grid coordinate, stencil bases and weights of the
+//      axis, unshifted and shifted, into the monomer's record in shared memory,
+//      and the tiles it is filed under;
+//   B  16 lanes per monomer component, lane (i, j) with the four z points of
+//      stencil column (i, j): a row's four points are one access, so a component
+//      costs its 16 rows of L1 lookups and four loads a lane, all independent;
+//      the 16 partial sums are added by shuffles in a fixed order;
+//   C  thread (monomer, component): drag, noise and the explicit update of
+//      lagrangian_update() (cuda/SELM_Kernel.cu:302-373); the records go to
+//      memory as 16-byte vectors.
+// A thread per component that gathered its own 16 rows took two 16-byte loads
+// a row on 32 distinct lines each (8.4 M L1 lookups at 1e5 monomers against
+// 4.8 M), recomputed the axes' weights and tiles in every component (2300
+// instructions a thread), and for few monomers was one long chain of dependent
+// latencies and instruction misses on few SMs (19 us for 20 monomers).
+constexpr int kMonThreads = 192, kMonMax = kMonThreads / 3, kMonGroups = kMonThreads / 16;
+// Monomers per block: four blocks on each of the 148 SMs while there are
+// enough, 64 at most (a thread per component in phases A and C) and 4 at least
+// (a group of lanes per component in phase B).
+static int monomers_per_block(int M) { return std::max(4, std::min(kMonMax, (M + 591) / 592)); }
+
+template <typename T> struct alignas(4 * sizeof(T) < 16 ? 4 * sizeof(T) : 16) Vec4 { T v[4]; };
+
+// a record in shared memory: 16 bytes more than in memory, so that the threads
+// of ten monomers, which write the same field, spread over the banks
+template <typename T> struct MonRec : WRec<T> {
+  uint4 pad;
+};
+template <typename T> struct MonBlock {
+  MonRec<T> rec[kMonMax];
+  T val[3 * kMonMax];
+  int tiles[kMonMax][3][3];  // per axis: the tiles of the union stencil, -1: none (home mode: [axis][0] the home tile)
+  int home[kMonMax][3];      // home mode: per axis 2 (cell in tile) + (frac < 1/2)
+};
+template <typename T> constexpr size_t mon_smem() { return sizeof(MonBlock<T>); }
+
+// tiles of one axis that the cells c0 .. c0 + 4 (wrapped) reach: up to three
+// distinct ones (a partial last tile can add a third)
+template <int TILE> __device__ __forceinline__ void axis_tile_set(double g, int n, int (&t)[3]) {
+  if (!isfinite(g)) g = 0.0;
+  const int c0 = wrapi((int)floor(g - 0.5) - 1, n);
+  t[0] = c0 / TILE;
+  t[1] = t[2] = -1;
+#pragma unroll
+  for (int i = 1; i < 5; i++) {
+    int c = c0 + i;
+    if (c >= n) c -= n;
+    const int q = c / TILE;
+    if (q != t[0] && q != t[1] && q != t[2]) {
+      if (t[1] < 0) t[1] = q;
+      else t[2] = q;
+    }
+  }
+}
+
+// phase A: the records of monomers p0 .. p0 + mc - 1 (and their tiles)
+template <typename T>
+__device__ __forceinline__ void stage_axis(MonBlock<T>& S, const double* __restrict__ x, int p0, int mc,
+                                           const CouplingArgs& a, const TileSlots& ts) {
+  const int q = threadIdx.x;
+  if (q >= 3 * mc) return;
+  const int m = q / 3, ax = q - 3 * m;
+  const int n = ax == 0 ? a.nx : ax == 1 ? a.ny : a.nz;
+  const double g = (x[3L * p0 + q] - a.lo) / a.dx;
+  WRec<T>& R = S.rec[m];
+#pragma unroll 1
+  for (int sh = 0; sh < 2; sh++) {
+    const double r = sh ? g - 0.5 : g;
+    const int base = (int)floor(r) - 1;
+    Vec4<T> w;
+#pragma unroll
+    for (int i = 0; i < 4; i++) w.v[i] = ref_weight<T>(fabs(r - (double)(base + i)));
+    *reinterpret_cast<Vec4<T>*>(R.w[ax][sh]) = w;
+    R.b[ax][sh] = wrapi(base, n);
+  }
+  if (!ts.count) return;
+  if (ts.home) {
+    bool low;
+    const int c = home_cell(g, n, low);
+    const int t = ax == 1 ? c / kTY : c / kTX;  // (kTZ = kTX)
+    S.tiles[m][ax][0] = t;
+    S.home[m][ax] = 2 * (c - t * (ax == 1 ? kTY : kTX)) + (low ? 1 : 0);
+  } else {
+    int t[3];
+    if (ax == 1) axis_tile_set<kTY>(g, n, t);
+    else axis_tile_set<kTX>(g, n, t);
+#pragma unroll
+    for (int i = 0; i < 3; i++) S.tiles[m][ax][i] = t[i];
+  }
+}
+
+// The home tile of monomer m of the block
+template <typename T> __device__ __forceinline__ int staged_home_tile(const MonBlock<T>& S, int m, const BinSpec& bs) {
+  return (S.tiles[m][2][0] * bs.nb[1] + S.tiles[m][1][0]) * bs.nb[0] + S.tiles[m][0][0];
+}
+
+// after phase A, thread (monomer, component): the box slot of the component
+// (home mode), and the filing by the thread of component 0
+template <typename T>
+__device__ __forceinline__ void file_staged(MonBlock<T>& S, int p0, int mc, const TileSlots& ts, uint32_t* err) {
+  const int q = threadIdx.x;
+  if (!ts.count || q >= 3 * mc) return;
+  const int m = q / 3, d = q - 3 * m;
+  if (ts.home) {
+    // With home cell c (tile origin t0) the unshifted base floor(g) - 1 sits at
+    // box coordinate c - t0 + 1, the shifted base floor(g - 1/2) - 1 at c - t0
+    // or c - t0 + 1: always in [0, tile], and the 4 stencil points stay inside
+    // the box of the tile plus 2 cells on each side (x fastest).
+    int c[3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) {
+      const int l = S.home[m][ax] >> 1, low = S.home[m][ax] & 1;
+      c[ax] = (ax != d && low) ? l : l + 1;
+    }
+    S.rec[m].hs[d] = (unsigned short)((c[2] * (kTY + 4) + c[1]) * (kTX + 4) + c[0]);
+    if (d == 0) {
+      const int t = staged_home_tile(S, m, ts.bs);
+      tile_place(ts, p0 + m, t, atomicAdd(&ts.count[t], 1), err);
+    }
+  } else if (d == 0) {
+    tile_append(ts, p0 + m, S.tiles[m], err);
+  }
+}
+
+// phase B: S.val[3 m + d] = Gamma_d u at monomer m.  SLAB: u holds only the
+// planes [z0, z0 + nzl) of the grid (a decomposed instance's slab); points on
+// other planes are left out (the slabs' sums add up to the whole gather).
+template <typename T, bool SLAB>
+__device__ __forceinline__ void gather_staged(MonBlock<T>& S, int mc, const T* __restrict__ u, const CouplingArgs& a,
+                                              int z0, int nzl) {
+  const int lane = threadIdx.x & 15, i = lane & 3, j = lane >> 2;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  const long cstride = (long)a.nx * a.ny * (SLAB ? nzl : a.nz);
+  const int plane = a.nx * a.ny;
+  constexpr int U = 4;  // components in flight per group of lanes
+  for (int q0 = threadIdx.x >> 4; q0 < 3 * mc; q0 += U * kMonGroups) {
+    T v[U][4], sum[U];
+#pragma unroll
+    for (int s = 0; s < U; s++) {
+      const int q = q0 + s * kMonGroups;
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[s][k] = T(0);
+      if (q < 3 * mc) {
+        const int m = q / 3, d = q - 3 * m;
+        const WRec<T>& R = S.rec[m];
+        int xi = R.b[0][d != 0] + i, yj = R.b[1][d != 1] + j, zk = R.b[2][d != 2];
+        if (xi >= a.nx) xi -= a.nx;
+        if (yj >= a.ny) yj -= a.ny;
+        const T* col = u + d * cstride + yj * a.nx + xi;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const int zr = SLAB ? zk - z0 : zk;
+          if (!SLAB || (unsigned)zr < (unsigned)nzl) v[s][k] = __ldg(col + (long)zr * plane);
+          if (++zk == a.nz) zk = 0;
+        }
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < U; s++) {
+      const int q = min(q0 + s * kMonGroups, 3 * mc - 1);
+      const int m = q / 3, d = q - 3 * m;
+      const WRec<T>& R = S.rec[m];
+      const Vec4<T> wz = *reinterpret_cast<const Vec4<T>*>(R.w[2][d != 2]);
+      T t = v[s][0] * wz.v[0];
+#pragma unroll
+      for (int k = 1; k < 4; k++) t += v[s][k] * wz.v[k];
+      sum[s] = t * (R.w[0][d != 0][i] * R.w[1][d != 1][j]);
+    }
+    // the sums over the 16 lanes, four at once: after two exchanges a lane
+    // holds a quarter of component (lane >> 2)'s sum, two more add the quarters
+    const bool up8 = lane & 8, up4 = lane & 4;
+    T a0 = up8 ? sum[2] : sum[0], a1 = up8 ? sum[3] : sum[1];
+    a0 += __shfl_xor_sync(half, up8 ? sum[0] : sum[2], 8);
+    a1 += __shfl_xor_sync(half, up8 ? sum[1] : sum[3], 8);
+    T t = up4 ? a1 : a0;
+    t += __shfl_xor_sync(half, up4 ? a0 : a1, 4);
+    t += __shfl_xor_sync(half, t, 2);
+    t += __shfl_xor_sync(half, t, 1);
+    const int q = q0 + (lane >> 2) * kMonGroups;
+    if ((lane & 3) == 0 && q < 3 * mc) S.val[q] = t;
+  }
+}
+
+// the block's records to memory
+template <typename T>
+__device__ __forceinline__ void store_records(const MonBlock<T>& S, int p0, int mc, WRec<T>* __restrict__ rec) {
+  constexpr int V = sizeof(WRec<T>) / 16, VS = sizeof(MonRec<T>) / 16;
+  const uint4* s = reinterpret_cast<const uint4*>(S.rec);
+  uint4* d = reinterpret_cast<uint4*>(rec + p0);
+  for (int i = threadIdx.x; i < V * mc; i += kMonThreads) d[i] = s[(i / V) * VS + i % V];
 }
 
 // Home mode: the scale data of the home tile's fixed-point box, from the
 // thread of one component: its impulse |tf| and its weight factors.
 template <typename T>
-__device__ __forceinline__ void home_scale_note(const TileSlots& ts, double gx, double gy, double gz, double tf,
-                                                const T (&w)[3][4]) {
-  const int t = home_tile(gx, gy, gz, ts.bs);
+__device__ __forceinline__ void home_scale_note(const TileSlots& ts, const MonBlock<T>& S, int m, int d, double tf) {
+  const int t = staged_home_tile(S, m, ts.bs);
   atomicMax(&ts.tmax[t], (unsigned long long)__double_as_longlong(fabs(tf)));
   bool big = false;
 #pragma unroll
   for (int ax = 0; ax < 3; ax++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) big |= (w[ax][i] > T(0.5));
+    for (int i = 0; i < 4; i++) big |= (S.rec[m].w[ax][ax != d][i] > T(0.5));
   if (big) atomicOr(&ts.quirk[t], 1);
 }
 
-// File monomer p under every spread tile its union stencil reaches (home
-// mode: under its home tile only): a slot of the tile while it has room,
-// else the overflow list.
-__device__ __forceinline__ void tile_append(const TileSlots& ts, int p, double gx, double gy, double gz, uint32_t* err) {
-  const BinSpec& bs = ts.bs;
-  if (ts.home) {
-    const int t = home_tile(gx, gy, gz, bs);
-    const int slot = atomicAdd(&ts.count[t], 1);
-    if (slot < ts.cap) {
-      ts.slots[(long)t * ts.cap + slot] = p;
-    } else {
-      const int q = atomicAdd(ts.ovf_count, 1);
-      if (q < ts.ovf_cap) ts.ovf[q] = make_int2(t, p);
-      else atomicOr(err, ERR_BUCKET_OVERFLOW);
-    }
-    return;
-  }
-  if (!isfinite(gx)) gx = 0.0;
-  if (!isfinite(gy)) gy = 0.0;
-  if (!isfinite(gz)) gz = 0.0;
-  int x0, x1, x2, y0, y1, y2, z0, z1, z2;
-  const int nxs = axis_tile_set(gx, 0, bs, x0, x1, x2);
-  const int nys = axis_tile_set(gy, 1, bs, y0, y1, y2);
-  const int nzs = axis_tile_set(gz, 2, bs, z0, z1, z2);
-  auto place = [&](int t, int slot) {
-    if (slot < ts.cap) {
-      ts.slots[(long)t * ts.cap + slot] = p;
-    } else {
-      const int q = atomicAdd(ts.ovf_count, 1);
-      if (q < ts.ovf_cap) ts.ovf[q] = make_int2(t, p);
-      else atomicOr(err, ERR_BUCKET_OVERFLOW);
-    }
-  };
-  // a slab of a decomposed instance files only under its own tile layers
-  auto zin = [&](int tz) { return ts.tz1 == 0 || (tz >= ts.tz0 && tz < ts.tz1); };
-  if (nxs <= 2 && nys <= 2 && nzs <= 2) {
-    // at most 2 x 2 x 2 tiles (tiles of at least 5 cells): all counters bumped
-    // before any slot is written, so the atomics overlap
-    int tt[8], sl[8];
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int i = c & 1, j = (c >> 1) & 1, k = c >> 2;
-      const bool ok = i < nxs && j < nys && k < nzs && zin(k ? z1 : z0);
-      tt[c] = ok ? ((k ? z1 : z0) * bs.nb[1] + (j ? y1 : y0)) * bs.nb[0] + (i ? x1 : x0) : -1;
-      sl[c] = ok ? atomicAdd(&ts.count[tt[c]], 1) : 0;
-    }
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-      if (tt[c] >= 0) place(tt[c], sl[c]);
-    return;
-  }
-#pragma unroll 1
-  for (int k = 0; k < nzs; k++) {
-    const int tz = (k == 0) ? z0 : (k == 1) ? z1 : z2;
-    if (!zin(tz)) continue;
-#pragma unroll 1
-    for (int j = 0; j < nys; j++) {
-      const int ty = (j == 0) ? y0 : (j == 1) ? y1 : y2;
-#pragma unroll 1
-      for (int i = 0; i < nxs; i++) {
-        const int tx = (i == 0) ? x0 : (i == 1) ? x1 : x2;
-        const int t = (tz * bs.nb[1] + ty) * bs.nb[0] + tx;
-        place(t, atomicAdd(&ts.count[t], 1));
-      }
-    }
-  }
-}
-
-// lagrangian_update() of cuda/SELM_Kernel.cu:302-373, one thread per
-// (monomer, component); the spread part lives in k_spread_tiles.  The thread
-// of component d also stores, for the spread of the same step, the stencil
-// bases and weights of axis d (unshifted) and axis d+1 (shifted) in the
-// monomer's record, so the three threads together fill it.  GATHERED: u is
-// the interpolated velocity itself, [3M] by monomer component (a decomposed
-// instance sums it over its slabs), and only the update and the filing run.
+// GATHERED: u is the interpolated velocity itself, [3M] by monomer component
+// (a decomposed instance sums it over its slabs), and only the update and the
+// filing run.
 template <typename T, bool GATHERED = false>
-// 256 threads, at least four blocks per SM in FP32 (64 registers): more warps in flight
-// for the latency-bound stencil gathers
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_interp_update(const T* __restrict__ u, const double* __restrict__ x_old,
-                                                       double* __restrict__ x_new, double* __restrict__ v,
-                                                       double* __restrict__ f, const double* __restrict__ m,
-                                                       double* __restrict__ tf_out, const int* __restrict__ order,
-                                                       WRec<T>* __restrict__ rec, CouplingArgs a,
-                                                       uint32_t* __restrict__ err, TileSlots ts) {
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 3L * a.M) return;
-  const int s = (int)(gid / 3), d = (int)(gid % 3);
-  const int p = order ? order[s] : s;
-  const long g = 3L * p + d;
-  const long N = (long)a.nx * a.ny * a.nz;
-  const double gx = (x_old[3L * p] - a.lo) / a.dx, gy = (x_old[3L * p + 1] - a.lo) / a.dx,
-               gz = (x_old[3L * p + 2] - a.lo) / a.dx;
-  int base[3];
-  T w[3][4];
-  stencil_of<T>(gx, gy, gz, d, base, w);
-  const T val = GATHERED ? u[g] : stencil_gather<T>(u + d * N, base, w, a);
-  if (rec) {
-    record_store<T>(rec[p], d, base, w, a);
-    if (ts.home) home_slot_store(rec[p].hs, d, gx, gy, gz, ts.bs);
+__global__ void __launch_bounds__(kMonThreads, sizeof(T) == 4 ? 6 : 5)
+    k_interp_update(const T* __restrict__ u, const double* __restrict__ x_old, double* __restrict__ x_new,
+                    double* __restrict__ v, double* __restrict__ f, const double* __restrict__ m,
+                    double* __restrict__ tf_out, WRec<T>* __restrict__ rec, CouplingArgs a,
+                    uint32_t* __restrict__ err, TileSlots ts, int mb) {
+  __shared__ __align__(16) MonBlock<T> S;
+  const int p0 = blockIdx.x * mb, mc = min(mb, a.M - p0), q = threadIdx.x;
+  stage_axis<T>(S, x_old, p0, mc, a, ts);
+  __syncthreads();
+  const bool mine = q < 3 * mc;
+  const long g = 3L * p0 + q;
+  const int mq = q / 3, d = q - 3 * mq;
+  double kick = 0.0, vg = 0.0, fg = 0.0, xg = 0.0;
+  if (mine) {
+    vg = v[g];
+    fg = f[g];
+    xg = x_old[g];
+    if (a.stochastic) {
+      double z1;
+      const uint64_t step = a.step_ptr ? *a.step_ptr : a.step;
+      philox_normal2(a.seed, (uint32_t)(p0 + mq), 4u + (uint32_t)d, step, kick, z1);
+      kick *= a.coef;
+    }
   }
-  if (ts.count && d == 0) tile_append(ts, p, gx, gy, gz, err);  // the spread of this step reads x_old
-  const double vg = v[g];
+  file_staged<T>(S, p0, mc, ts, err);  // the spread of this step reads x_old
+  if (!GATHERED) gather_staged<T, false>(S, mc, u, a, 0, 0);
+  __syncthreads();
+  store_records<T>(S, p0, mc, rec);
+  if (!mine) return;
+  const T val = GATHERED ? u[g] : S.val[q];
   double t_f = -a.upsilon * (vg - (double)val) * a.dt;
-  if (a.stochastic) {
-    double z0, z1;
-    const uint64_t step = a.step_ptr ? *a.step_ptr : a.step;
-    philox_normal2(a.seed, (uint32_t)p, 4u + (uint32_t)d, step, z0, z1);
-    t_f += z0 * a.coef;
-  }
+  if (a.stochastic) t_f += kick;
   tf_out[g] = t_f;
-  if (ts.home) home_scale_note<T>(ts, gx, gy, gz, t_f, w);
-  t_f += a.dt * f[g];
+  if (ts.home) home_scale_note<T>(ts, S, mq, d, t_f);
+  t_f += a.dt * fg;
   f[g] = t_f / a.dt;
   const double tmp = vg * a.dt;
+  const double L = a.hi - a.lo;
+  if (fabs(tmp) > L / 2) atomicOr(err, ERR_DISPLACEMENT);
+  double tx = xg + tmp;
+  if (tx > a.hi) tx -= L;
+  else if (tx < a.lo) tx += L;
+  x_new[g] = tx;
+  const double vn = vg + t_f / m[p0 + mq];
+  v[g] = vn;
+  if (!isfinite(vn) || !isfinite(tx)) atomicOr(err, ERR_NONFINITE);
+}
+
+// ---- quasi-steady (overdamped) form, no reference counterpart
+// Before the fluid solve: the stencil records at x^n for binning, spreading and
+// the move, and the impulse array the spread subtracts, tf = -F / dV, so that
+// the grid receives the force density +F / dV of the conservative forces.
+template <typename T>
+__global__ void __launch_bounds__(kMonThreads) k_qs_prepare(const double* __restrict__ x, const double* __restrict__ f,
+                                                            double* __restrict__ tf_out, WRec<T>* __restrict__ rec,
+                                                            CouplingArgs a, double inv_dv, TileSlots ts,
+                                                            uint32_t* __restrict__ err, int mb) {
+  __shared__ __align__(16) MonBlock<T> S;
+  const int p0 = blockIdx.x * mb, mc = min(mb, a.M - p0), q = threadIdx.x;
+  stage_axis<T>(S, x, p0, mc, a, ts);
+  __syncthreads();
+  file_staged<T>(S, p0, mc, ts, err);
+  if (q < 3 * mc) {
+    const long g = 3L * p0 + q;
+    const double t = -f[g] * inv_dv;
+    tf_out[g] = t;
+    if (ts.home) home_scale_note<T>(ts, S, q / 3, q % 3, t);
+  }
+  __syncthreads();
+  store_records<T>(S, p0, mc, rec);
+}
+
+// After the fluid solve: v = Gamma u (x^n) with the records of x^n, x^{n+1} =
+// x^n + dt v with the inertial form's single periodic wrap; f keeps the
+// conservative force.
+template <typename T>
+__global__ void __launch_bounds__(kMonThreads, sizeof(T) == 4 ? 8 : 6)
+    k_qs_move(const T* __restrict__ u, const double* __restrict__ x_old, double* __restrict__ x_new,
+              double* __restrict__ v, const WRec<T>* __restrict__ rec, CouplingArgs a, uint32_t* __restrict__ err,
+              int mb) {
+  __shared__ __align__(16) MonBlock<T> S;
+  const int p0 = blockIdx.x * mb, mc = min(mb, a.M - p0), q = threadIdx.x;
+  {
+    constexpr int V = sizeof(WRec<T>) / 16, VS = sizeof(MonRec<T>) / 16;
+    uint4* s = reinterpret_cast<uint4*>(S.rec);
+    const uint4* src = reinterpret_cast<const uint4*>(rec + p0);
+    for (int i = q; i < V * mc; i += kMonThreads) s[(i / V) * VS + i % V] = src[i];
+  }
+  __syncthreads();
+  gather_staged<T, false>(S, mc, u, a, 0, 0);
+  __syncthreads();
+  if (q >= 3 * mc) return;
+  const long g = 3L * p0 + q;
+  const double vel = (double)S.val[q];
+  const double tmp = vel * a.dt;
   const double L = a.hi - a.lo;
   if (fabs(tmp) > L / 2) atomicOr(err, ERR_DISPLACEMENT);
   double tx = x_old[g] + tmp;
   if (tx > a.hi) tx -= L;
   else if (tx < a.lo) tx += L;
   x_new[g] = tx;
-  const double vn = vg + t_f / m[p];
-  v[g] = vn;
-  if (!isfinite(vn) || !isfinite(tx)) atomicOr(err, ERR_NONFINITE);
-}
-
-
-// ---- quasi-steady (overdamped) form, no reference counterpart
-// Before the fluid solve: the stencil records at x^n for binning and spreading,
-// and the impulse array the spread subtracts, tf = -F / dV, so that the grid
-// receives the force density +F / dV of the conservative forces.
-template <typename T>
-__global__ void __launch_bounds__(256) k_qs_prepare(const double* __restrict__ x, const double* __restrict__ f,
-                                                    double* __restrict__ tf_out, WRec<T>* __restrict__ rec,
-                                                    CouplingArgs a, double inv_dv, TileSlots ts,
-                                                    uint32_t* __restrict__ err) {
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 3L * a.M) return;
-  const int p = (int)(gid / 3), d = (int)(gid % 3);
-  const double gx = (x[3L * p] - a.lo) / a.dx, gy = (x[3L * p + 1] - a.lo) / a.dx, gz = (x[3L * p + 2] - a.lo) / a.dx;
-  int base[3];
-  T w[3][4];
-  stencil_of<T>(gx, gy, gz, d, base, w);
-  record_store<T>(rec[p], d, base, w, a);
-  if (ts.home) home_slot_store(rec[p].hs, d, gx, gy, gz, ts.bs);
-  if (ts.count && d == 0) tile_append(ts, p, gx, gy, gz, err);
-  tf_out[gid] = -f[gid] * inv_dv;
-  if (ts.home) home_scale_note<T>(ts, gx, gy, gz, tf_out[gid], w);
-}
-
-// After the fluid solve: v = Gamma u (x^n), x^{n+1} = x^n + dt v with the
-// inertial form's single periodic wrap; f keeps the conservative force.
-template <typename T>
-__global__ void __launch_bounds__(384) k_qs_move(const T* __restrict__ u, const double* __restrict__ x_old,
-                                                 double* __restrict__ x_new, double* __restrict__ v, CouplingArgs a,
-                                                 uint32_t* __restrict__ err) {
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 3L * a.M) return;
-  const int p = (int)(gid / 3), d = (int)(gid % 3);
-  const long N = (long)a.nx * a.ny * a.nz;
-  const double gx = (x_old[3L * p] - a.lo) / a.dx, gy = (x_old[3L * p + 1] - a.lo) / a.dx,
-               gz = (x_old[3L * p + 2] - a.lo) / a.dx;
-  int base[3];
-  T w[3][4];
-  stencil_of<T>(gx, gy, gz, d, base, w);
-  const double vel = (double)stencil_gather<T>(u + d * N, base, w, a);
-  const double tmp = vel * a.dt;
-  const double L = a.hi - a.lo;
-  if (fabs(tmp) > L / 2) atomicOr(err, ERR_DISPLACEMENT);
-  double tx = x_old[gid] + tmp;
-  if (tx > a.hi) tx -= L;
-  else if (tx < a.lo) tx += L;
-  x_new[gid] = tx;
-  v[gid] = vel;
+  v[g] = vel;
   if (!isfinite(vel) || !isfinite(tx)) atomicOr(err, ERR_NONFINITE);
 }
 
@@ -699,17 +715,19 @@ template <typename T>
 cudaError_t qs_prepare(const double* x, const double* f, double* tf, WRec<T>* rec, const CouplingArgs& a,
                        double inv_dv, cudaStream_t st, const TileSlots* ts, uint32_t* err) {
   if (a.M <= 0) return cudaSuccess;
-  k_qs_prepare<T><<<(unsigned)((3L * a.M + 255) / 256), 256, 0, st>>>(x, f, tf, rec, a, inv_dv,
-                                                                      ts ? *ts : TileSlots{}, err);
+  const int mb = monomers_per_block(a.M);
+  k_qs_prepare<T><<<(unsigned)((a.M + mb - 1) / mb), kMonThreads, 0, st>>>(x, f, tf, rec, a, inv_dv,
+                                                                           ts ? *ts : TileSlots{}, err, mb);
   count_launches(1);
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t qs_move(const T* u, const double* x_old, double* x_new, double* v, const CouplingArgs& a, uint32_t* err,
-                    cudaStream_t st) {
+cudaError_t qs_move(const T* u, const double* x_old, double* x_new, double* v, const WRec<T>* rec, const CouplingArgs& a,
+                    uint32_t* err, cudaStream_t st) {
   if (a.M <= 0) return cudaSuccess;
-  k_qs_move<T><<<(unsigned)((3L * a.M + 383) / 384), 384, 0, st>>>(u, x_old, x_new, v, a, err);
+  const int mb = monomers_per_block(a.M);
+  k_qs_move<T><<<(unsigned)((a.M + mb - 1) / mb), kMonThreads, 0, st>>>(u, x_old, x_new, v, rec, a, err, mb);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -717,10 +735,10 @@ template cudaError_t qs_prepare<double>(const double*, const double*, double*, W
                                         double, cudaStream_t, const TileSlots*, uint32_t*);
 template cudaError_t qs_prepare<float>(const double*, const double*, double*, WRec<float>*, const CouplingArgs&,
                                        double, cudaStream_t, const TileSlots*, uint32_t*);
-template cudaError_t qs_move<double>(const double*, const double*, double*, double*, const CouplingArgs&, uint32_t*,
-                                     cudaStream_t);
-template cudaError_t qs_move<float>(const float*, const double*, double*, double*, const CouplingArgs&, uint32_t*,
-                                    cudaStream_t);
+template cudaError_t qs_move<double>(const double*, const double*, double*, double*, const WRec<double>*,
+                                     const CouplingArgs&, uint32_t*, cudaStream_t);
+template cudaError_t qs_move<float>(const float*, const double*, double*, double*, const WRec<float>*,
+                                    const CouplingArgs&, uint32_t*, cudaStream_t);
 
 // Pure interpolation (operator entry point): out[p][d] = Gamma_d u (x_p)
 template <typename T>
@@ -753,12 +771,12 @@ template cudaError_t interp_only<float>(const float*, const double*, int, int, i
 
 template <typename T>
 cudaError_t interp_update(const T* u, const double* x_old, double* x_new, double* v, double* f, const double* m,
-                          double* tf, const int* order, WRec<T>* rec, const CouplingArgs& a, uint32_t* err,
-                          cudaStream_t st, const TileSlots* ts) {
+                          double* tf, WRec<T>* rec, const CouplingArgs& a, uint32_t* err, cudaStream_t st,
+                          const TileSlots* ts) {
   if (a.M <= 0) return cudaSuccess;
-  const long nt = 3L * a.M;
-  k_interp_update<T><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(u, x_old, x_new, v, f, m, tf, order, rec, a,
-                                                                    err, ts ? *ts : TileSlots{});
+  const int mb = monomers_per_block(a.M);
+  k_interp_update<T><<<(unsigned)((a.M + mb - 1) / mb), kMonThreads, 0, st>>>(u, x_old, x_new, v, f, m, tf, rec, a, err,
+                                                                              ts ? *ts : TileSlots{}, mb);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -767,24 +785,24 @@ cudaError_t interp_update(const T* u, const double* x_old, double* x_new, double
 // interpolation that comes from the slab's planes [z0, z0 + nzl) (u: the
 // slab's velocity [3][nzl][ny][nx]), into out [3M]
 template <typename T>
-__global__ void __launch_bounds__(256) k_interp_partial(const T* __restrict__ u, const double* __restrict__ x, CouplingArgs a,
-                                                        int z0, int nzl, T* __restrict__ out) {
-  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 3L * a.M) return;
-  const int p = (int)(gid / 3), d = (int)(gid % 3);
-  const double gx = (x[3L * p] - a.lo) / a.dx, gy = (x[3L * p + 1] - a.lo) / a.dx, gz = (x[3L * p + 2] - a.lo) / a.dx;
-  int base[3];
-  T w[3][4];
-  stencil_of<T>(gx, gy, gz, d, base, w);
-  out[gid] = stencil_gather<T, true>(u + (long)d * nzl * a.ny * a.nx, base, w, a, z0, nzl);
+__global__ void __launch_bounds__(kMonThreads) k_interp_partial(const T* __restrict__ u, const double* __restrict__ x,
+                                                                CouplingArgs a, int z0, int nzl, T* __restrict__ out,
+                                                                int mb) {
+  __shared__ __align__(16) MonBlock<T> S;
+  const int p0 = blockIdx.x * mb, mc = min(mb, a.M - p0);
+  stage_axis<T>(S, x, p0, mc, a, TileSlots{});
+  __syncthreads();
+  gather_staged<T, true>(S, mc, u, a, z0, nzl);
+  __syncthreads();
+  if (threadIdx.x < 3 * mc) out[3L * p0 + threadIdx.x] = S.val[threadIdx.x];
 }
 
 template <typename T>
 cudaError_t interp_partial(const T* u_slab, const double* x, const CouplingArgs& a, int z0, int nzl, T* out,
                            cudaStream_t st) {
   if (a.M <= 0) return cudaSuccess;
-  const long nt = 3L * a.M;
-  k_interp_partial<T><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(u_slab, x, a, z0, nzl, out);
+  const int mb = monomers_per_block(a.M);
+  k_interp_partial<T><<<(unsigned)((a.M + mb - 1) / mb), kMonThreads, 0, st>>>(u_slab, x, a, z0, nzl, out, mb);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -799,9 +817,9 @@ cudaError_t interp_update_gathered(const T* gathered, const double* x_old, doubl
                                    const double* m, double* tf, WRec<T>* rec, const CouplingArgs& a, uint32_t* err,
                                    cudaStream_t st, const TileSlots& ts) {
   if (a.M <= 0) return cudaSuccess;
-  const long nt = 3L * a.M;
-  k_interp_update<T, true><<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(gathered, x_old, x_new, v, f, m, tf, nullptr,
-                                                                         rec, a, err, ts);
+  const int mb = monomers_per_block(a.M);
+  k_interp_update<T, true><<<(unsigned)((a.M + mb - 1) / mb), kMonThreads, 0, st>>>(gathered, x_old, x_new, v, f, m, tf,
+                                                                                    rec, a, err, ts, mb);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -839,7 +857,6 @@ template cudaError_t interp_update_gathered<double>(const double*, const double*
 //          overflow for |v| < 2^(62 - 2k); a step of m 2^-(62-2k), 2^-44 of
 //          the tile's largest impulse for n <= 512.  Shared-memory 32-bit
 //          integer atomics are native; 64-bit ones are not.
-constexpr int kTX = 16, kTY = 8, kTZ = 16;  // 16 cells in z: fewer candidates straddle two tiles
 constexpr int kSpreadThreads = 3 * kTY * kTZ;  // also the number of tile rows (component, y, z)
 constexpr int kSpreadCells = 3 * kTZ * kTY * kTX;
 constexpr int kSpreadPad = 32;  // per-lane dummy slots: points outside the tile add there (never read)
@@ -864,8 +881,6 @@ __device__ __forceinline__ long long to_fixed(double v) { return __double2ll_rn(
 __device__ __forceinline__ int round_small(float v) {  // rint(v) for |v| < 2^22
   return __float_as_int(v + 12582912.0f) - 0x4B400000;
 }
-
-template <typename T> struct alignas(4 * sizeof(T)) Vec4 { T v[4]; };
 
 // Tile geometry and fixed-point state shared by the plane additions of a block.
 struct SpreadTile {
@@ -1657,11 +1672,11 @@ template cudaError_t spread_slots<float>(float*, bool, const double*, const doub
                                          const CouplingArgs&, cudaStream_t, const WRec<float>*);
 
 template cudaError_t interp_update<double>(const double*, const double*, double*, double*, double*, const double*,
-                                           double*, const int*, WRec<double>*, const CouplingArgs&, uint32_t*,
-                                           cudaStream_t, const TileSlots*);
+                                           double*, WRec<double>*, const CouplingArgs&, uint32_t*, cudaStream_t,
+                                           const TileSlots*);
 template cudaError_t interp_update<float>(const float*, const double*, double*, double*, double*, const double*,
-                                          double*, const int*, WRec<float>*, const CouplingArgs&, uint32_t*,
-                                          cudaStream_t, const TileSlots*);
+                                          double*, WRec<float>*, const CouplingArgs&, uint32_t*, cudaStream_t,
+                                          const TileSlots*);
 // The tile accumulators (49 KB in FP32, 74 KB in FP64) exceed the default 48 KB of dynamic
 // shared memory: raise the limit once per device (the first call on a device
 // does it; make that call before any stream capture).

@@ -703,7 +703,7 @@ template <typename T> static int fused_step_t(selm_sim* s, bool* forces_done) {
     if (rc) return rc;
     if (s->M > 0) {
       prof_mark(s, "interp_update", true);
-      CUF(qs_move<T>((const T*)z->u, xo, xn, s->v, a, s->err, s->st));
+      CUF(qs_move<T>((const T*)z->u, xo, xn, s->v, static_cast<const WRec<T>*>(s->wrec), a, s->err, s->st));
       prof_mark(s, "interp_update", false);
     }
     return SELM_OK;
@@ -711,7 +711,7 @@ template <typename T> static int fused_step_t(selm_sim* s, bool* forces_done) {
   if (s->M > 0) {
     WRec<T>* rec = static_cast<WRec<T>*>(s->wrec);
     prof_mark(s, "interp_update", true);
-    CUF(interp_update<T>((const T*)z->u, xo, xn, s->v, s->f, s->m, s->tf, nullptr, rec, a, s->err, s->st,
+    CUF(interp_update<T>((const T*)z->u, xo, xn, s->v, s->f, s->m, s->tf, rec, a, s->err, s->st,
                          &s->tslots));
     prof_mark(s, "interp_update", false);
     // The forces at x^{n+1} need only the positions just written: they run on

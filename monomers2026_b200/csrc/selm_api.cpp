@@ -918,7 +918,7 @@ static int plain_body(selm_sim* s, bool side) {
   if (s->M > 0) {
     WRec<double>* rec = static_cast<WRec<double>*>(s->wrec);
     prof_mark(s, "interp_update", true);
-    CU(interp_update<double>(s->u64[s->cu], xo, xn, s->v, s->f, s->m, s->tf, nullptr, rec, a, s->err, s->st,
+    CU(interp_update<double>(s->u64[s->cu], xo, xn, s->v, s->f, s->m, s->tf, rec, a, s->err, s->st,
                              &s->tslots));
     prof_mark(s, "interp_update", false);
     if (forces) {

@@ -176,8 +176,8 @@ struct CouplingArgs {
 };
 template <typename T>
 cudaError_t interp_update(const T* u, const double* x_old, double* x_new, double* v, double* f, const double* m,
-                          double* tf, const int* order, WRec<T>* rec, const CouplingArgs& a, uint32_t* err,
-                          cudaStream_t st, const TileSlots* ts = nullptr);
+                          double* tf, WRec<T>* rec, const CouplingArgs& a, uint32_t* err, cudaStream_t st,
+                          const TileSlots* ts = nullptr);
 // decomposed instance: the slab's part of the interpolation, and the update
 // from the interpolation summed over the slabs
 template <typename T>
@@ -213,8 +213,8 @@ template <typename T>
 cudaError_t qs_prepare(const double* x, const double* f, double* tf, WRec<T>* rec, const CouplingArgs& a,
                        double inv_dv, cudaStream_t st, const TileSlots* ts, uint32_t* err);
 template <typename T>
-cudaError_t qs_move(const T* u, const double* x_old, double* x_new, double* v, const CouplingArgs& a, uint32_t* err,
-                    cudaStream_t st);
+cudaError_t qs_move(const T* u, const double* x_old, double* x_new, double* v, const WRec<T>* rec, const CouplingArgs& a,
+                    uint32_t* err, cudaStream_t st);
 
 struct ForceTopo {
   int M, ntypes;
