@@ -279,20 +279,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
   const int nz = p.z.n, nl = p.nl, wb = p.wb;
   C* A = reinterpret_cast<C*>(smem_raw);
   C* tw = A + nz * nl;
-  int* pos = reinterpret_cast<int*>(tw + nz);  // nz positions
-  int* coli = pos + nz;                        // the columns' (i, j)
-  int* colj = coli + wb;
+  ColSym<T>* col = reinterpret_cast<ColSym<T>*>(tw + nz);
+  PlaneSym<T>* pz = reinterpret_cast<PlaneSym<T>*>(col + wb);
+  int* pos = reinterpret_cast<int*>(pz + nz);  // nz positions
   const long plane = (long)g.ny * g.nxh, col0 = (long)blockIdx.x * wb;
   const int wn = (int)min((long)wb, plane - col0);
   for (int t = threadIdx.x; t < nz; t += blockDim.x) {
     tw[t] = twz[t];
     pos[t] = mode_pos(p.z, t);
+    pz[t] = plane_sym<T>(g, t, symz);
   }
-  if (threadIdx.x < wn) {
-    const int col = (int)col0 + threadIdx.x;
-    colj[threadIdx.x] = col / g.nxh;
-    coli[threadIdx.x] = col - colj[threadIdx.x] * g.nxh;
-  }
+  if (threadIdx.x < wn) col[threadIdx.x] = col_sym<T>(g, col0 + threadIdx.x, symx, symy);
   __syncthreads();
   z_load_forward<T>(p, work, plane, col0, wn, tw, A);
   __syncthreads();
@@ -302,8 +299,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
     const int k = div_by(p.dwb, u), w = u - k * wb;
     if (w >= wn) continue;
     C* a = A + pos[k] * nl + w;
-    mode_update<T, true>(g, mc, nz, coli[w], colj[w], k, symx, symy, symz, uhat + (long)k * plane + col0 + w,
-                   (long)nz * plane, a, wb);
+    mode_update<T, true>(g, mc, nz, col[w], pz[k], k, uhat + (long)k * plane + col0 + w, (long)nz * plane, a, wb);
   }
   __syncthreads();
   z_inverse_store<T>(p, work, plane, col0, wn, tw, A);

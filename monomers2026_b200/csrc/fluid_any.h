@@ -150,7 +150,11 @@ template <typename T> bool any_plan(int n, AnyPlan* out) {
   p.xy.drp = fast_div(p.xy.rp);
   // z: columns of 128 bytes (16 FP32, 8 FP64), fewer where three (FP32) or two blocks would not fit on an SM
   p.z.wb = sizeof(T) == 4 ? 16 : 8;
-  auto bytes = [&](int wb) { return sizeof(cpx<T>) * ((size_t)n * 3 * wb + n) + sizeof(int) * (size_t)(n + 2 * wb); };
+  // (columns, twiddles, symbols of columns and planes, positions)
+  auto bytes = [&](int wb) {
+    return sizeof(cpx<T>) * ((size_t)n * 3 * wb + n) + sizeof(ColSym<T>) * (size_t)wb +
+           (sizeof(PlaneSym<T>) + sizeof(int)) * (size_t)n;
+  };
   while (p.z.wb > 4 && bytes(p.z.wb) > kSmBytes / (sizeof(T) == 4 ? 3 : 2) - 1024) p.z.wb /= 2;
   p.smem_z = bytes(p.z.wb);
   if (p.smem_z > kSmBytes) return false;

@@ -24,53 +24,68 @@ namespace selm {
 template <int N1, int N2> __device__ __forceinline__ int dpos(int k) { return N2 * (k % N1) + k / N1; }
 
 // ---------------------------------------------------------------- z pencils + update
-// reference noise draw of a half-spectrum mode (cuda/SELM_Kernel.cu:56-79); the
-// amplitude sqrt(lambda_h) comes from the symbol tables (cm = cos - 1).  The
-// FP64 forms draw FP64 normals (same stream as the plain form) and scale them
-// in FP64; the caller multiplies by the prefactor noise_amp.  The FP32 form
-// draws FP32 normals from the same Philox counters (philox_normal2_f32, the
-// FP64 normals to FP32 precision) and scales them by the whole per-mode
-// amplitude noise_amp sqrt(lambda_h) (times 1/sqrt 2 for a complex draw),
-// which is formed in FP64 and rounded to FP32 once: the noise-variance
-// prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).  MID (FP32): the
-// normals to 1e-10 instead (philox_normal2_mid), scaled in FP64 and rounded once.
+template <typename T>
+__device__ __forceinline__ ColSym<T> col_sym(const ZGeom& g, long col, const double* __restrict__ symx,
+                                             const double* __restrict__ symy) {
+  ColSym<T> s;
+  s.j = (int)(col / g.nxh);
+  s.i = (int)(col - (long)s.j * g.nxh);
+  const T idx1 = (T)(1.0 / g.dx);
+  s.c = symx[2 * s.i] + symy[2 * s.j];
+  s.dx = fftk::mk<cpx<T>>((T)symx[2 * s.i] * idx1, (T)symx[2 * s.i + 1] * idx1);
+  s.dy = fftk::mk<cpx<T>>((T)symy[2 * s.j] * idx1, (T)symy[2 * s.j + 1] * idx1);
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ PlaneSym<T> plane_sym(const ZGeom& g, int k, const double* __restrict__ symz) {
+  const T idx1 = (T)(1.0 / g.dx);
+  return PlaneSym<T>{symz[2 * k], fftk::mk<cpx<T>>((T)symz[2 * k] * idx1, (T)symz[2 * k + 1] * idx1)};
+}
+
+// (T)(1 / a) and sqrt(a), a > 0: FP64, or for an FP32 result an FP32
+// approximation with a Newton step in FP64 (1e-14 before the rounding to FP32)
+template <typename T> __device__ __forceinline__ T recip_of(double a) {
+  if constexpr (sizeof(T) == 8) return 1.0 / a;
+  const double q = (double)__frcp_rn((float)a);
+  return (T)fma(q, fma(-a, q, 1.0), q);
+}
+template <typename T> __device__ __forceinline__ double sqrt_of(double a) {
+  if constexpr (sizeof(T) == 8) return sqrt(a);
+  const double q = (double)rsqrtf((float)a), h = a * q;
+  return fma(fma(-h, h, a), 0.5 * q, h);
+}
+
+// reference noise draw of a half-spectrum mode (cuda/SELM_Kernel.cu:56-79).
+// The FP64 forms draw FP64 normals (same stream as the plain form) and scale
+// them in FP64 by coef = sqrt(lambda_h); the caller multiplies by the prefactor
+// noise_amp.  The FP32 form draws FP32 normals from the same Philox counters
+// (philox_normal2_f32, the FP64 normals to FP32 precision) and scales them by
+// the whole per-mode amplitude coef = noise_amp sqrt(lambda_h) (times 1/sqrt 2
+// for a complex draw), which is formed in FP64 and rounded to FP32 once: the
+// noise-variance prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).
+// MID (FP32): the normals to 1e-10 instead (philox_normal2_mid), scaled in FP64
+// and rounded once.
 template <typename T, bool MID>
-__device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int nz, int i, int j, int k, double cmx,
-                                                double cmy, double cmz, cpx<T> out[3]) {
-  const int k1 = (k == 0) ? 0 : nz - k, j1 = (j == 0) ? 0 : g.ny - j, i1 = (i == 0) ? 0 : g.nx - i;
-  const bool selfc = (k1 == k && j1 == j && i1 == i);
+__device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int nz, int i, int j, int k, double coef,
+                                                cpx<T> out[3]) {
+  const bool selfc = (k == 0 || 2 * k == nz) && (j == 0 || 2 * j == g.ny) && (i == 0 || 2 * i == g.nx);
   const uint32_t q = (uint32_t)(((long)k * g.ny + j) * g.nxh + i);
-  if constexpr (sizeof(T) == 8) {
-    const double lam = -2.0 * (cmx + cmy + cmz) / (g.dx * g.dx);
-    const double coef = sqrt(fmax(lam, 0.0));
-    const double re = selfc ? coef : coef * 0.7071067811865476;
-    const double im = selfc ? 0.0 : re;
+  const double re = selfc ? coef : coef * 0.7071067811865476, im = selfc ? 0.0 : re;
+  const T ret = (T)re, imt = (T)im;
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
+  for (int d = 0; d < 3; d++) {
+    if constexpr (sizeof(T) == 8) {
       double z0, z1;
       philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
       out[d] = make_double2(z0 * re, z1 * im);
-    }
-  } else {
-    const double lam = -2.0 * (cmx + cmy + cmz) * g.idx2;
-    const double amp = g.noise_amp * sqrt(fmax(lam, 0.0));
-    if constexpr (MID) {
-      const double re = selfc ? amp : amp * 0.7071067811865476, im = selfc ? 0.0 : re;
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        double z0, z1;
-        philox_normal2_mid(g.rk, q, (uint32_t)d, step, z0, z1);
-        out[d] = make_float2((float)(z0 * re), (float)(z1 * im));
-      }
+    } else if constexpr (MID) {
+      double z0, z1;
+      philox_normal2_mid(g.rk, q, (uint32_t)d, step, z0, z1);
+      out[d] = make_float2((float)(z0 * re), (float)(z1 * im));
     } else {
-      const float re = (float)(selfc ? amp : amp * 0.7071067811865476);
-      const float im = selfc ? 0.0f : re;
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        float z0, z1;
-        philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
-        out[d] = make_float2(z0 * re, z1 * im);
-      }
+      float z0, z1;
+      philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
+      out[d] = make_float2(z0 * ret, z1 * imt);
     }
   }
 }
@@ -78,11 +93,11 @@ __device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, i
 // constants of the spectral update
 template <typename T> struct ModeConsts {
   uint64_t step;
-  double idx2;
-  T invN, idx1, irho;
+  double idx2, visc;  // 1/dx^2, mu dt / rho
+  T invN, irho;
 };
 template <typename T> __device__ __forceinline__ ModeConsts<T> mode_consts(const ZGeom& g, int nz) {
-  return ModeConsts<T>{*g.step, 1.0 / (g.dx * g.dx), (T)(1.0 / ((double)g.nx * g.ny * nz)), (T)(1.0 / g.dx),
+  return ModeConsts<T>{*g.step, 1.0 / (g.dx * g.dx), g.mu * g.dt / g.rho, (T)(1.0 / ((double)g.nx * g.ny * nz)),
                        (T)(1.0 / g.rho)};
 }
 
@@ -90,29 +105,27 @@ template <typename T> __device__ __forceinline__ ModeConsts<T> mode_consts(const
 // transformed forcing at a[c astep] is replaced by the new velocity over N,
 // u_hat (component c at uh[c cplane]) by the new velocity.  MID: the
 // FP32 form's normals to 1e-10 (noise_draw_fast).
-template <typename T, bool MID = false>
-__device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>& mc, int nz, int i, int j, int k,
-                                            const double* __restrict__ symx, const double* __restrict__ symy,
-                                            const double* __restrict__ symz, cpx<T>* __restrict__ uh, long cplane,
+template <typename T, bool MID>
+__device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>& mc, int nz, const ColSym<T>& col,
+                                            const PlaneSym<T>& pz, int k, cpx<T>* __restrict__ uh, long cplane,
                                             cpx<T>* a, int astep) {
   using C = cpx<T>;
-  const int ny = g.ny;
-  const double idx2 = mc.idx2;
-  const T idx1 = mc.idx1;
+  const int i = col.i, j = col.j, ny = g.ny;
+  const double Lk = 2.0 * (col.c + pz.c) * mc.idx2;  // sum_d 2(cos - 1)/dx^2 (<= 0)
   C X[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) X[c] = a[c * astep];
-  const double cx = symx[2 * i], sx = symx[2 * i + 1];
-  const double cy = symy[2 * j], sy = symy[2 * j + 1];
-  const double cz = symz[2 * k], sz = symz[2 * k + 1];
-  if (g.stochastic) {
+  const bool zero = i == 0 && j == 0 && k == 0;
+  if (g.stochastic && !zero) {  // (the zero mode's draw has amplitude 0)
+    double coef = sqrt_of<T>(-Lk);
+    if (sizeof(T) == 4) coef *= g.noise_amp;
     C Xn[3];
-    noise_draw_fast<T, MID>(g, mc.step, nz, i, j, k, cx, cy, cz, Xn);
-    if (i == 0 || ((g.nx & 1) == 0 && i == g.nx / 2)) {
+    noise_draw_fast<T, MID>(g, mc.step, nz, i, j, k, coef, Xn);
+    if (i == 0 || 2 * i == g.nx) {
       const int jc = (j == 0) ? 0 : ny - j, kc = (k == 0) ? 0 : nz - k;
       if (jc != j || kc != k) {
         C Xc[3];
-        noise_draw_fast<T, MID>(g, mc.step, nz, i, jc, kc, cx, symy[2 * jc], symz[2 * kc], Xc);
+        noise_draw_fast<T, MID>(g, mc.step, nz, i, jc, kc, coef, Xc);
         const T s = (g.noise_mode == 1 || g.qs) ? T(0.7071067811865476) : T(0.5);
 #pragma unroll
         for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<C>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
@@ -137,18 +150,16 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
     }
   }
   C un[3];
-  if (i == 0 && j == 0 && k == 0) {
+  const C D[3] = {col.dx, col.dy, pz.d};
+  if (zero) {
 #pragma unroll
     for (int c = 0; c < 3; c++) un[c] = fftk::mk<C>(T(0), T(0));
   } else if (g.qs) {
     // steady Stokes: u_hat = P f_hat / (mu lambda_h), lambda_h = -L_h > 0
-    const double Lk = 2.0 * (cx + cy + cz) * idx2;
-    const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
-                    fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
     C s = cmul(D[0], X[0]);
     s = cadd(s, cmul(D[1], X[1]));
     s = cadd(s, cmul(D[2], X[2]));
-    const T iL = (T)(1.0 / Lk), imuL = (T)(-1.0 / (g.mu * Lk));
+    const T iL = recip_of<T>(Lk), imuL = -recip_of<T>(g.mu * Lk);
     s = fftk::mk<C>(s.x * iL, s.y * iL);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -156,20 +167,17 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
       un[c] = fftk::mk<C>(pf.x * imuL, pf.y * imuL);
     }
   } else {
-    const double Lk = 2.0 * (cx + cy + cz) * idx2;
-    const T visc = (T)(1.0 + g.mu * g.dt * Lk / g.rho);
+    const T visc = (T)fma(mc.visc, Lk, 1.0);
     C us[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const C q = uh[c * cplane];
       us[c] = fftk::mk<C>(q.x * visc + X[c].x * mc.irho, q.y * visc + X[c].y * mc.irho);
     }
-    const C D[3] = {fftk::mk<C>((T)cx * idx1, (T)sx * idx1), fftk::mk<C>((T)cy * idx1, (T)sy * idx1),
-                    fftk::mk<C>((T)cz * idx1, (T)sz * idx1)};
     C s = cmul(D[0], us[0]);
     s = cadd(s, cmul(D[1], us[1]));
     s = cadd(s, cmul(D[2], us[2]));
-    const T iL = (T)(1.0 / Lk);
+    const T iL = recip_of<T>(Lk);
     s = fftk::mk<C>(s.x * iL, s.y * iL);
 #pragma unroll
     for (int c = 0; c < 3; c++) un[c] = csub(us[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
@@ -250,11 +258,11 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   C* A = reinterpret_cast<C*>(TMA ? ((reinterpret_cast<uintptr_t>(zsmem_raw) + 127) & ~(uintptr_t)127)
                                   : reinterpret_cast<uintptr_t>(zsmem_raw));
   C* tw = A + N * NL;
-  const int nxh = g.nxh, ny = g.ny;
   const long col0 = (long)blockIdx.x * WB;
-  const long plane = g.ncol ? g.ncol : (long)ny * nxh;
+  const long plane = g.ncol ? g.ncol : (long)g.ny * g.nxh;
   const int wn = (int)min((long)WB, plane - col0);
-  __shared__ int coli[WB], colj[WB];  // (i, j) of the block's columns
+  __shared__ ColSym<T> col[WB];
+  __shared__ PlaneSym<T> pz[N];
   __shared__ __align__(8) unsigned long long zbar;
   if constexpr (TMA) {
     if (threadIdx.x == 0) {
@@ -262,12 +270,11 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
       zbar_load(A, &tmap, &zbar, (unsigned)(sizeof(C) * N * NL), (int)col0, 0, 0);
     }
   }
-  for (int t = threadIdx.x; t < N; t += blockDim.x) tw[t] = twz[t];
-  if (threadIdx.x < wn) {
-    const int col = (int)(g.c0 + col0) + threadIdx.x;
-    colj[threadIdx.x] = col / nxh;
-    coli[threadIdx.x] = col - colj[threadIdx.x] * nxh;
+  for (int t = threadIdx.x; t < N; t += blockDim.x) {
+    tw[t] = twz[t];
+    pz[t] = plane_sym<T>(g, t, symz);
   }
+  if (threadIdx.x < wn) col[threadIdx.x] = col_sym<T>(g, g.c0 + col0 + threadIdx.x, symx, symy);
   __syncthreads();
   if constexpr (TMA) {
     // one thread polls (bounded) and tells the block, so that all of it goes on or stops
@@ -313,8 +320,8 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   for (int u = threadIdx.x; u < WB * N; u += blockDim.x) {
     const int w = u % WB, k = u / WB;
     if (w >= wn) continue;
-    mode_update<T, MID>(g, mc, N, coli[w], colj[w], k, symx, symy, symz, uhat + (long)k * plane + col0 + w,
-                   (long)N * plane, A + dpos<N1, N2>(k) * NL + w, WB);
+    mode_update<T, MID>(g, mc, N, col[w], pz[k], k, uhat + (long)k * plane + col0 + w, (long)N * plane,
+                        A + dpos<N1, N2>(k) * NL + w, WB);
   }
   __syncthreads();
   // pass B inverse in place: thread (line, k1)

@@ -84,6 +84,18 @@ struct ZGeom {
   uint32_t* err = nullptr;  // status word (a TMA copy that timed out)
 };
 
+// Symbols of a column (i, j) and of a z plane k, worked out once per block:
+// c = (cos theta_x - 1) + (cos theta_y - 1) and cos theta_z - 1 in FP64, the
+// forward-difference symbols D = (cos theta - 1 + i sin theta)/dx in T.
+template <typename T> struct ColSym {
+  double c;
+  cpx<T> dx, dy;
+  int i, j;
+};
+template <typename T> struct PlaneSym {
+  double c;
+  cpx<T> d;
+};
 // ---- binning (counting sort of monomers into buckets, deterministic order)
 struct BinSpec {
   int mode;      // 0: grid tiles (cell = floor((x-lo)/dx), bucket = cell / tile), 1: cells of size L/nc,
