@@ -35,6 +35,9 @@ unsigned long long launches_total() { return g_launches.load(); }
 
 extern "C" unsigned long long selm_kernel_launches(void) { return g_launches.load(); }
 
+static void stage_sim_created();
+static void stage_sim_destroyed();
+
 int selm_fail(int code, const std::string& msg) {
   g_err = msg;
   return code;
@@ -239,6 +242,7 @@ extern "C" int selm_create(const selm_params* params, selm_sim** out) {
   int rc = validate(params);
   if (rc) return rc;
   selm_sim* s = new selm_sim();
+  stage_sim_created();
   s->prm = *params;
   s->nx = params->num_mesh_pts[0];
   s->ny = params->num_mesh_pts[1];
@@ -249,6 +253,7 @@ extern "C" int selm_create(const selm_params* params, selm_sim** out) {
   s->hi = params->box_hi;
   s->dx = (s->hi - s->lo) / s->nx;  // cuda/SELM_Eulerian_Period.cu:18
   if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
+    stage_sim_destroyed();
     delete s;
     return selm_fail(SELM_ERR_CUDA, "cudaStreamCreate failed");
   }
@@ -280,6 +285,7 @@ extern "C" int selm_slab_create(const selm_params* params, int rank, int nranks,
     return selm_fail(SELM_ERR_INVALID, "a decomposed instance needs a compile-time FFT size that splits into "
                                        "whole 16-plane tile layers per rank");
   selm_sim* s = new selm_sim();
+  stage_sim_created();
   s->prm = *params;
   s->nx = s->ny = s->nz = n;
   s->N = (long)n * n * n;
@@ -295,6 +301,7 @@ extern "C" int selm_slab_create(const selm_params* params, int rank, int nranks,
   s->slab.c0 = std::min(ncol, rank * per);
   s->slab.ncl = std::min(ncol, s->slab.c0 + per) - s->slab.c0;
   if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess) {
+    stage_sim_destroyed();
     delete s;
     return selm_fail(SELM_ERR_CUDA, "cudaStreamCreate failed");
   }
@@ -1085,15 +1092,83 @@ extern "C" int selm_destroy(selm_sim* s) {
   if (s->ev_committed) cudaEventDestroy(s->ev_committed);
   if (s->ev_ready) cudaEventDestroy(s->ev_ready);
   if (s->st_copy) cudaStreamDestroy(s->st_copy);
+  stage_sim_destroyed();
   delete s;
   return SELM_OK;
 }
 
 // ---------------------------------------------------------------- access
+// Page-locked staging for read-backs of few monomers into pageable arrays: a
+// pageable device-to-host copy is a round trip of its own, three a call (65 us
+// for 1000 monomers, of which 48 replicas of an ensemble paid 48), while three
+// copies into one page-locked buffer are queued together and waited for once.
+// Above kStageMonomers the copy out of the buffer costs what it saves.  The
+// buffers are shared by the process' simulations: a call takes one (or makes
+// one) and gives it back, at most kStageKept are kept, and the last
+// simulation's destruction frees them.
+namespace {
+constexpr int kStageMonomers = 8192, kStageKept = 8;
+constexpr size_t kStageBytes = sizeof(double) * 9 * kStageMonomers;
+std::mutex g_stage_mu;
+std::vector<double*> g_stage_free;
+int g_stage_sims = 0;
+
+struct StageBuffer {
+  double* p = nullptr;
+  StageBuffer() {
+    {
+      std::lock_guard<std::mutex> lk(g_stage_mu);
+      if (!g_stage_free.empty()) {
+        p = g_stage_free.back();
+        g_stage_free.pop_back();
+        return;
+      }
+    }
+    if (cudaHostAlloc((void**)&p, kStageBytes, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~StageBuffer() {
+    if (!p) return;
+    {
+      std::lock_guard<std::mutex> lk(g_stage_mu);
+      if (g_stage_sims > 0 && (int)g_stage_free.size() < kStageKept) {
+        g_stage_free.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+  StageBuffer(const StageBuffer&) = delete;
+  StageBuffer& operator=(const StageBuffer&) = delete;
+};
+
+bool pageable(const void* q) {
+  cudaPointerAttributes at{};
+  const bool known = cudaPointerGetAttributes(&at, q) == cudaSuccess;
+  if (!known) cudaGetLastError();
+  return !known || at.type == cudaMemoryTypeUnregistered;
+}
+}  // namespace
+
+static void stage_sim_created() {
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  g_stage_sims++;
+}
+static void stage_sim_destroyed() {
+  std::vector<double*> gone;
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (--g_stage_sims == 0) gone.swap(g_stage_free);
+  }
+  for (double* p : gone) cudaFreeHost(p);
+}
+
 extern "C" int selm_get_particles(selm_sim* s, double* x, double* v, double* f) {
   if (!s) return selm_fail(SELM_ERR_INVALID, "sim is NULL");
   if (s->M == 0) return SELM_OK;
-  const size_t b = sizeof(double) * 3 * s->M;
+  const size_t n = 3 * (size_t)s->M, b = sizeof(double) * n;
   // right after a graph step: copy once the step's monomer state is final,
   // while the spread and the fluid solve of that step still run
   cudaStream_t cs = s->st;
@@ -1103,12 +1178,31 @@ extern "C" int selm_get_particles(selm_sim* s, double* x, double* v, double* f) 
     CU(cudaStreamWaitEvent(s->st_copy, s->ev_xv, 0));
     cs = s->st_copy;
   }
-  if (x) CU(cudaMemcpyAsync(x, s->x[s->cx], b, cudaMemcpyDeviceToHost, cs));
-  if (v) CU(cudaMemcpyAsync(v, s->v, b, cudaMemcpyDeviceToHost, cs));
-  if (early) CU(cudaStreamWaitEvent(cs, s->ev_ready, 0));  // f: after the side-stream forces
-  if (f) CU(cudaMemcpyAsync(f, s->f, b, cudaMemcpyDeviceToHost, cs));
-  CU(cudaStreamSynchronize(cs));
-  return SELM_OK;
+  auto copies = [&](double* cx, double* cv, double* cf) -> int {
+    if (cx) CU(cudaMemcpyAsync(cx, s->x[s->cx], b, cudaMemcpyDeviceToHost, cs));
+    if (cv) CU(cudaMemcpyAsync(cv, s->v, b, cudaMemcpyDeviceToHost, cs));
+    if (early) CU(cudaStreamWaitEvent(cs, s->ev_ready, 0));  // f: after the side-stream forces
+    if (cf) CU(cudaMemcpyAsync(cf, s->f, b, cudaMemcpyDeviceToHost, cs));
+    CU(cudaStreamSynchronize(cs));
+    return SELM_OK;
+  };
+  const double* some = x ? x : v ? v : f;
+  if (s->M <= kStageMonomers && some && pageable(some)) {
+    StageBuffer sb;
+    if (sb.p) {
+      double *sx = x ? sb.p : nullptr, *sv = v ? sb.p + n : nullptr, *sf = f ? sb.p + 2 * n : nullptr;
+      const int rc = copies(sx, sv, sf);
+      if (rc) {
+        cudaStreamSynchronize(cs);  // nothing still writes the buffer
+        return rc;
+      }
+      if (x) memcpy(x, sx, b);
+      if (v) memcpy(v, sv, b);
+      if (f) memcpy(f, sf, b);
+      return SELM_OK;
+    }
+  }
+  return copies(x, v, f);
 }
 
 extern "C" int selm_get_coupling_impulse(selm_sim* s, double* tf, double* dt) {
