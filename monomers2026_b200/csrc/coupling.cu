@@ -1164,9 +1164,9 @@ constexpr int kHomeWarps = kHomeThreads / 32;
 constexpr int kHomeSplitK = 11;  // single-word path for n <= 2^11
 static_assert(kHX % 32 == 20 && (kHX * kHY) % 32 == 16, "bank pattern of the box atomics");
 static_assert(kHBox <= 65536, "box slots of the stencil records are 16-bit");
-constexpr int kHomeStage = 112;  // candidates staged in shared memory at a time (three blocks per SM)
+constexpr int kHomeStage = 128;  // candidates staged in shared memory at a time (three blocks per SM)
 constexpr size_t kHomeBoxBytes = sizeof(unsigned) * 3 * kHBox;  // 57,600 B
-constexpr size_t kHomeSmem = kHomeBoxBytes + kHomeStage * (sizeof(WRec<float>) + 3 * sizeof(double));  // 74,624 B
+constexpr size_t kHomeSmem = kHomeBoxBytes + kHomeStage * sizeof(WRec<float>);  // 73,984 B
 static_assert(sizeof(WRec<float>) % 16 == 0 && kHomeBoxBytes % 16 == 0, "16-byte staging copies");
 
 // 16- and 8-byte asynchronous copies global -> shared (LDGSTS), and the wait for all of this thread's
@@ -1180,6 +1180,43 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// One staged candidate: the first 96 bytes of its record (the weights), and in
+// place of the bases its impulses at the tile's scale (FP32) and box slots.
+struct HomeCand {
+  float w[3][2][4];
+  float t[3];
+  unsigned pad;
+  uint2 hs;
+  uint2 pad2;
+};
+static_assert(sizeof(HomeCand) == sizeof(WRec<float>) && offsetof(WRec<float>, hs) == 120, "staged records");
+
+// The staged candidates 0 .. nc-1: a warp each, lane l adding the points
+// (l & 3, (l >> 2) & 3, l >> 4) and two z-planes apart of all three components.
+__device__ __forceinline__ void home_add_staged(const HomeCand* __restrict__ cand, int nc, unsigned* acc) {
+  const int lane = threadIdx.x & 31;
+  const int ix = lane & 3, jy = (lane >> 2) & 3, kz = lane >> 4;
+  unsigned* base = acc + (kz * kHY + jy) * kHX + ix;
+#pragma unroll 2
+  for (int c = threadIdx.x >> 5; c < nc; c += kHomeWarps) {
+    const HomeCand& R = cand[c];
+    const float4 t = *reinterpret_cast<const float4*>(R.t);
+    const uint2 h = R.hs;
+    const float wx[2] = {R.w[0][0][ix], R.w[0][1][ix]}, wy[2] = {R.w[1][0][jy], R.w[1][1][jy]};
+    const float wz[2][2] = {{R.w[2][0][kz], R.w[2][0][kz + 2]}, {R.w[2][1][kz], R.w[2][1][kz + 2]}};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const int sx = (d != 0), sy = (d != 1), sz = (d != 2);
+      const float A = (d == 0 ? t.x : d == 1 ? t.y : t.z) * wy[sy] * wx[sx];
+      const unsigned slot = d * kHBox + (d == 0 ? (h.x & 0xffffu) : d == 1 ? (h.x >> 16) : (h.y & 0xffffu));
+      atomicAdd(base + slot, (unsigned)round_small(A * wz[sz][0]));
+      atomicAdd(base + slot + 2 * kHY * kHX, (unsigned)round_small(A * wz[sz][1]));
+    }
+  }
+}
+
+// Candidates taken from memory: the entries of the overflow list (SPLIT 0), or
+// every candidate of a tile on the split path, one component at a time.
 template <int SPLIT>
 __device__ __forceinline__ void home_add(const int* __restrict__ ids, int n_prim, int n_ovf, const TileSlots& ts, int tb,
                                          int dsel, double scale, int L, unsigned* acc,
@@ -1187,44 +1224,9 @@ __device__ __forceinline__ void home_add(const int* __restrict__ ids, int n_prim
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int ix = lane & 3, jy = (lane >> 2) & 3, kz = lane >> 4;
   const int loff = (kz * kHY + jy) * kHX + ix;
-  auto one2 = [&](int p0, int p1, bool two) {
-    const WRec<float>& R0 = rec[p0];
-    const WRec<float>& R1 = rec[two ? p1 : p0];
-    const uint2 h0 = *reinterpret_cast<const uint2*>(&R0.hs[0]);  // hs[0..2] and two bytes of padding
-    const uint2 h1 = *reinterpret_cast<const uint2*>(&R1.hs[0]);
-    float wxa[2][2], wya[2][2], wza[2][2][2];
-    float wxb[2][2], wyb[2][2], wzb[2][2][2];
-#pragma unroll
-    for (int sh = 0; sh < 2; sh++) {
-      wxa[sh][0] = R0.w[0][sh][ix]; wya[sh][0] = R0.w[1][sh][jy];
-      wza[sh][0][0] = R0.w[2][sh][kz]; wza[sh][0][1] = R0.w[2][sh][kz + 2];
-      wxb[sh][0] = R1.w[0][sh][ix]; wyb[sh][0] = R1.w[1][sh][jy];
-      wzb[sh][0][0] = R1.w[2][sh][kz]; wzb[sh][0][1] = R1.w[2][sh][kz + 2];
-    }
-    double t0[3], t1[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      t0[d] = tf[3L * p0 + d];
-      t1[d] = two ? tf[3L * p1 + d] : 0.0;
-    }
-    auto add = [&](const uint2 hsw, const float (&wx)[2][2], const float (&wy)[2][2], const float (&wz)[2][2][2],
-                   const double (&tv)[3]) {
-      const unsigned short* hs = reinterpret_cast<const unsigned short*>(&hsw);
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const int sx = (d != 0), sy = (d != 1), sz = (d != 2);
-        const float A = (float)(-tv[d] * scale) * wy[sy][0] * wx[sx][0];
-        const int slot = d * kHBox + hs[d] + loff;
-        atomicAdd(acc + slot, (unsigned)round_small(A * wz[sz][0][0]));
-        atomicAdd(acc + slot + 2 * kHY * kHX, (unsigned)round_small(A * wz[sz][0][1]));
-      }
-    };
-    add(h0, wxa, wya, wza, t0);
-    if (two) add(h1, wxb, wyb, wzb, t1);
-  };
   auto one = [&](int p) {
     const WRec<float>& R = rec[p];
-    const uint2 hsw = *reinterpret_cast<const uint2*>(&R.hs[0]);
+    const uint2 hsw = *reinterpret_cast<const uint2*>(&R.hs[0]);  // hs[0..2] and two bytes of padding
     const unsigned short* hs = reinterpret_cast<const unsigned short*>(&hsw);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -1254,24 +1256,7 @@ __device__ __forceinline__ void home_add(const int* __restrict__ ids, int n_prim
       }
     }
   };
-  if (!SPLIT) {
-    // two candidates per pass (their loads overlap), the next pair's indices loaded ahead
-    int c = wid;
-    // (ids null: the candidates are the records 0 .. n_prim-1 themselves, staged in shared memory)
-    auto id = [&](int q) { return ids ? ids[q] : q; };
-    int pa = (c < n_prim) ? id(c) : 0;
-    int pb = (c + kHomeWarps < n_prim) ? id(c + kHomeWarps) : 0;
-    while (c < n_prim) {
-      const int p0 = pa, p1 = pb;
-      const bool two = c + kHomeWarps < n_prim;
-      c += 2 * kHomeWarps;
-      if (c < n_prim) pa = id(c);
-      if (c + kHomeWarps < n_prim) pb = id(c + kHomeWarps);
-      one2(p0, p1, two);
-    }
-  } else {
-    for (int c = wid; c < n_prim; c += kHomeWarps) one(ids[c]);
-  }
+  for (int c = wid; c < n_prim; c += kHomeWarps) one(ids[c]);
   for (int q = wid; q < n_ovf; q += kHomeWarps) {
     const int2 e = ts.ovf[q];
     if (e.x == tb) one(e.y);
@@ -1281,9 +1266,7 @@ __device__ __forceinline__ void home_add(const int* __restrict__ ids, int n_prim
 __global__ void __launch_bounds__(kHomeThreads, 3) k_spread_home(const double* __restrict__ tf, TileSlots ts,
                                                                  const WRec<float>* __restrict__ rec) {
   extern __shared__ __align__(16) unsigned hacc[];  // [3][kHZ][kHY][kHX], or [2][kHZ][kHY][kHX] (split path)
-  // the staged candidates: their records and impulses
-  WRec<float>* srec = reinterpret_cast<WRec<float>*>(reinterpret_cast<unsigned char*>(hacc) + kHomeBoxBytes);
-  double* stf = reinterpret_cast<double*>(srec + kHomeStage);
+  HomeCand* cand = reinterpret_cast<HomeCand*>(reinterpret_cast<unsigned char*>(hacc) + kHomeBoxBytes);
   const int tb = blockIdx.x, tid = threadIdx.x;
   const int n = ts.count[tb];
   const int n_prim = min(n, ts.cap);
@@ -1306,19 +1289,27 @@ __global__ void __launch_bounds__(kHomeThreads, 3) k_spread_home(const double* _
       if (k <= kHomeSplitK) {
         const int S = max(-1000, min(1000, min(30 - k, 22) - em - ew));
         const double scale = ldexp(1.0, S);
-        // the candidates' records and impulses go to shared memory in chunks,
-        // each by asynchronous copies that every thread issues at once (the
-        // first chunk's while the box is zeroed), so that their load latency
-        // is paid once per chunk rather than once per candidate pair
+        // The candidates' records go to shared memory in chunks, the weights and
+        // slots by asynchronous copies that every thread issues at once (the
+        // first chunk's while the box is zeroed), so that their load latency is
+        // paid once per chunk; the impulses are scaled and rounded to FP32 by
+        // the staging thread, once per candidate (every lane of the adding warp
+        // multiplied and converted three FP64 values: 90 instructions a
+        // candidate against 55)
         auto stage = [&](int c0, int nc) {
           for (int i = tid; i < nc * 8; i += kHomeThreads) {
             const int c = i >> 3, q = i & 7;
-            cp_async16(reinterpret_cast<unsigned char*>(srec + c) + 16 * q,
-                       reinterpret_cast<const unsigned char*>(rec + ids[c0 + c]) + 16 * q);
-          }
-          for (int i = tid; i < nc * 3; i += kHomeThreads) {
-            const int c = i / 3, q = i - 3 * c;
-            cp_async8(stf + i, tf + 3L * ids[c0 + c] + q);
+            const int p = ids[c0 + c];
+            unsigned char* dst = reinterpret_cast<unsigned char*>(cand + c);
+            if (q < 6) {
+              cp_async16(dst + 16 * q, reinterpret_cast<const unsigned char*>(rec + p) + 16 * q);
+            } else if (q == 6) {
+              const float t0 = (float)(-tf[3L * p] * scale), t1 = (float)(-tf[3L * p + 1] * scale),
+                          t2 = (float)(-tf[3L * p + 2] * scale);
+              *reinterpret_cast<float4*>(cand[c].t) = make_float4(t0, t1, t2, 0.0f);
+            } else {
+              cp_async8(&cand[c].hs, &rec[p].hs[0]);
+            }
           }
         };
         int c0 = 0, nc = min(kHomeStage, n_prim);
@@ -1327,7 +1318,7 @@ __global__ void __launch_bounds__(kHomeThreads, 3) k_spread_home(const double* _
         for (;;) {
           cp_async_wait_all();
           __syncthreads();  // the chunk and the zeroed box are visible to every thread
-          home_add<0>(nullptr, nc, 0, ts, tb, 0, scale, 0, hacc, stf, srec);
+          home_add_staged(cand, nc, hacc);
           c0 += nc;
           if (c0 >= n_prim) break;
           nc = min(kHomeStage, n_prim - c0);
@@ -1385,83 +1376,91 @@ __global__ void __launch_bounds__(kHomeThreads, 3) k_spread_home(const double* _
   }
 }
 
-// The fold on grids whose sizes are multiples of the tile (every tile full):
-// block per (tile, component), a thread per (x, y) column of the tile that
-// walks its 16 cells along z, so that a half-warp reads 64-byte runs of box
-// rows.  Cell (x, y, z) of tile (tx, ty, tz) lies in the boxes of the tiles
-// (tx + dx, ty + dy, tz + dz): dx = 0 at box column x + 2, dx = -1 (cells
-// 0, 1) at column x + T_x + 2, dx = +1 (cells T_x - 2, T_x - 1) at column
-// x - T_x + 2, and the same along y and z.  Per cell the order of addition is
-// fixed: dz, then dy, then dx, each ascending.  Tiles one or two per axis wrap
-// onto themselves: the same rule holds, with tx-1 and tx+1 naming the same
-// tile.  Every box is written, zeros for a tile without monomers.
+// The fold on grids of 4 m cells along x whose tiles are at least 4 cells wide
+// (a partial last tile included): block per (tile, component), a thread per
+// four x cells of a (y, z) row.  Cell l of a tile of e cells lies in the boxes
+// of its own tile at coordinate l + 2; of the tile below (cells 0, 1) at
+// l + 2 + that tile's e; of the tile above (cells e - 2, e - 1) at l - e + 2:
+// along x two float2 of the tile's own box and, for the first and the last four
+// cells, one of the neighbour's.  Per cell the order of addition is fixed: z,
+// then y, then x, each ascending.  Tiles one or two per axis wrap onto
+// themselves by the same rule.  Every box is written, zeros for a tile without
+// monomers.
+// All loads of a row's boxes are issued before the first is added.  A thread
+// per (x, y) column that walked z with scalar loads, and a thread per cell where
+// the tiles do not divide the grid, took, with the home kernel, 55.5 us at 128^3
+// (49.4 now), 60 at 100^3 (32), 146 at 192^3 (130).  Box rows in memory split
+// into 64-byte tile rows and halo columns were slower (52.6 and 150: the home
+// kernel's writes), so were rows of the z boxes one after another (52.7).
+constexpr int kFoldThreads = 128;
+struct FoldAxis {
+  int t[2], b[2], n;  // tiles, box coordinates of the row, how many
+};
+__device__ __forceinline__ FoldAxis fold_axis(int l, int t, int nb, int T, int n) {
+  FoldAxis f;
+  const int e = min(T, n - t * T);
+  f.t[0] = f.t[1] = t;
+  f.b[0] = f.b[1] = l + 2;
+  f.n = 1;
+  if (l < 2) {
+    const int q = (t == 0 ? nb : t) - 1;
+    f.t[0] = q;
+    f.b[0] = l + 2 + min(T, n - q * T);
+    f.n = 2;
+  } else if (l >= e - 2) {
+    f.t[1] = (t + 1 == nb) ? 0 : t + 1;
+    f.b[1] = l - e + 2;
+    f.n = 2;
+  }
+  return f;
+}
 template <typename T>
-__global__ void __launch_bounds__(kTX * kTY) k_spread_fold_cols(T* __restrict__ f, int accumulate,
+__global__ void __launch_bounds__(kFoldThreads, 8) k_spread_fold4(T* __restrict__ f, int accumulate,
                                                                const float* __restrict__ box, BinSpec bs) {
   const int tb = blockIdx.x, d = blockIdx.y;
-  const int nbx = bs.nb[0], nby = bs.nb[1], nbz = bs.nb[2];
+  const int nbx = bs.nb[0], nby = bs.nb[1], nbz = bs.nb[2], nx = bs.n[0], ny = bs.n[1], nz = bs.n[2];
   const int tx = tb % nbx, ty = (tb / nbx) % nby, tz = tb / (nbx * nby);
-  const int lx = threadIdx.x % kTX, ly = threadIdx.x / kTX;
-  // (tile, box coordinate) along x and y, in ascending order of the offset
-  int xt0 = tx, xc0 = lx + 2, xt1 = tx, xc1 = lx + 2, nxe = 1;
-  if (lx < 2) {
-    xt0 = (tx == 0 ? nbx : tx) - 1;
-    xc0 = lx + kTX + 2;
-    nxe = 2;
-  } else if (lx >= kTX - 2) {
-    xt1 = (tx + 1 == nbx) ? 0 : tx + 1;
-    xc1 = lx - kTX + 2;
-    nxe = 2;
-  }
-  int yt0 = ty, yr0 = ly + 2, yt1 = ty, yr1 = ly + 2, nye = 1;
-  if (ly < 2) {
-    yt0 = (ty == 0 ? nby : ty) - 1;
-    yr0 = ly + kTY + 2;
-    nye = 2;
-  } else if (ly >= kTY - 2) {
-    yt1 = (ty + 1 == nby) ? 0 : ty + 1;
-    yr1 = ly - kTY + 2;
-    nye = 2;
-  }
-  // the (y, x) part of the box offsets: entries (y0, x0), (y0, x1), (y1, x0), (y1, x1)
-  long po[4];
-  bool pu[4];
+  const int ex = min(kTX, nx - tx * kTX), ey = min(kTY, ny - ty * kTY), ez = min(kTZ, nz - tz * kTZ);
+  const int x4 = (threadIdx.x & 3) * 4, y = (threadIdx.x >> 2) & (kTY - 1);
+  if (x4 >= ex || y >= ey) return;
+  const int txl = (tx == 0 ? nbx : tx) - 1, txr = (tx + 1 == nbx) ? 0 : tx + 1;
+  const int xl = min(kTX, nx - txl * kTX) + 2;  // the left tile's box column of cell 0
+  const bool first = x4 == 0, last = x4 + 4 == ex;
+  const FoldAxis fy = fold_axis(y, ty, nby, kTY, ny);
+  for (int z = threadIdx.x >> 5; z < ez; z += kFoldThreads / 32) {
+    const FoldAxis fz = fold_axis(z, tz, nbz, kTZ, nz);
+    float2 a[4], b[4], l[4], r[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int ye = q >> 1, xe = q & 1;
-    pu[q] = ye < nye && xe < nxe;
-    const int t = (ye ? yt1 : yt0) * nbx + (xe ? xt1 : xt0);
-    po[q] = ((long)t * 3 + d) * kHBox + (ye ? yr1 : yr0) * kHX + (xe ? xc1 : xc0);
-  }
-  const long tzs = (long)nbx * nby * 3 * kHBox;  // one tile along z in the box buffer
-  const int nx = bs.n[0], ny = bs.n[1], nz = bs.n[2];
-  T* dst = f + ((long)(d * nz + tz * kTZ) * ny + ty * kTY + ly) * nx + tx * kTX + lx;
-  for (int lz = 0; lz < kTZ; lz++) {
-    int zt0 = tz, zp0 = lz + 2, zt1 = tz, zp1 = lz + 2, nze = 1;
-    if (lz < 2) {
-      zt0 = (tz == 0 ? nbz : tz) - 1;
-      zp0 = lz + kTZ + 2;
-      nze = 2;
-    } else if (lz >= kTZ - 2) {
-      zt1 = (tz + 1 == nbz) ? 0 : tz + 1;
-      zp1 = lz - kTZ + 2;
-      nze = 2;
+    for (int q = 0; q < 4; q++) {
+      const int iz = q >> 1, iy = q & 1;
+      a[q] = b[q] = l[q] = r[q] = make_float2(0.0f, 0.0f);
+      if (iz < fz.n && iy < fy.n) {
+        const float* row = box + (long)d * kHBox + (fz.b[iz] * kHY + fy.b[iy]) * kHX;
+        const int t = (fz.t[iz] * nby + fy.t[iy]) * nbx;
+        const float* own = row + (long)(t + tx) * (3 * kHBox) + x4 + 2;
+        a[q] = __ldg(reinterpret_cast<const float2*>(own));
+        b[q] = __ldg(reinterpret_cast<const float2*>(own + 2));
+        if (first) l[q] = __ldg(reinterpret_cast<const float2*>(row + (long)(t + txl) * (3 * kHBox) + xl));
+        if (last) r[q] = __ldg(reinterpret_cast<const float2*>(row + (long)(t + txr) * (3 * kHBox)));
+      }
     }
-    float v[2][4];
+    // (adding the zeros of the boxes that do not hold the cell changes nothing)
+    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
 #pragma unroll
-    for (int ze = 0; ze < 2; ze++) {
-      const long zo = (ze ? zt1 : zt0) * tzs + (long)(ze ? zp1 : zp0) * (kHY * kHX);
-#pragma unroll
-      for (int q = 0; q < 4; q++) v[ze][q] = (ze < nze && pu[q]) ? __ldg(box + zo + po[q]) : 0.0f;
+    for (int q = 0; q < 4; q++) {
+      s0 = (s0 + l[q].x) + a[q].x;
+      s1 = (s1 + l[q].y) + a[q].y;
+      s2 = (s2 + b[q].x) + r[q].x;
+      s3 = (s3 + b[q].y) + r[q].y;
     }
-    float s = 0.0f;
+    T* o = f + ((long)(d * nz + tz * kTZ + z) * ny + ty * kTY + y) * nx + tx * kTX + x4;
+    if (!accumulate && sizeof(T) == 4 && ((uintptr_t)f & 15) == 0) {
+      *reinterpret_cast<float4*>(o) = make_float4(s0, s1, s2, s3);
+    } else {
+      const float s[4] = {s0, s1, s2, s3};
 #pragma unroll
-    for (int ze = 0; ze < 2; ze++)
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (ze < nze && pu[q]) s += v[ze][q];
-    T* o = dst + (long)lz * ny * nx;
-    *o = accumulate ? (T)((double)*o + (double)s) : (T)s;
+      for (int i = 0; i < 4; i++) o[i] = accumulate ? (T)((double)o[i] + (double)s[i]) : (T)s[i];
+    }
   }
 }
 
@@ -1501,33 +1500,10 @@ __device__ __forceinline__ void box_axis(int c, int n, int T, int nb, BoxAxis& L
   }
 }
 
-// The same on grids of 3 or more tiles per axis, none narrower than 4 cells
-// (so no cell lies both in the lowest 2 and the highest 2 of its tile), in
-// registers: the home tile's box, and below (cells 0, 1 of the tile: the
-// previous tile's box) or above (the last 2 cells: the next tile's box).
-__device__ __forceinline__ int box_axis2(int c, int n, int T, int nb, int& t0, int& b0, int& t1, int& b1) {
-  const int th = c / T, l = c - th * T, e = min(T, n - th * T);
-  if (l < 2) {
-    t0 = (th == 0) ? nb - 1 : th - 1;
-    b0 = c - t0 * T + 2 + ((th == 0) ? n : 0);
-    t1 = th;
-    b1 = l + 2;
-    return 2;
-  }
-  t0 = th;
-  b0 = l + 2;
-  if (l >= e - 2) {
-    t1 = (th == nb - 1) ? 0 : th + 1;
-    b1 = l - e + 2;  // the next tile starts at th T + e
-    return 2;
-  }
-  return 1;
-}
-
 // f[d][z][y][x] (=, or +=) the sum over the boxes holding the cell, in a
-// fixed order (z, y, x entries nested); boxes of empty tiles are skipped.
-// GENERAL: any grid (lists in local memory); else box_axis2's grids.
-template <typename T, bool GENERAL>
+// fixed order (z, y, x entries nested); boxes of empty tiles are skipped.  Any
+// grid.
+template <typename T>
 __global__ void __launch_bounds__(256) k_spread_fold(T* __restrict__ f, int accumulate, const float* __restrict__ box,
                                                      const int* __restrict__ live, BinSpec bs) {
   const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
@@ -1535,35 +1511,17 @@ __global__ void __launch_bounds__(256) k_spread_fold(T* __restrict__ f, int accu
   const int z = blockIdx.z % nz, d = blockIdx.z / nz;
   if (x >= nx || y >= ny) return;
   float s = 0.0f;
-  if constexpr (GENERAL) {
-    BoxAxis Lx, Ly, Lz;
-    box_axis(x, nx, bs.tile[0], bs.nb[0], Lx);
-    box_axis(y, ny, bs.tile[1], bs.nb[1], Ly);
-    box_axis(z, nz, bs.tile[2], bs.nb[2], Lz);
-    for (int iz = 0; iz < Lz.n; iz++)
-      for (int iy = 0; iy < Ly.n; iy++)
-        for (int ix = 0; ix < Lx.n; ix++) {
-          const int t = (Lz.t[iz] * bs.nb[1] + Ly.t[iy]) * bs.nb[0] + Lx.t[ix];
-          if (!live[t]) continue;
-          s += __ldg(box + ((long)t * 3 + d) * kHBox + (Lz.b[iz] * kHY + Ly.b[iy]) * kHX + Lx.b[ix]);
-        }
-  } else {
-    int tx[2], bx[2], ty[2], by[2], tz[2], bz[2];
-    const int cx = box_axis2(x, nx, kTX, bs.nb[0], tx[0], bx[0], tx[1], bx[1]);
-    const int cy = box_axis2(y, ny, kTY, bs.nb[1], ty[0], by[0], ty[1], by[1]);
-    const int cz = box_axis2(z, nz, kTZ, bs.nb[2], tz[0], bz[0], tz[1], bz[1]);
-#pragma unroll
-    for (int iz = 0; iz < 2; iz++)
-#pragma unroll
-      for (int iy = 0; iy < 2; iy++)
-#pragma unroll
-        for (int ix = 0; ix < 2; ix++) {
-          if (iz >= cz || iy >= cy || ix >= cx) continue;
-          const int t = (tz[iz] * bs.nb[1] + ty[iy]) * bs.nb[0] + tx[ix];
-          if (!live[t]) continue;
-          s += __ldg(box + ((long)t * 3 + d) * kHBox + (bz[iz] * kHY + by[iy]) * kHX + bx[ix]);
-        }
-  }
+  BoxAxis Lx, Ly, Lz;
+  box_axis(x, nx, bs.tile[0], bs.nb[0], Lx);
+  box_axis(y, ny, bs.tile[1], bs.nb[1], Ly);
+  box_axis(z, nz, bs.tile[2], bs.nb[2], Lz);
+  for (int iz = 0; iz < Lz.n; iz++)
+    for (int iy = 0; iy < Ly.n; iy++)
+      for (int ix = 0; ix < Lx.n; ix++) {
+        const int t = (Lz.t[iz] * bs.nb[1] + Ly.t[iy]) * bs.nb[0] + Lx.t[ix];
+        if (!live[t]) continue;
+        s += __ldg(box + ((long)t * 3 + d) * kHBox + (Lz.b[iz] * kHY + Ly.b[iy]) * kHX + Lx.b[ix]);
+      }
   T* dst = f + ((long)(d * nz + z) * ny + y) * nx + x;
   *dst = accumulate ? (T)((double)*dst + (double)s) : (T)s;
 }
@@ -1638,22 +1596,14 @@ cudaError_t spread_slots(T* fgrid, bool accumulate, const double* x_old, const d
       if (!ts.box || !ts.live || !rec) return cudaErrorInvalidValue;
       if (!ts.tmax || !ts.quirk) return cudaErrorInvalidValue;
       k_spread_home<<<ntiles, kHomeThreads, kHomeSmem, st>>>(tf, ts, rec);
-      bool full = true;  // every tile full: the column fold
-      for (int ax = 0; ax < 3; ax++) full &= (bs.n[ax] % bs.tile[ax] == 0);
-      if (full) {
-        k_spread_fold_cols<T><<<dim3((unsigned)ntiles, 3), kTX * kTY, 0, st>>>(fgrid, accumulate ? 1 : 0, ts.box,
-                                                                               bs);
-        count_launches(2);
-        return cudaGetLastError();
+      bool four = bs.n[0] % 4 == 0;  // no tile narrower than 4 cells, whole groups of 4 along x
+      for (int ax = 0; ax < 3; ax++) four &= bs.n[ax] >= 4 && (bs.n[ax] % bs.tile[ax] == 0 || bs.n[ax] % bs.tile[ax] >= 4);
+      if (four) {
+        k_spread_fold4<T><<<dim3((unsigned)ntiles, 3), kFoldThreads, 0, st>>>(fgrid, accumulate ? 1 : 0, ts.box, bs);
+      } else {
+        const dim3 fb(32, 8), fg((unsigned)((a.nx + 31) / 32), (unsigned)((a.ny + 7) / 8), (unsigned)(3 * a.nz));
+        k_spread_fold<T><<<fg, fb, 0, st>>>(fgrid, accumulate ? 1 : 0, ts.box, ts.live, bs);
       }
-      const dim3 fb(32, 8), fg((unsigned)((a.nx + 31) / 32), (unsigned)((a.ny + 7) / 8), (unsigned)(3 * a.nz));
-      bool regs = true;  // box_axis2 holds: 3 or more tiles per axis, none narrower than 4 cells
-      for (int ax = 0; ax < 3; ax++)
-        regs &= bs.nb[ax] >= 3 && (bs.n[ax] % bs.tile[ax] == 0 || bs.n[ax] % bs.tile[ax] >= 4);
-      if (regs)
-        k_spread_fold<T, false><<<fg, fb, 0, st>>>(fgrid, accumulate ? 1 : 0, ts.box, ts.live, bs);
-      else
-        k_spread_fold<T, true><<<fg, fb, 0, st>>>(fgrid, accumulate ? 1 : 0, ts.box, ts.live, bs);
       count_launches(2);
       return cudaGetLastError();
     }
