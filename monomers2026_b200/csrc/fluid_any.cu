@@ -374,7 +374,7 @@ cudaError_t any_plain_stage(int stage, const AnyPlan& p, const PlainBufs& b, con
   const unsigned nz3 = (unsigned)(((long)n * nh + p.z.wb - 1) / p.z.wb);
   switch (stage) {
     case kPlainForward:
-      k_xy_forward_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(DivergencePlanes{b.u, b.dx}, b.work, p.xy,
+      k_xy_forward_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(DivergencePlanes{b.u, 1.0 / b.dx}, b.work, p.xy,
                                                                              tb.wx_f, tb.wy_f);
       break;
     case kPlainPoisson:

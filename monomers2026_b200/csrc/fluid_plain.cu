@@ -21,33 +21,35 @@
 namespace selm {
 
 // ---------------------------------------------------------------- viscous step
-// u* = u + (mu*dt*lap7(u) + f)/rho   (cuda/SELM_Kernel.cu:155-195)
-__global__ void k_u2uAsterisk(const double* __restrict__ u, const double* __restrict__ f,
-                              double* __restrict__ us, double dx, double dt, double mu, double rho, int Nx,
-                              int Ny, int Nz) {
-  const long N = (long)Nx * Ny * Nz;
-  const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const long Nyx = (long)Ny * Nx;
-  const int k = (int)(n / Nyx), j = (int)(n % Nyx / Nx), i = (int)(n % Nx);
-  const long i1 = (i != Nx - 1) ? 1 : -i;
-  const long j1 = (j != Ny - 1) ? Nx : -(long)j * Nx;
-  const long k1 = (k != Nz - 1) ? Nyx : -(long)k * Nyx;
-  const long i0 = (i != 0) ? -1 : Nx - 1;
-  const long j0 = (j != 0) ? -(long)Nx : (long)(Ny - 1) * Nx;
-  const long k0 = (k != 0) ? -Nyx : (long)(Nz - 1) * Nyx;
-  const double dxsq = dx * dx;
+// u* = u + (mu*dt*lap7(u) + f)/rho   (cuda/SELM_Kernel.cu:155-195), f the
+// forcing with the spread impulses.  A thread per cell of a
+// row (block: threadIdx.x along x, blockIdx = (row, plane)), by the reciprocals
+// of dx^2 and rho: with two FP64 divisions per component and three integer ones
+// per cell the kernel was bound by them (51 us at 128^3; its 150 MB take 23).
+__global__ void __launch_bounds__(256) k_u2uAsterisk(const double* __restrict__ u, const double* __restrict__ f,
+                                                     double* __restrict__ us, double c, double irho, int Nx, int Ny,
+                                                     int Nz) {
+  const int j = blockIdx.x * blockDim.y + threadIdx.y, k = blockIdx.y;
+  if (j >= Ny) return;
+  const long Nyx = (long)Ny * Nx, N = Nyx * Nz;
+  const double* up = u + k * Nyx + (long)j * Nx;
+  const long j1 = (j != Ny - 1) ? Nx : -(long)j * Nx, j0 = (j != 0) ? -(long)Nx : (long)(Ny - 1) * Nx;
+  const long k1 = (k != Nz - 1) ? Nyx : -(long)k * Nyx, k0 = (k != 0) ? -Nyx : (long)(Nz - 1) * Nyx;
+  for (int i = threadIdx.x; i < Nx; i += blockDim.x) {
+    const int i1 = (i != Nx - 1) ? i + 1 : 0, i0 = (i != 0) ? i - 1 : Nx - 1;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    const double* ud = u + d * N;
-    const double r = ud[n];
-    const double lap = (ud[n + i1] + ud[n + i0] + ud[n + j1] + ud[n + j0] + ud[n + k1] + ud[n + k0] - 6 * r) / dxsq;
-    us[d * N + n] = r + (mu * lap * dt + f[d * N + n]) / rho;
+    for (int d = 0; d < 3; d++) {
+      const double* ud = up + d * N;
+      const long n = d * N + k * Nyx + (long)j * Nx + i;
+      const double r = ud[i];
+      const double lap = ud[i1] + ud[i0] + ud[i + j1] + ud[i + j0] + ud[i + k1] + ud[i + k0] - 6 * r;
+      us[n] = r + (c * lap + f[n]) * irho;
+    }
   }
 }
 
 // p = div(u*) with forward differences (cuda/SELM_Kernel.cu:100-116)
-__global__ void k_div(const double* __restrict__ in, double* __restrict__ out, int Nx, int Ny, int Nz, double dx) {
+__global__ void k_div(const double* __restrict__ in, double* __restrict__ out, int Nx, int Ny, int Nz, double idx) {
   const long N = (long)Nx * Ny * Nz;
   const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
@@ -59,7 +61,7 @@ __global__ void k_div(const double* __restrict__ in, double* __restrict__ out, i
   const double* a = in;
   const double* b = in + N;
   const double* c = in + 2 * N;
-  out[n] = (a[n + i1] - a[n] + b[n + j1] - b[n] + c[n + k1] - c[n]) / dx;
+  out[n] = (a[n + i1] - a[n] + b[n + j1] - b[n] + c[n + k1] - c[n]) * idx;
 }
 
 // the Poisson solve in the half spectrum (sizes of the axis passes)
@@ -77,45 +79,49 @@ __global__ void k_poisson(double2* in, int Nx, int Ny, int Nz, const double* __r
 // u = u* - (p[n] - p[n - e_d])/(dx*N) (cuda/SELM_Kernel.cu:119-152), with the
 // sums of the new components: one partial per block and component, in a fixed
 // order.  At 128^3 the separate passes read the velocity three times and wrote
-// it twice; the sums' own pass is gone.
+// it twice; the sums' own pass is gone, and the division by dx N, three a cell,
+// is a product (34 us with it; 117 MB take 18).
 constexpr int kGradThreads = 512;
 __device__ __forceinline__ double block_total(double v, double* sh) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int t = threadIdx.y * blockDim.x + threadIdx.x, w = t >> 5, nw = (blockDim.x * blockDim.y) >> 5;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[w] = v;
+  if ((t & 31) == 0) sh[w] = v;
   __syncthreads();
   double s = 0.0;
   for (int i = 0; i < nw; i++) s += sh[i];
   return s;
 }
 __global__ void __launch_bounds__(kGradThreads) k_grad_sum(const double* __restrict__ p, double* __restrict__ u, int Nx,
-                                                           int Ny, int Nz, double dx, double* __restrict__ partial) {
+                                                           int Ny, int Nz, double c, double* __restrict__ partial) {
   __shared__ double sh[kGradThreads / 32];
   const long N = (long)Nx * Ny * Nz, Nyx = (long)Ny * Nx;
+  const int rows = Ny * Nz;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (long n = (long)blockIdx.x * kGradThreads + threadIdx.x; n < N; n += (long)gridDim.x * kGradThreads) {
-    const long row = n / Nx;
-    const int i = (int)(n - row * Nx), k = (int)(row / Ny), j = (int)(row - (long)k * Ny);
-    const long o0 = (i != 0) ? -1 : Nx - 1;
+  // a row of blockDim.x lanes (threadIdx.y rows at a time)
+  for (int row = blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += gridDim.x * blockDim.y) {
+    const int k = row / Ny, j = row - k * Ny;
     const long o1 = (j != 0) ? -(long)Nx : (long)(Ny - 1) * Nx;
     const long o2 = (k != 0) ? -Nyx : (long)(Nz - 1) * Nyx;
-    const double pn = p[n];
-    const double a = u[n] - (pn - p[n + o0]) / (dx * N);
-    const double b = u[N + n] - (pn - p[n + o1]) / (dx * N);
-    const double c = u[2 * N + n] - (pn - p[n + o2]) / (dx * N);
-    u[n] = a;
-    u[N + n] = b;
-    u[2 * N + n] = c;
-    s0 += a;
-    s1 += b;
-    s2 += c;
+    for (int i = threadIdx.x; i < Nx; i += blockDim.x) {
+      const long n = (long)row * Nx + i;
+      const double pn = p[n];
+      const double a = u[n] - (pn - p[n + ((i != 0) ? -1 : Nx - 1)]) * c;
+      const double b = u[N + n] - (pn - p[n + o1]) * c;
+      const double e = u[2 * N + n] - (pn - p[n + o2]) * c;
+      u[n] = a;
+      u[N + n] = b;
+      u[2 * N + n] = e;
+      s0 += a;
+      s1 += b;
+      s2 += e;
+    }
   }
   s0 = block_total(s0, sh);
   s1 = block_total(s1, sh);
   s2 = block_total(s2, sh);
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     partial[blockIdx.x] = s0;
     partial[gridDim.x + blockIdx.x] = s1;
     partial[2 * gridDim.x + blockIdx.x] = s2;
@@ -339,8 +345,9 @@ static cudaError_t plain_stage(int stage, const PlainPlan& pp, const PlainBufs& 
 // u_new = P(u_old + (mu dt lap u_old + f)/rho) - mean.
 cudaError_t plain_ustar(const double* u_old, double* u_new, const PlainBufs& b, int nx, int ny, int nz, double dt,
                         double mu, double rho, cudaStream_t st) {
-  const long N = (long)nx * ny * nz;
-  k_u2uAsterisk<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(u_old, b.f, u_new, b.dx, dt, mu, rho, nx, ny, nz);
+  const int tx = nx <= 32 ? 32 : nx <= 64 ? 64 : 128, ty = 256 / tx;
+  k_u2uAsterisk<<<dim3((unsigned)((ny + ty - 1) / ty), (unsigned)nz), dim3(tx, ty), 0, st>>>(
+      u_old, b.f, u_new, mu * dt / (b.dx * b.dx), 1.0 / rho, nx, ny, nz);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -355,7 +362,7 @@ cudaError_t plain_project(double* u_new, const PlainPlan& pp, const PlainBufs& b
       if (e == cudaSuccess) e = plain_stage(stage, pp, b, nx, tb, st);
     if (e != cudaSuccess) return e;
   } else {
-    k_div<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(u_new, b.p, nx, ny, nz, b.dx);
+    k_div<<<(unsigned)((N + 127) / 128), 128, 0, st>>>(u_new, b.p, nx, ny, nz, 1.0 / b.dx);
     count_launches(1);
     if ((e = fft3_r2c<double>(b.p, b.work, nx, ny, nz, 1, tb, st)) != cudaSuccess) return e;
     k_poisson<<<(unsigned)((N2 + 127) / 128), 128, 0, st>>>(b.work, nx, ny, nz, b.sym, b.dx * b.dx);
@@ -363,7 +370,8 @@ cudaError_t plain_project(double* u_new, const PlainPlan& pp, const PlainBufs& b
     if ((e = fft3_c2r<double>(b.work, b.p, nx, ny, nz, 1, 1.0, tb, st)) != cudaSuccess) return e;
   }
   const unsigned parts = (unsigned)std::min<long>(kSumParts, (N + kGradThreads - 1) / kGradThreads);
-  k_grad_sum<<<parts, kGradThreads, 0, st>>>(b.p, u_new, nx, ny, nz, b.dx, partial);
+  const int tx = nx <= 32 ? 32 : nx <= 64 ? 64 : 128;
+  k_grad_sum<<<parts, dim3(tx, kGradThreads / tx), 0, st>>>(b.p, u_new, nx, ny, nz, 1.0 / (b.dx * N), partial);
   k_subtract_mean<<<dim3(parts, 3), kGradThreads, 0, st>>>(u_new, partial, (int)parts, N);
   count_launches(2);
   return cudaGetLastError();

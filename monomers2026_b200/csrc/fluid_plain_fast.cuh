@@ -149,7 +149,7 @@ template <int N> struct PlainKernels {
     constexpr long ncol = (long)N * (N / 2 + 1);
     switch (stage) {
       case kPlainForward:
-        k_xy_forward_fast<double, N, NP><<<N, P::TPB, P::smem, st>>>(DivergencePlanes{b.u, b.dx}, b.work, tb.wx_f);
+        k_xy_forward_fast<double, N, NP><<<N, P::TPB, P::smem, st>>>(DivergencePlanes{b.u, 1.0 / b.dx}, b.work, tb.wx_f);
         break;
       case kPlainPoisson:
         k_z_poisson_fast<N, N1, PB, PT>

@@ -84,20 +84,20 @@ template <typename T> struct ArrayPlanes {
 };
 struct DivergencePlanes {
   const double* __restrict__ u;
-  double dx;
+  double idx;  // 1/dx
   struct Plane {
     const double *a, *b, *c, *cn;  // the three components, the third's next plane
-    double dx;
+    double idx;
     __device__ __forceinline__ double at(int y, int x, int n) const {
       const int q = y * n + x;
       const int i1 = (x != n - 1) ? 1 : -x, j1 = (y != n - 1) ? n : -y * n;
-      return (a[q + i1] - a[q] + b[q + j1] - b[q] + cn[q] - c[q]) / dx;
+      return (a[q + i1] - a[q] + b[q + j1] - b[q] + cn[q] - c[q]) * idx;
     }
   };
   __device__ __forceinline__ Plane plane(int z, int n) const {
     const long pl = (long)n * n, N = pl * n;
     const double* c = u + 2 * N + z * pl;
-    return Plane{u + z * pl, u + N + z * pl, c, (z != n - 1) ? c + pl : u + 2 * N, dx};
+    return Plane{u + z * pl, u + N + z * pl, c, (z != n - 1) ? c + pl : u + 2 * N, idx};
   }
 };
 
