@@ -214,14 +214,16 @@ __device__ __forceinline__ void philox_normal2_mid(const Key& key, uint32_t c0, 
 // philox_normal2 to FP32 precision.  The FP64 uniforms are u = (x + 1/2) 2^-52
 // with x = o0 2^20 + (o1 >> 12).  Rounding u to FP32 costs 2^-24 absolute,
 // which near u = 1 (radius sqrt(-2 ln u) ~ sqrt(2 (1 - u))) is a large
-// relative error of the radius; so for u >= 1/2 the complement d = 1 - u is
-// built from the complemented integer bits (exact to FP32 rounding, relative)
-// and -ln u = -ln(1 - d) = 2 atanh(s), s = d / (2 - d) <= 1/3, by its odd
-// series to s^13 (the first term left out is below 5e-9 of the sum).  For
-// u < 1/2, -ln u >= ln 2 and the fast logarithm's 3-ulp error is already
-// FP32 precision.  The angle 2 pi u2 is taken as pi t with the signed
+// relative error of the radius; so for u >= 3/4 the complement 1 - u is built
+// from the complemented integer bits (exact to FP32 rounding, relative) and
+// taken as m - 1 = -(1 - u), e = 0; for smaller u = m 2^e, m in [3/4, 3/2),
+// m - 1 is exact in FP32.  Then -ln u = -(e ln 2 + 2 atanh s), s = (m - 1)/(m + 1),
+// |s| <= 1/5, by its odd series to s^9 (the first term left out is below 1e-8 of
+// the sum): one path for both, where a branch on u took the series and the fast
+// logarithm in every warp.  The angle 2 pi u2 is taken as pi t with the signed
 // t = 2 u2 (mod 2) in [-1, 1), so the fast sine and cosine see |pi t| <= pi,
-// where their absolute error is below 2^-21.4.
+// where their absolute error is below 2^-21.4 (t's bits below 2^-32 are of no
+// account beside it).
 template <typename Key>
 __device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, float& z0,
                                                    float& z1) {
@@ -230,24 +232,22 @@ __device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, 
     philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), key, o);
   else
     philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), (uint32_t)key, (uint32_t)(key >> 32), o);
-  float nl;  // -ln u1
-  if (o[0] & 0x80000000u) {
-    const float d = fmaf((float)(~o[0]), 0x1p-32f, ((float)((~o[1]) >> 12) + 0.5f) * 0x1p-52f);
-    const float s = __fdividef(d, 2.0f - d), s2 = s * s;
-    float p = 1.0f / 13.0f;
-    p = fmaf(p, s2, 1.0f / 11.0f);
-    p = fmaf(p, s2, 1.0f / 9.0f);
-    p = fmaf(p, s2, 1.0f / 7.0f);
-    p = fmaf(p, s2, 1.0f / 5.0f);
-    p = fmaf(p, s2, 1.0f / 3.0f);
-    p = fmaf(p, s2, 1.0f);
-    nl = 2.0f * s * p;
-  } else {
-    const float u = fmaf((float)o[0], 0x1p-32f, ((float)(o[1] >> 12) + 0.5f) * 0x1p-52f);
-    nl = -__logf(u);
-  }
-  const float r = sqrtf(2.0f * nl);
-  const float t = fmaf((float)(int32_t)o[2], 0x1p-31f, ((float)(o[3] >> 12) + 0.5f) * 0x1p-51f);
+  const uint32_t flip = o[0] >= 0xc0000000u ? 0xffffffffu : 0u;
+  // u, or 1 - u where u >= 3/4
+  const float q = fmaf((float)(o[0] ^ flip), 0x1p-32f, ((float)((o[1] ^ flip) >> 12) + 0.5f) * 0x1p-52f);
+  const int bits = __float_as_int(q);
+  const int e = (bits - 0x3f400000) >> 23;                  // q = m 2^e, m in [3/4, 3/2)
+  const float mm = __int_as_float(bits - (e << 23)) - 1.0f;
+  const float t1 = flip ? -q : mm, fe = flip ? 0.0f : (float)e;
+  const float s = __fdividef(t1, 2.0f + t1), s2 = s * s;
+  float p = 2.0f / 9.0f;
+  p = fmaf(p, s2, 2.0f / 7.0f);
+  p = fmaf(p, s2, 2.0f / 5.0f);
+  p = fmaf(p, s2, 2.0f / 3.0f);
+  p = fmaf(p, s2, 2.0f);
+  // -2 ln u
+  const float r = sqrtf(-2.0f * fmaf(fe, 0.693147180559945f, s * p));
+  const float t = fmaf((float)(int32_t)o[2], 0x1p-31f, 0x1p-32f);
   float sn, cs;
   __sincosf(3.14159265358979f * t, &sn, &cs);
   z0 = r * cs;

@@ -279,9 +279,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
   const int nz = p.z.n, nl = p.nl, wb = p.wb;
   C* A = reinterpret_cast<C*>(smem_raw);
   C* tw = A + nz * nl;
-  ColSym<T>* col = reinterpret_cast<ColSym<T>*>(tw + nz);
-  PlaneSym<T>* pz = reinterpret_cast<PlaneSym<T>*>(col + wb);
-  int* pos = reinterpret_cast<int*>(pz + nz);  // nz positions
+  PlaneSym<T>* pz = reinterpret_cast<PlaneSym<T>*>(tw + nz);
+  ColArrays<T> col;
+  col.dx = reinterpret_cast<C*>(pz + nz);
+  col.dy = col.dx + wb;
+  col.c = reinterpret_cast<double*>(col.dy + wb);
+  col.ij = reinterpret_cast<int*>(col.c + wb);
+  int* pos = col.ij + wb;  // nz positions
   const long plane = (long)g.ny * g.nxh, col0 = (long)blockIdx.x * wb;
   const int wn = (int)min((long)wb, plane - col0);
   for (int t = threadIdx.x; t < nz; t += blockDim.x) {
@@ -289,7 +293,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
     pos[t] = mode_pos(p.z, t);
     pz[t] = plane_sym<T>(g, t, symz);
   }
-  if (threadIdx.x < wn) col[threadIdx.x] = col_sym<T>(g, col0 + threadIdx.x, symx, symy);
+  if (threadIdx.x < wn) put_col(col, threadIdx.x, col_sym<T>(g, col0 + threadIdx.x, symx, symy));
   __syncthreads();
   z_load_forward<T>(p, work, plane, col0, wn, tw, A);
   __syncthreads();
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
     const int k = div_by(p.dwb, u), w = u - k * wb;
     if (w >= wn) continue;
     C* a = A + pos[k] * nl + w;
-    mode_update<T, true>(g, mc, nz, col[w], pz[k], k, uhat + (long)k * plane + col0 + w, (long)nz * plane, a, wb);
+    mode_update<T, true>(g, mc, nz, get_col(col, w), pz[k], k, uhat + (long)k * plane + col0 + w, (long)nz * plane, a, wb);
   }
   __syncthreads();
   z_inverse_store<T>(p, work, plane, col0, wn, tw, A);

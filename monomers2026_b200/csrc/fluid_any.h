@@ -152,7 +152,7 @@ template <typename T> bool any_plan(int n, AnyPlan* out) {
   p.z.wb = sizeof(T) == 4 ? 16 : 8;
   // (columns, twiddles, symbols of columns and planes, positions)
   auto bytes = [&](int wb) {
-    return sizeof(cpx<T>) * ((size_t)n * 3 * wb + n) + sizeof(ColSym<T>) * (size_t)wb +
+    return sizeof(cpx<T>) * ((size_t)n * 3 * wb + n) + col_bytes<T>() * (size_t)wb +
            (sizeof(PlaneSym<T>) + sizeof(int)) * (size_t)n;
   };
   while (p.z.wb > 4 && bytes(p.z.wb) > kSmBytes / (sizeof(T) == 4 ? 3 : 2) - 1024) p.z.wb /= 2;

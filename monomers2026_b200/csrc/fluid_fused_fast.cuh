@@ -36,6 +36,16 @@ __device__ __forceinline__ ColSym<T> col_sym(const ZGeom& g, long col, const dou
   s.dy = fftk::mk<cpx<T>>((T)symy[2 * s.j] * idx1, (T)symy[2 * s.j + 1] * idx1);
   return s;
 }
+template <typename T> __device__ __forceinline__ void put_col(const ColArrays<T>& A, int w, const ColSym<T>& s) {
+  A.c[w] = s.c;
+  A.dx[w] = s.dx;
+  A.dy[w] = s.dy;
+  A.ij[w] = s.i | (s.j << 16);
+}
+template <typename T> __device__ __forceinline__ ColSym<T> get_col(const ColArrays<T>& A, int w) {
+  const int ij = A.ij[w];
+  return ColSym<T>{A.c[w], A.dx[w], A.dy[w], ij & 0xffff, ij >> 16};
+}
 template <typename T>
 __device__ __forceinline__ PlaneSym<T> plane_sym(const ZGeom& g, int k, const double* __restrict__ symz) {
   const T idx1 = (T)(1.0 / g.dx);
@@ -261,7 +271,10 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   const long col0 = (long)blockIdx.x * WB;
   const long plane = g.ncol ? g.ncol : (long)g.ny * g.nxh;
   const int wn = (int)min((long)WB, plane - col0);
-  __shared__ ColSym<T> col[WB];
+  __shared__ double col_c[WB];
+  __shared__ C col_dx[WB], col_dy[WB];
+  __shared__ int col_ij[WB];
+  const ColArrays<T> col{col_c, col_dx, col_dy, col_ij};
   __shared__ PlaneSym<T> pz[N];
   __shared__ __align__(8) unsigned long long zbar;
   if constexpr (TMA) {
@@ -274,7 +287,7 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
     tw[t] = twz[t];
     pz[t] = plane_sym<T>(g, t, symz);
   }
-  if (threadIdx.x < wn) col[threadIdx.x] = col_sym<T>(g, g.c0 + col0 + threadIdx.x, symx, symy);
+  if (threadIdx.x < wn) put_col(col, threadIdx.x, col_sym<T>(g, g.c0 + col0 + threadIdx.x, symx, symy));
   __syncthreads();
   if constexpr (TMA) {
     // one thread polls (bounded) and tells the block, so that all of it goes on or stops
@@ -320,7 +333,7 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   for (int u = threadIdx.x; u < WB * N; u += blockDim.x) {
     const int w = u % WB, k = u / WB;
     if (w >= wn) continue;
-    mode_update<T, MID>(g, mc, N, col[w], pz[k], k, uhat + (long)k * plane + col0 + w, (long)N * plane,
+    mode_update<T, MID>(g, mc, N, get_col(col, w), pz[k], k, uhat + (long)k * plane + col0 + w, (long)N * plane,
                         A + dpos<N1, N2>(k) * NL + w, WB);
   }
   __syncthreads();

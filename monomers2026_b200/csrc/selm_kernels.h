@@ -92,6 +92,14 @@ template <typename T> struct ColSym {
   cpx<T> dx, dy;
   int i, j;
 };
+// those of a block's columns in shared memory, an array per field (records of
+// 32 bytes put the lanes of a warp on every eighth bank)
+template <typename T> struct ColArrays {
+  double* c;
+  cpx<T>*dx, *dy;
+  int* ij;  // i | j << 16
+};
+template <typename T> constexpr size_t col_bytes() { return sizeof(double) + 2 * sizeof(cpx<T>) + sizeof(int); }
 template <typename T> struct PlaneSym {
   double c;
   cpx<T> d;
