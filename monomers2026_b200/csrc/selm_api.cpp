@@ -979,18 +979,26 @@ void step_graphs_invalidate(selm_sim* s) {
   fused_invalidate_graphs(s);
 }
 
-// the step of the current buffers, captured and instantiated once
+// the step of the current buffers, captured and instantiated once, on a stream
+// of its own: the caller's may be one that cannot be captured (the legacy default stream)
 static int plain_capture(selm_sim* s, int q) {
   int rc = engine_side_stream(s);
   if (rc) return rc;
+  cudaStream_t cap = nullptr;
   if (!s->st3) CU(cudaStreamCreateWithFlags(&s->st3, cudaStreamNonBlocking));
   for (cudaEvent_t* e : {&s->ev_fork3, &s->ev_ustar, &s->ev_join3})
     if (!*e) CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   const unsigned long long l0 = launches_total();
-  CU(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-  rc = plain_body(s, true);
+  CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   cudaGraph_t g = nullptr;
-  const cudaError_t ec = cudaStreamEndCapture(s->st, &g);
+  cudaError_t ec = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+  if (ec == cudaSuccess) {
+    std::swap(s->st, cap);
+    rc = plain_body(s, true);
+    std::swap(s->st, cap);
+    ec = cudaStreamEndCapture(cap, &g);
+  }
+  cudaStreamDestroy(cap);
   s->pkernels[q] = launches_total() - l0;
   uncount_launches(s->pkernels[q]);  // recorded, not run
   cudaError_t ei = cudaSuccess;
@@ -1005,10 +1013,19 @@ static int plain_capture(selm_sim* s, int q) {
   return SELM_OK;
 }
 
+// the caller is recording the simulation's stream into a graph of their own
+static bool stream_is_captured(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
+}
+
 // One graph launch; launches one by one with a host force provider, per-kernel
-// timing, or the axis passes of the sizes without spectral kernels.
+// timing, a caller's own capture, or the axis passes of the sizes without
+// spectral kernels.
 static int plain_step(selm_sim* s) {
-  if (!s->cb && !s->prof && (s->plan64.fast || s->plan64.any)) {
+  if (!s->cb && !s->prof && (s->plan64.fast || s->plan64.any) && !stream_is_captured(s->st)) {
     const int q = s->cu + 2 * s->cx;
     if (!s->pexec[q]) {
       const int rc = plain_capture(s, q);
