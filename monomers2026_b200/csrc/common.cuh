@@ -42,6 +42,19 @@ template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
 }
 template <typename C> __device__ __forceinline__ C cscale(C a, decltype(C::x) s) { return cmk<C>(a.x * s, a.y * s); }
 
+// ---------------------------------------------------------------- dependent launches
+// Kernels launched by launch_next (selm_kernels.h) may start while the kernel
+// before them on the stream still runs: what they do before previous_done()
+// may not touch memory that an earlier kernel reads or writes.  The call waits
+// until that kernel has finished (so everything before it has), then lets the
+// next one start.  Every block makes it before it returns, and pointers to what
+// earlier kernels write are not __restrict__: the compiler may not move or
+// cache those reads across it.
+__device__ __forceinline__ void previous_done() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // ---------------------------------------------------------------- Philox
 __host__ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
                                                        uint32_t k0, uint32_t k1, uint32_t out[4]) {

@@ -29,7 +29,7 @@ template <typename T> __device__ __forceinline__ PlaneSmem<T> plane_smem(const P
 // load(row, x): the plane's real values
 template <typename T, typename LD>
 __device__ __forceinline__ void xy_forward_any(const PlaneGeom& g, const cpx<T>* __restrict__ twx,
-                                               const cpx<T>* __restrict__ twy, cpx<T>* __restrict__ dst,
+                                               const cpx<T>* __restrict__ twy, cpx<T>* dst,
                                                unsigned char* raw, LD&& load) {
   using C = cpx<T>;
   const PlaneSmem<T> s = plane_smem<T>(g, raw);
@@ -39,6 +39,7 @@ __device__ __forceinline__ void xy_forward_any(const PlaneGeom& g, const cpx<T>*
     s.posx[t] = mode_pos(g.x, t);
   }
   for (int t = threadIdx.x; t < ny; t += blockDim.x) s.twy[t] = twy[t];
+  previous_done();
   for (int y0 = 0; y0 < g.hp; y0 += rp) {
     __syncthreads();
     for (int idx = threadIdx.x; idx < rp * nx; idx += blockDim.x) {
@@ -88,8 +89,8 @@ __device__ __forceinline__ void xy_forward_any(const PlaneGeom& g, const cpx<T>*
 // y inverse FFT and x c2r of one plane
 template <typename T>
 __device__ __forceinline__ void xy_inverse_any(const PlaneGeom& g, const cpx<T>* __restrict__ twx,
-                                               const cpx<T>* __restrict__ twy, const cpx<T>* __restrict__ src,
-                                               T* __restrict__ dst, unsigned char* raw) {
+                                               const cpx<T>* __restrict__ twy, const cpx<T>* src,
+                                               T* dst, unsigned char* raw) {
   using C = cpx<T>;
   const PlaneSmem<T> s = plane_smem<T>(g, raw);
   const int nx = g.x.n, ny = g.y.n, nh = g.nh, rp = g.rp, rpp = rp + 1;
@@ -98,6 +99,7 @@ __device__ __forceinline__ void xy_inverse_any(const PlaneGeom& g, const cpx<T>*
     s.twy[t] = twy[t];
     s.posy[t] = mode_pos(g.y, t);
   }
+  previous_done();
   __syncthreads();
   // the first y pass, straight from global memory: thread (m, n2), m fastest
   with_radix(g.y.r[0], [&](auto rc) {
@@ -181,7 +183,7 @@ __device__ __forceinline__ void xy_inverse_any(const PlaneGeom& g, const cpx<T>*
 }
 
 template <typename T, typename In>
-__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_forward_any(In in, cpx<T>* __restrict__ out, PlaneGeom g,
+__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_forward_any(In in, cpx<T>* out, PlaneGeom g,
                                                                          const cpx<T>* __restrict__ twx,
                                                                          const cpx<T>* __restrict__ twy) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -191,14 +193,14 @@ __global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_forward_any(In in
 }
 
 template <typename T>
-__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_inverse_any(const cpx<T>* __restrict__ in, T* __restrict__ out,
+__global__ void __launch_bounds__(plane_threads_max<T>()) k_xy_inverse_any(const cpx<T>* in, T* out,
                                                                          PlaneGeom g, const cpx<T>* __restrict__ twx,
                                                                          const cpx<T>* __restrict__ twy,
                                                                          uint64_t* step) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;  // as k_xy_inverse_fast
   const long plane = blockIdx.x;
   xy_inverse_any<T>(g, twx, twy, in + plane * g.y.n * g.nh, out + plane * g.x.n * g.y.n, smem_raw);
+  if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;  // as k_xy_inverse_fast
 }
 
 // ---------------------------------------------------------------- z pencils
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
 
 // ---------------------------------------------------------------- the reference-structured form's z passes (FP64)
 // z FFT, Poisson solve and inverse z FFT of one component
-__global__ void __launch_bounds__(256, 2) k_z_poisson_any(double2* __restrict__ work, int nh, PencilGeom p,
+__global__ void __launch_bounds__(256, 2) k_z_poisson_any(double2* work, int nh, PencilGeom p,
                                                           const double2* __restrict__ twz,
                                                           const double* __restrict__ sym, double dxsq) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(256, 2) k_z_poisson_any(double2* __restrict__ 
     tw[t] = twz[t];
     pos[t] = mode_pos(p.z, t);
   }
+  previous_done();
   __syncthreads();
   z_load_forward<double>(p, work, plane, col0, wn, tw, A);
   __syncthreads();
@@ -378,22 +381,22 @@ cudaError_t any_plain_stage(int stage, const AnyPlan& p, const PlainBufs& b, con
   const unsigned nz3 = (unsigned)(((long)n * nh + p.z.wb - 1) / p.z.wb);
   switch (stage) {
     case kPlainForward:
-      k_xy_forward_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(DivergencePlanes{b.u, 1.0 / b.dx}, b.work, p.xy,
-                                                                             tb.wx_f, tb.wy_f);
+      launch_next(k_xy_forward_any<double, DivergencePlanes>, (unsigned)n, p.threads_xy, p.smem_xy, st,
+                  DivergencePlanes{b.u, 1.0 / b.dx}, b.work, p.xy, tb.wx_f, tb.wy_f);
       break;
     case kPlainPoisson:
-      k_z_poisson_any<<<nz1, 256, p.smem_z, st>>>(b.work, nh, one, tb.wz_f, b.sym, b.dx * b.dx);
+      launch_next(k_z_poisson_any, nz1, 256, p.smem_z, st, b.work, nh, one, tb.wz_f, b.sym, b.dx * b.dx);
       break;
     case kPlainInverse:
-      k_xy_inverse_any<double><<<(unsigned)n, p.threads_xy, p.smem_xy, st>>>(b.work, b.p, p.xy, tb.wx_f, tb.wy_f,
-                                                                             nullptr);
+      launch_next(k_xy_inverse_any<double>, (unsigned)n, p.threads_xy, p.smem_xy, st, b.work, b.p, p.xy,
+                  tb.wx_f, tb.wy_f, nullptr);
       break;
     case kPlainNoise:
       k_z_noise_any<<<nz3, 256, p.smem_z, st>>>(b.nwork, nh, p.z, tb.wz_f, b.sym, b.noise);
       break;
     default:
-      k_xy_inverse_any<double><<<(unsigned)(3 * n), p.threads_xy, p.smem_xy, st>>>(b.nwork, b.f, p.xy, tb.wx_f,
-                                                                                   tb.wy_f, (uint64_t*)b.noise.step);
+      launch_next(k_xy_inverse_any<double>, (unsigned)(3 * n), p.threads_xy, p.smem_xy, st, b.nwork, b.f,
+                  p.xy, tb.wx_f, tb.wy_f, (uint64_t*)b.noise.step);
   }
   count_launches(1);
   return cudaGetLastError();

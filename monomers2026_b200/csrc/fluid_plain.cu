@@ -26,10 +26,10 @@ namespace selm {
 // row (block: threadIdx.x along x, blockIdx = (row, plane)), by the reciprocals
 // of dx^2 and rho: with two FP64 divisions per component and three integer ones
 // per cell the kernel was bound by them (51 us at 128^3; its 150 MB take 23).
-__global__ void __launch_bounds__(256) k_u2uAsterisk(const double* __restrict__ u, const double* __restrict__ f,
-                                                     double* __restrict__ us, double c, double irho, int Nx, int Ny,
+__global__ void __launch_bounds__(256) k_u2uAsterisk(const double* u, const double* f, double* us, double c, double irho, int Nx, int Ny,
                                                      int Nz) {
   const int j = blockIdx.x * blockDim.y + threadIdx.y, k = blockIdx.y;
+  previous_done();
   if (j >= Ny) return;
   const long Nyx = (long)Ny * Nx, N = Nyx * Nz;
   const double* up = u + k * Nyx + (long)j * Nx;
@@ -93,11 +93,12 @@ __device__ __forceinline__ double block_total(double v, double* sh) {
   for (int i = 0; i < nw; i++) s += sh[i];
   return s;
 }
-__global__ void __launch_bounds__(kGradThreads) k_grad_sum(const double* __restrict__ p, double* __restrict__ u, int Nx,
-                                                           int Ny, int Nz, double c, double* __restrict__ partial) {
+__global__ void __launch_bounds__(kGradThreads) k_grad_sum(const double* p, double* u, int Nx,
+                                                           int Ny, int Nz, double c, double* partial) {
   __shared__ double sh[kGradThreads / 32];
   const long N = (long)Nx * Ny * Nz, Nyx = (long)Ny * Nx;
   const int rows = Ny * Nz;
+  previous_done();
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
   // a row of blockDim.x lanes (threadIdx.y rows at a time)
   for (int row = blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += gridDim.x * blockDim.y) {
@@ -130,10 +131,10 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_sum(const double* __restr
 
 // u -= sum/N (cuda/SELM_Kernel.cu:197-207); every block adds the partials of
 // its component itself, in the same order
-__global__ void __launch_bounds__(kGradThreads) k_subtract_mean(double* __restrict__ u,
-                                                                const double* __restrict__ partial, int nparts, long N) {
+__global__ void __launch_bounds__(kGradThreads) k_subtract_mean(double* u, const double* partial, int nparts, long N) {
   __shared__ double sh[kGradThreads / 32];
   const int d = blockIdx.y;
+  previous_done();
   double s = 0.0;
   for (int i = threadIdx.x; i < nparts; i += kGradThreads) s += partial[d * nparts + i];
   const double mean = block_total(s, sh) / N;
@@ -346,8 +347,8 @@ static cudaError_t plain_stage(int stage, const PlainPlan& pp, const PlainBufs& 
 cudaError_t plain_ustar(const double* u_old, double* u_new, const PlainBufs& b, int nx, int ny, int nz, double dt,
                         double mu, double rho, cudaStream_t st) {
   const int tx = nx <= 32 ? 32 : nx <= 64 ? 64 : 128, ty = 256 / tx;
-  k_u2uAsterisk<<<dim3((unsigned)((ny + ty - 1) / ty), (unsigned)nz), dim3(tx, ty), 0, st>>>(
-      u_old, b.f, u_new, mu * dt / (b.dx * b.dx), 1.0 / rho, nx, ny, nz);
+  launch_next(k_u2uAsterisk, dim3((unsigned)((ny + ty - 1) / ty), (unsigned)nz), dim3(tx, ty), 0, st, u_old, b.f, u_new,
+              mu * dt / (b.dx * b.dx), 1.0 / rho, nx, ny, nz);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -371,8 +372,8 @@ cudaError_t plain_project(double* u_new, const PlainPlan& pp, const PlainBufs& b
   }
   const unsigned parts = (unsigned)std::min<long>(kSumParts, (N + kGradThreads - 1) / kGradThreads);
   const int tx = nx <= 32 ? 32 : nx <= 64 ? 64 : 128;
-  k_grad_sum<<<parts, dim3(tx, kGradThreads / tx), 0, st>>>(b.p, u_new, nx, ny, nz, 1.0 / (b.dx * N), partial);
-  k_subtract_mean<<<dim3(parts, 3), kGradThreads, 0, st>>>(u_new, partial, (int)parts, N);
+  launch_next(k_grad_sum, parts, dim3(tx, kGradThreads / tx), 0, st, b.p, u_new, nx, ny, nz, 1.0 / (b.dx * N), partial);
+  launch_next(k_subtract_mean, dim3(parts, 3), kGradThreads, 0, st, u_new, partial, (int)parts, N);
   count_launches(2);
   return cudaGetLastError();
 }

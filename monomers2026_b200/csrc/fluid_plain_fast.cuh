@@ -56,7 +56,7 @@ template <int N> constexpr int poisson_columns() {
 // DFT, the division and the second factor's inverse DFT in registers, so a
 // column goes through shared memory twice
 template <int N, int N1, int WB, int TPB>
-__global__ void __launch_bounds__(TPB) k_z_poisson_fast(double2* __restrict__ work, const double2* __restrict__ twz,
+__global__ void __launch_bounds__(TPB) k_z_poisson_fast(double2* work, const double2* __restrict__ twz,
                                                         const double* __restrict__ sym, double dxsq) {
   constexpr int N2 = N / N1, NH = N / 2 + 1;
   constexpr long plane = (long)N * NH;
@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(TPB) k_z_poisson_fast(double2* __restrict__ wo
   const long col0 = (long)blockIdx.x * WB;
   const int wn = (int)min((long)WB, plane - col0);
   for (int t = threadIdx.x; t < N; t += TPB) tw[t] = twz[t];
+  previous_done();
   __syncthreads();
   for (int u = threadIdx.x; u < WB * N2; u += TPB) {
     const int l = u % WB, n2 = u / WB;
@@ -149,21 +150,23 @@ template <int N> struct PlainKernels {
     constexpr long ncol = (long)N * (N / 2 + 1);
     switch (stage) {
       case kPlainForward:
-        k_xy_forward_fast<double, N, NP><<<N, P::TPB, P::smem, st>>>(DivergencePlanes{b.u, 1.0 / b.dx}, b.work, tb.wx_f);
+        launch_next(k_xy_forward_fast<double, N, NP, DivergencePlanes>, N, P::TPB, P::smem, st,
+                    DivergencePlanes{b.u, 1.0 / b.dx}, b.work, tb.wx_f);
         break;
       case kPlainPoisson:
-        k_z_poisson_fast<N, N1, PB, PT>
-            <<<(unsigned)((ncol + PB - 1) / PB), PT, smem_p, st>>>(b.work, tb.wz_f, b.sym, b.dx * b.dx);
+        launch_next(k_z_poisson_fast<N, N1, PB, PT>, (unsigned)((ncol + PB - 1) / PB), PT, smem_p, st, b.work,
+                    tb.wz_f, b.sym, b.dx * b.dx);
         break;
       case kPlainInverse:
-        k_xy_inverse_fast<double, N, NP><<<N, P::TPB, P::smem, st>>>(b.work, b.p, tb.wx_f, nullptr);
+        launch_next(k_xy_inverse_fast<double, N, NP>, N, P::TPB, P::smem, st, b.work, b.p, tb.wx_f, nullptr);
         break;
       case kPlainNoise:
         k_z_noise_fast<N, N1, WB, ZT>
             <<<(unsigned)((ncol + WB - 1) / WB), ZT, smem_n, st>>>(b.nwork, tb.wz_f, b.sym, b.noise);
         break;
       default:
-        k_xy_inverse_fast<double, N, NP><<<3 * N, P::TPB, P::smem, st>>>(b.nwork, b.f, tb.wx_f, (uint64_t*)b.noise.step);
+        launch_next(k_xy_inverse_fast<double, N, NP>, 3 * N, P::TPB, P::smem, st, b.nwork, b.f, tb.wx_f,
+                    (uint64_t*)b.noise.step);
     }
     count_launches(1);
     return cudaGetLastError();

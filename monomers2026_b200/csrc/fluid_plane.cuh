@@ -75,7 +75,7 @@ template <int R, int S, typename C> __device__ __forceinline__ void twiddle_row(
 // What the forward kernel transforms: the planes of an array, or the
 // divergence of a velocity (forward differences, cuda/SELM_Kernel.cu:100-116).
 template <typename T> struct ArrayPlanes {
-  const T* __restrict__ in;
+  const T* in;
   struct Plane {
     const T* src;
     __device__ __forceinline__ T at(int y, int x, int n) const { return src[y * n + x]; }
@@ -83,7 +83,7 @@ template <typename T> struct ArrayPlanes {
   __device__ __forceinline__ Plane plane(int p, int n) const { return Plane{in + (long)p * (n * n)}; }
 };
 struct DivergencePlanes {
-  const double* __restrict__ u;
+  const double* u;
   double idx;  // 1/dx
   struct Plane {
     const double *a, *b, *c, *cn;  // the three components, the third's next plane
@@ -103,7 +103,7 @@ struct DivergencePlanes {
 
 template <typename T, int N, int N1, typename In>
 __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1>::NB)
-    k_xy_forward_fast(In in, cpx<T>* __restrict__ out, const cpx<T>* __restrict__ twx) {
+    k_xy_forward_fast(In in, cpx<T>* out, const cpx<T>* __restrict__ twx) {
   using C = cpx<T>;
   using S = PlaneShape<T, N, N1>;
   constexpr int N2 = S::N2, NH = S::NH, HP = S::HP, G = S::GF, PW = S::PW;
@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1
   const auto src = in.plane(blockIdx.x, N);
   C* dst = out + (long)blockIdx.x * (N * NH);
   for (int t = threadIdx.x; t < N; t += S::TPB) tw[t] = twx[t];
+  previous_done();
   __syncthreads();
   // x, first factor: thread (row pair, n2), n2 fastest (runs of N2 values of a row)
   for (int u = threadIdx.x; u < HP * N2; u += S::TPB) {
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1
 
 template <typename T, int N, int N1>
 __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1>::NB)
-    k_xy_inverse_fast(const cpx<T>* __restrict__ in, T* __restrict__ out, const cpx<T>* __restrict__ twx,
+    k_xy_inverse_fast(const cpx<T>* in, T* out, const cpx<T>* __restrict__ twx,
                       uint64_t* step) {
   using C = cpx<T>;
   using S = PlaneShape<T, N, N1>;
@@ -229,10 +230,11 @@ __global__ void __launch_bounds__(PlaneShape<T, N, N1>::TPB, PlaneShape<T, N, N1
   C* tw = P + HP * PW;
   const C* src = in + (long)blockIdx.x * (N * NH);
   T* dst = out + (long)blockIdx.x * (N * N);
+  for (int t = threadIdx.x; t < N; t += S::TPB) tw[t] = twx[t];
+  previous_done();
   // the last kernel of the step's fluid solve advances the device step counter
   // (the step's noise has been drawn; nothing later in the step reads it)
   if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
-  for (int t = threadIdx.x; t < N; t += S::TPB) tw[t] = twx[t];
   __syncthreads();
   auto slot_a = [](int m) { return (m / N1) * G + m % N1; };
   auto slot_b = [&](int m) { return m == 0 ? X0 : (2 * m == N ? X0 + 1 : slot_a(N - m)); };

@@ -929,9 +929,9 @@ static int plain_body(selm_sim* s, bool side) {
                              &s->tslots));
     prof_mark(s, "interp_update", false);
     if (forces) {
-      CU(cudaEventRecordWithFlags(s->ev_xv, s->st, cudaEventRecordExternal));  // x^{n+1} and v final
       CU(cudaEventRecord(s->ev_fork, s->st));
       CU(cudaStreamWaitEvent(s->st2, s->ev_fork, 0));
+      CU(cudaEventRecordWithFlags(s->ev_xv, s->st2, cudaEventRecordExternal));  // x^{n+1} and v final
       const int rc = engine_forces_on(s, xn, s->st2);
       if (rc) return rc;
       CU(cudaEventRecordWithFlags(s->ev_ready, s->st2, cudaEventRecordExternal));  // f too

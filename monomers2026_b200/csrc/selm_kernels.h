@@ -13,6 +13,30 @@ void count_launches(unsigned n);
 void uncount_launches(unsigned long long n);  // launches recorded into a graph capture, not run
 unsigned long long launches_total();
 
+// Launch that may start while the kernel before it on the stream still runs (a
+// programmatic dependency, also in a captured graph), for kernels that call
+// previous_done() (common.cuh): scheduling and the tables of a kernel's
+// prologue come off the chain.  The plain form's fluid kernels, which follow
+// one another with nothing between: 32^3 step 37.4 -> 33.9 us, solve alone at
+// 128^3 128.4 -> 118.8, its step 332.6 -> 331.  The spectral form's are launched
+// one after the other: the blocks that wait hold what other members' (or the side
+// stream's) kernels could use, 32 members at 48^3 959 -> 973 us a step, and the
+// FP32 step at 64^3 45.0 -> 53.7.
+template <typename... P, typename... A>
+cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 constexpr int kSumParts = 592;  // at most so many partial sums (4 blocks of 512 threads per SM)
 
 // Twiddle tables of the three axes, forward (sign -1) and backward (+1).
