@@ -300,10 +300,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_z_update_any(cp
   z_load_forward<T>(p, work, plane, col0, wn, tw, A);
   __syncthreads();
   const ModeConsts<T> mc = mode_consts<T>(g, nz);
+  const ModeOrder order = mode_order((int)col0, wn, g.nx, g.nxh);
 #pragma unroll 1
-  for (int u = threadIdx.x; u < wb * nz; u += blockDim.x) {
-    const int k = div_by(p.dwb, u), w = u - k * wb;
-    if (w >= wn) continue;
+  for (int u = threadIdx.x; u < wn * nz; u += blockDim.x) {
+    int w, k;
+    mode_unit(order, nz, u, w, k);
     C* a = A + pos[k] * nl + w;
     mode_update<T, true>(g, mc, nz, get_col(col, w), pz[k], k, uhat + (long)k * plane + col0 + w, (long)nz * plane, a, wb);
   }
