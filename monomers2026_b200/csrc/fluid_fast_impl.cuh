@@ -47,7 +47,8 @@ template <int N> constexpr int plane_balanced() {
 // tensor copies need: kTma).  The sizes that are not tuned take the multiple
 // of 4 (32-byte runs) up to 24 (FP32) or 12 (FP64) with the least of: columns
 // on the fullest SM, as iterations of the update over the SM's threads, plus
-// half an iteration of latency for each of a block's, in every wave.
+// half an iteration of latency for each of a block's, in every wave; from 8
+// columns on where those fill the chip once (192^3 FP32: 201 us with the model's 4, 183).
 template <typename T, int N> struct ZShape {
   static constexpr bool kTuned = tuned_size<T, N>();
   static constexpr bool kWide = sizeof(T) == 4 && N == kZTmaSize;
@@ -57,9 +58,10 @@ template <typename T, int N> struct ZShape {
   static constexpr int columns() {
     if (kTuned) return sizeof(T) == 8 ? 8 : (kWide ? kZTmaColumns : 16);
     constexpr long ncol = (long)N * (N / 2 + 1);
-    int best = 4;
+    constexpr int least = ncol >= 8L * 148 * MINB ? 8 : 4;
+    int best = least;
     long cost = -1;
-    for (int wb = 4; wb <= (sizeof(T) == 4 ? 24 : 12); wb += 4) {
+    for (int wb = least; wb <= (sizeof(T) == 4 ? 24 : 12); wb += 4) {
       const long smem = (long)sizeof(cpx<T>) * (3L * N * wb + N) + 1024;
       if (MINB * smem > 228 * 1024) break;
       const long blocks = (ncol + wb - 1) / wb, waves = (blocks + 148 * MINB - 1) / (148 * MINB);
