@@ -15,7 +15,10 @@
 // Everything is in place, one buffer, with the passes' indices worked out by
 // multiplication (FastDiv).  Against the Stockham stages of common.cuh
 // (radix 2-7 by run-time loops over local arrays, two buffers, an integer
-// division or two per point): see the kernels of fluid_any.cuh.
+// division or two per point): the FP32 step at 100^3 637 -> 200 us, at 192^3
+// 2976 -> 763.  The same size at compile time is 1.3 to 2 times faster (128^3
+// plane kernels 49 us here against 25, twice the instructions): what has such
+// kernels takes them.
 #pragma once
 #include "common.cuh"
 #include "fft_fast.cuh"

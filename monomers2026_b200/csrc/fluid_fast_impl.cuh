@@ -42,9 +42,12 @@ template <int N> constexpr int plane_balanced() {
 // per SM (register bound).
 // The 128^3 FP32 kernel takes 20 columns in blocks held to three per SM's
 // registers: its 416 blocks then all fit at once, where 16 columns left a
-// second wave of 76 blocks (measured 64 us against 78 with 19 columns; 20
-// makes the block's columns a whole number of 16-byte units, which its
-// tensor copies need: kTma).  The sizes that are not tuned take the multiple
+// second wave of 76 blocks (measured, when the kernel took 64 us, against 78
+// with 19 columns; 47.6 us now, bound by issue and dependent arithmetic, its 102
+// MB take 16; 20 makes the block's columns a whole number of 16-byte units,
+// which its tensor copies need: kTma).  FP64 at 128^3, 83 us for 204 MB that
+// take 31, has the same bound with two blocks of 128 registers a thread: 10
+// columns (three waves instead of four) measured 82.5.  The sizes that are not tuned take the multiple
 // of 4 (32-byte runs) up to 24 (FP32) or 12 (FP64) with the least of: columns
 // on the fullest SM, as iterations of the update over the SM's threads, plus
 // half an iteration of latency for each of a block's, in every wave; from 8

@@ -396,7 +396,7 @@ struct FusedState {
   bool ready_node[2] = {false, false};
   bool body_ready = false;  // set by the step body just issued
   bool fast = false;  // compile-time four-step kernels for this grid size
-  bool any = false;   // run-time factor kernels (fluid_any.cuh), where not fast
+  bool any = false;   // run-time factor kernels (fluid_any.cu), where not fast
   AnyPlan aplan{};
   // tuning knobs (SELM_TUNE_*): four-step split, blocks per SM of the z kernel
   int tune_split = 0;

@@ -26,8 +26,8 @@ namespace selm {
 // row (block: threadIdx.x along x, blockIdx = (row, plane)), by the reciprocals
 // of dx^2 and rho: with two FP64 divisions per component and three integer ones
 // per cell the kernel was bound by them (51 us at 128^3; its 150 MB take 23).
-__global__ void __launch_bounds__(256) k_u2uAsterisk(const double* u, const double* f, double* us, double c, double irho, int Nx, int Ny,
-                                                     int Nz) {
+__global__ void __launch_bounds__(256) k_u2uAsterisk(const double* u, const double* f, double* us, double c, double irho,
+                                                     int Nx, int Ny, int Nz) {
   const int j = blockIdx.x * blockDim.y + threadIdx.y, k = blockIdx.y;
   previous_done();
   if (j >= Ny) return;

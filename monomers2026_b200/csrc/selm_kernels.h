@@ -20,8 +20,8 @@ unsigned long long launches_total();
 // one another with nothing between: 32^3 step 37.4 -> 33.9 us, solve alone at
 // 128^3 128.4 -> 118.8, its step 332.6 -> 331.  The spectral form's are launched
 // one after the other: the blocks that wait hold what other members' (or the side
-// stream's) kernels could use, 32 members at 48^3 959 -> 973 us a step, and the
-// FP32 step at 64^3 45.0 -> 53.7.
+// stream's) kernels could use: 48 members at 32^3 to 96^3 959 -> 973 us a step,
+// the FP32 step at 64^3 45.0 -> 53.7.
 template <typename... P, typename... A>
 cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg{};
