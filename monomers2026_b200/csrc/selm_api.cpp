@@ -1127,17 +1127,16 @@ namespace {
 constexpr int kStageMonomers = 8192, kStageKept = 8;
 constexpr size_t kStageBytes = sizeof(double) * 9 * kStageMonomers;
 std::mutex g_stage_mu;
-std::vector<double*> g_stage_free;
-int g_stage_sims = 0;
+double* g_stage_free[kStageKept];
+int g_stage_nfree = 0, g_stage_sims = 0;
 
 struct StageBuffer {
   double* p = nullptr;
   StageBuffer() {
     {
       std::lock_guard<std::mutex> lk(g_stage_mu);
-      if (!g_stage_free.empty()) {
-        p = g_stage_free.back();
-        g_stage_free.pop_back();
+      if (g_stage_nfree > 0) {
+        p = g_stage_free[--g_stage_nfree];
         return;
       }
     }
@@ -1150,8 +1149,8 @@ struct StageBuffer {
     if (!p) return;
     {
       std::lock_guard<std::mutex> lk(g_stage_mu);
-      if (g_stage_sims > 0 && (int)g_stage_free.size() < kStageKept) {
-        g_stage_free.push_back(p);
+      if (g_stage_sims > 0 && g_stage_nfree < kStageKept) {
+        g_stage_free[g_stage_nfree++] = p;
         return;
       }
     }
@@ -1174,12 +1173,14 @@ static void stage_sim_created() {
   g_stage_sims++;
 }
 static void stage_sim_destroyed() {
-  std::vector<double*> gone;
+  double* gone[kStageKept];
+  int n = 0;
   {
     std::lock_guard<std::mutex> lk(g_stage_mu);
-    if (--g_stage_sims == 0) gone.swap(g_stage_free);
+    if (--g_stage_sims == 0)
+      while (g_stage_nfree > 0) gone[n++] = g_stage_free[--g_stage_nfree];
   }
-  for (double* p : gone) cudaFreeHost(p);
+  while (n > 0) cudaFreeHost(gone[--n]);
 }
 
 extern "C" int selm_get_particles(selm_sim* s, double* x, double* v, double* f) {
