@@ -56,12 +56,26 @@ template <typename T, int N, int N1> struct PlaneShape {
     return best;
   }
   static constexpr int NB = blocks();
-  // threads: the largest phase's units in equal rounds of at most what the registers give
+  // points that a thread of t goes through, one after another, in the four phases
+  static constexpr int chain(int t) {
+    const int units[4] = {HP * N2, HP * (N1 / 2 + 1), NH * N2, NH * N1}, points[4] = {N1, 2 * N2, N1, N2};
+    int c = 0;
+    for (int i = 0; i < 4; i++) c += (units[i] + t - 1) / t * points[i];
+    return c;
+  }
+  // threads: the largest phase's units in equal rounds of at most what the
+  // registers give; more where that shortens the chain by a quarter or more
+  // below that limit (a phase then needs a round less: FP64 112^3 39.4 -> 35.3
+  // us, 60^3 12.8 -> 11.2).  For less, and at the limit itself, more threads
+  // lost: FP64 128^3 37.6 -> 38.3, FP32 168^3 inverse 59.8 -> 66, 120^3 25.4 -> 28.1.
   static constexpr int threads() {
     const int cap = kThreadsPerSm / NB / 32 * 32, units = NH * (N1 > N2 ? N1 : N2);
     const int rounds = (units + cap - 1) / cap;
-    const int t = ((units + rounds - 1) / rounds + 31) / 32 * 32;
-    return t < 64 ? 64 : t;
+    const int even = ((units + rounds - 1) / rounds + 31) / 32 * 32;
+    int best = even < 64 ? 64 : even;
+    for (int t = best + 32; t < cap; t += 32)
+      if (4 * chain(t) <= 3 * chain(even) && chain(t) < chain(best)) best = t;
+    return best;
   }
   static constexpr int TPB = threads();
 };

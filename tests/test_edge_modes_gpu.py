@@ -15,7 +15,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,integrator,noise", [(6, "inertial", "exact"), (9, "inertial", "exact"),
                                                (16, "quasi_steady", "exact"), (22, "inertial", "exact"),
                                                (30, "inertial", "ref_compat"), (34, "inertial", "exact"),
-                                               (64, "inertial", "exact")])
+                                               (64, "inertial", "exact"),
+                                               # plane kernels with more threads than equal rounds need
+                                               (60, "inertial", "exact"), (84, "inertial", "ref_compat"),
+                                               (112, "inertial", "exact")])
 def test_edge_modes_match_the_oracle(oracle, n, integrator, noise, form, tol):
     wl = W.config(1, kT=1.0, grid=n, length=6, form=form)
     p = wl.params
