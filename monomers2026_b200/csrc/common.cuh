@@ -326,6 +326,44 @@ __device__ __forceinline__ void stockham_stage(const C* __restrict__ a, C* __res
   using T = decltype(C::x);
   const int L = Ls * p, r = n / L, rs = n / Ls;
   const int nbf = nlines * r * Ls;  // butterflies
+  if (p > 8) {
+    // primes 11..61, a p-point DFT: an item per output, its two twiddles one
+    // power w^(s (q r + v n/p)); bound by the shared-memory reads of the terms.
+    // A thread per butterfly, with two products and a remainder a term, was one
+    // chain of p^2 terms on few threads: the step at 34^3 282 -> 104 us FP32,
+    // 61^3 2636 -> 207 FP32, 6809 -> 233 FP64 and 2920 -> 282 plain, 122^3
+    // 11510 -> 1095 FP32 and 46070 -> 1510 FP64.
+    const int np = n / p;
+    for (int it = tid; it < nbf * p; it += nthr) {
+      const int v = it / nbf, bf = it - v * nbf;
+      int line, k, q;
+      if (line_fast) {
+        line = bf % nlines;
+        const int rest = bf / nlines;
+        k = rest % r;
+        q = rest / r;
+      } else {
+        k = bf % r;
+        const int rest = bf / r;
+        q = rest % Ls;
+        line = rest / Ls;
+      }
+      const C* y = a + line * sb + (q * rs + k) * st;
+      const int step = q * r + v * np, ys = r * st;
+      C acc = y[0];
+      int e = 0;
+#pragma unroll 4
+      for (int s = 1; s < p; s++) {
+        e += step;
+        if (e >= n) e -= n;
+        const C t = y[s * ys], z = w[e];
+        acc.x += t.x * z.x - t.y * z.y;
+        acc.y += t.x * z.y + t.y * z.x;
+      }
+      b[line * sb + ((q + v * Ls) * r + k) * st] = acc;
+    }
+    return;
+  }
   for (int it = tid; it < nbf; it += nthr) {
     int line, k, q;
     if (line_fast) {
@@ -341,21 +379,6 @@ __device__ __forceinline__ void stockham_stage(const C* __restrict__ a, C* __res
     }
     const C* ai = a + line * sb;
     C* bo = b + line * sb;
-    if (p > 8) {
-      // primes 11..61: the inputs are re-read from shared memory for each
-      // output (a p-point DFT, p^2 products, in the oracle's order)
-      const int np = n / p;
-      for (int v = 0; v < p; v++) {
-        C acc = ai[(q * rs + k) * st];
-        for (int s = 1; s < p; s++) {
-          const C y = ai[(q * rs + k + s * r) * st];
-          const C ys = (q == 0) ? y : cmul(y, w[s * q * r]);
-          acc = cadd(acc, cmul(ys, w[((s * v) % p) * np]));
-        }
-        bo[((q + v * Ls) * r + k) * st] = acc;
-      }
-      continue;
-    }
     C c[8];
 #pragma unroll 1
     for (int s = 0; s < p; s++) {
