@@ -1204,19 +1204,22 @@ extern "C" int selm_get_particles(selm_sim* s, double* x, double* v, double* f) 
     CU(cudaStreamSynchronize(cs));
     return SELM_OK;
   };
-  const double* some = x ? x : v ? v : f;
-  if (s->M <= kStageMonomers && some && pageable(some)) {
+  // each array by its own kind: what is not pageable is copied to directly
+  double* const out[3] = {x, v, f};
+  bool staged[3] = {}, any = false;
+  for (int i = 0; i < 3 && s->M <= kStageMonomers; i++) any |= staged[i] = out[i] && pageable(out[i]);
+  if (any) {
     StageBuffer sb;
     if (sb.p) {
-      double *sx = x ? sb.p : nullptr, *sv = v ? sb.p + n : nullptr, *sf = f ? sb.p + 2 * n : nullptr;
-      const int rc = copies(sx, sv, sf);
+      double* to[3];
+      for (int i = 0; i < 3; i++) to[i] = staged[i] ? sb.p + i * n : out[i];
+      const int rc = copies(to[0], to[1], to[2]);
       if (rc) {
         cudaStreamSynchronize(cs);  // nothing still writes the buffer
         return rc;
       }
-      if (x) memcpy(x, sx, b);
-      if (v) memcpy(v, sv, b);
-      if (f) memcpy(f, sf, b);
+      for (int i = 0; i < 3; i++)
+        if (staged[i]) memcpy(out[i], to[i], b);
       return SELM_OK;
     }
   }
