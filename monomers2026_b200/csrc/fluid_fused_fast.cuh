@@ -83,19 +83,6 @@ __device__ __forceinline__ void mode_unit(const ModeOrder& o, int nz, int u, int
   w = edge ? o.first + r : r + (r >= o.first ? o.edges : 0);
 }
 
-// (T)(1 / a) and sqrt(a), a > 0: FP64, or for an FP32 result an FP32
-// approximation with a Newton step in FP64 (1e-14 before the rounding to FP32)
-template <typename T> __device__ __forceinline__ T recip_of(double a) {
-  if constexpr (sizeof(T) == 8) return 1.0 / a;
-  const double q = (double)__frcp_rn((float)a);
-  return (T)fma(q, fma(-a, q, 1.0), q);
-}
-template <typename T> __device__ __forceinline__ double sqrt_of(double a) {
-  if constexpr (sizeof(T) == 8) return sqrt(a);
-  const double q = (double)rsqrtf((float)a), h = a * q;
-  return fma(fma(-h, h, a), 0.5 * q, h);
-}
-
 // reference noise draw of a half-spectrum mode (cuda/SELM_Kernel.cu:56-79).
 // The FP64 forms draw FP64 normals (same stream as the plain form) and scale
 // them in FP64 by coef = sqrt(lambda_h); the caller multiplies by the prefactor
@@ -158,7 +145,7 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
   for (int c = 0; c < 3; c++) X[c] = a[c * astep];
   const bool zero = i == 0 && j == 0 && k == 0;
   if (g.stochastic && !zero) {  // (the zero mode's draw has amplitude 0)
-    double coef = sqrt_of<T>(-Lk);
+    double coef = sqrt(-Lk);
     if (sizeof(T) == 4) coef *= g.noise_amp;
     C Xn[3];
     noise_draw_fast<T, MID>(g, mc.step, nz, i, j, k, coef, Xn);
@@ -200,7 +187,7 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
     C s = cmul(D[0], X[0]);
     s = cadd(s, cmul(D[1], X[1]));
     s = cadd(s, cmul(D[2], X[2]));
-    const T iL = recip_of<T>(Lk), imuL = -recip_of<T>(g.mu * Lk);
+    const T iL = (T)(1.0 / Lk), imuL = (T)(-1.0 / (g.mu * Lk));
     s = fftk::mk<C>(s.x * iL, s.y * iL);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -218,7 +205,7 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
     C s = cmul(D[0], us[0]);
     s = cadd(s, cmul(D[1], us[1]));
     s = cadd(s, cmul(D[2], us[2]));
-    const T iL = recip_of<T>(Lk);
+    const T iL = (T)(1.0 / Lk);
     s = fftk::mk<C>(s.x * iL, s.y * iL);
 #pragma unroll
     for (int c = 0; c < 3; c++) un[c] = csub(us[c], cmul(fftk::mk<C>(-D[c].x, D[c].y), s));
