@@ -906,9 +906,11 @@ static int plain_forcing_step(selm_sim* s) {
   return SELM_OK;
 }
 
-// The launches of one step on positions x[cx], velocity u64[cu].  side (in a
-// graph capture): the forces at the new positions and the next forcing's draw
-// run beside the spread and the fluid solve, on st2 and st3.
+// The launches of one step on positions x[cx], velocity u64[cu], up to the next
+// forcing.  side (in a graph capture): the next forcing's draw and the forces at
+// the new positions run beside the spread and the fluid solve, on st3 and st2;
+// otherwise the forces are the caller's part (plain_step), after the step's
+// state has been committed.
 static int plain_body(selm_sim* s, bool side) {
   CouplingArgs a = coupling_args(s, s->step + 1);
   a.step_ptr = s->step64;
@@ -956,14 +958,12 @@ static int plain_body(selm_sim* s, bool side) {
     CU(cudaStreamWaitEvent(s->st, s->ev_join3, 0));
     if (forces) CU(cudaStreamWaitEvent(s->st, s->ev_join, 0));
     if (forces || s->M == 0) return SELM_OK;
-  } else {
-    const int rc = plain_forcing_step(s);
-    if (rc) return rc;
+    s->cx ^= 1;  // no device force field: the forces at the new positions (zeros)
+    const int rc = engine_forces(s);
+    s->cx ^= 1;
+    return rc;
   }
-  s->cx ^= 1;  // the forces at the new positions
-  const int rc = engine_forces(s);
-  s->cx ^= 1;
-  return rc;
+  return plain_forcing_step(s);
 }
 
 static void plain_graphs_drop(selm_sim* s) {
@@ -1025,7 +1025,8 @@ static bool stream_is_captured(cudaStream_t st) {
 // timing, a caller's own capture, or the axis passes of the sizes without
 // spectral kernels.
 static int plain_step(selm_sim* s) {
-  if (!s->cb && !s->prof && (s->plan64.fast || s->plan64.any) && !stream_is_captured(s->st)) {
+  const bool graph = !s->cb && !s->prof && (s->plan64.fast || s->plan64.any) && !stream_is_captured(s->st);
+  if (graph) {
     const int q = s->cu + 2 * s->cx;
     if (!s->pexec[q]) {
       const int rc = plain_capture(s, q);
@@ -1041,7 +1042,8 @@ static int plain_step(selm_sim* s) {
   ++s->step;
   s->cu ^= 1;
   if (s->M > 0) s->cx ^= 1;
-  return SELM_OK;
+  // a host force provider sees, and an error of it leaves, the step as taken
+  return graph ? SELM_OK : engine_forces(s);
 }
 
 extern "C" int selm_initial(selm_sim* s) {
