@@ -979,9 +979,23 @@ void step_graphs_invalidate(selm_sim* s) {
   fused_invalidate_graphs(s);
 }
 
+// While it lives, the thread's calls are not bound by graph captures of others
+// (a capture in global mode, of this or another thread, forbids streams and
+// graphs being made, and ends with an error itself where they are tried).
+namespace {
+struct ApartFromCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  ApartFromCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~ApartFromCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ApartFromCaptures(const ApartFromCaptures&) = delete;
+  ApartFromCaptures& operator=(const ApartFromCaptures&) = delete;
+};
+}  // namespace
+
 // the step of the current buffers, captured and instantiated once, on a stream
 // of its own: the caller's may be one that cannot be captured (the legacy default stream)
 static int plain_capture(selm_sim* s, int q) {
+  const ApartFromCaptures apart;
   int rc = engine_side_stream(s);
   if (rc) return rc;
   cudaStream_t cap = nullptr;
