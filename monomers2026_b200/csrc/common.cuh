@@ -117,13 +117,10 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t
 //   and the square root by Newton steps from FP32 approximations; the angle's
 //   quarter turns come off exactly (4 u2 minus its nearest integer), and sine
 //   and cosine of the rest, within pi/4, are Taylor sums.
-// FULL: series to s^21 (left out: below 1e-18 of it), to a^17 and a^16 (below
-// 1e-19 and 3e-18), quotient and root corrected to FP64, ln 2 in two parts:
-// log, sqrt and sincos to about an ulp each at two thirds of their operations
-// (128^3 FP64 z kernel 96 us with the library's functions).  Otherwise to
-// about 1e-10: series to s^11, a^11 and a^12, one Newton step: what an FP32
-// result needs to be the FP64 draw rounded once.
-template <bool FULL>
+// Series to s^21 (left out: below 1e-18 of it), to a^17 and a^16 (below 1e-19 and
+// 3e-18), quotient and root corrected to FP64, ln 2 in two parts: log, sqrt and
+// sincos to about an ulp each at two thirds of their operations (128^3 FP64 z
+// kernel 96 us with the library's functions).
 __device__ __forceinline__ void box_muller(const uint32_t (&o)[4], double& z0, double& z1) {
   const double u1 = __hiloint2double((int)(0x3ff00000u | (o[0] >> 12)), (int)((o[0] << 20) | (o[1] >> 12))) -
                     (1.0 - 0x1p-53);
@@ -140,51 +137,35 @@ __device__ __forceinline__ void box_muller(const uint32_t (&o)[4], double& z0, d
   double q = (double)__frcp_rn((float)mp);
   q = fma(q, fma(-mp, q, 1.0), q);
   double s = mm * q;
-  if (FULL) s = fma(fma(-(m - (mp - 1.0)), s, fma(-mp, s, mm)), q, s);  // with the rounding of m + 1
+  s = fma(fma(-(m - (mp - 1.0)), s, fma(-mp, s, mm)), q, s);  // with the rounding of m + 1
   const double s2 = s * s;
-  double p;
-  if (FULL) {
-    p = 1.0 / 21.0;
-    p = fma(p, s2, 1.0 / 19.0);
-    p = fma(p, s2, 1.0 / 17.0);
-    p = fma(p, s2, 1.0 / 15.0);
-    p = fma(p, s2, 1.0 / 13.0);
-    p = fma(p, s2, 1.0 / 11.0);
-  } else {
-    p = 1.0 / 11.0;
-  }
+  double p = 1.0 / 21.0;
+  p = fma(p, s2, 1.0 / 19.0);
+  p = fma(p, s2, 1.0 / 17.0);
+  p = fma(p, s2, 1.0 / 15.0);
+  p = fma(p, s2, 1.0 / 13.0);
+  p = fma(p, s2, 1.0 / 11.0);
   p = fma(p, s2, 1.0 / 9.0);
   p = fma(p, s2, 1.0 / 7.0);
   p = fma(p, s2, 1.0 / 5.0);
   p = fma(p, s2, 1.0 / 3.0);
-  double y;  // -2 ln u1 > 0
-  if (FULL) {
-    // ln 2 = hi + lo, hi with 20 trailing zero bits: e hi is exact
-    constexpr double ln2hi = 0x1.62e42fefap-1, ln2lo = 0x1.cf79abc9e3b3ap-40;
-    y = -2.0 * fma((double)e, ln2hi, fma((double)e, ln2lo, 2.0 * fma(s * s2, p, s)));
-  } else {
-    y = -2.0 * fma((double)e, 0.69314718055994531, 2.0 * fma(s * s2, p, s));
-  }
+  // -2 ln u1 > 0; ln 2 = hi + lo, hi with 20 trailing zero bits: e hi is exact
+  constexpr double ln2hi = 0x1.62e42fefap-1, ln2lo = 0x1.cf79abc9e3b3ap-40;
+  const double y = -2.0 * fma((double)e, ln2hi, fma((double)e, ln2lo, 2.0 * fma(s * s2, p, s)));
   double g = (double)rsqrtf((float)y);
-  if (FULL) g = fma(g, fma(-0.5 * y * g, g, 0.5), g);
+  g = fma(g, fma(-0.5 * y * g, g, 0.5), g);
   const double h = y * g;
   const double r = fma(fma(-h, h, y), 0.5 * g, h);
   const double w = 4.0 * u2, big = w + 6755399441055744.0;  // 1.5 2^52: rounds w to an integer
   const int n = __double2loint(big);
   const double a = (w - (big - 6755399441055744.0)) * 1.5707963267948966, a2 = a * a;
-  double sn, cs;
-  if (FULL) {
-    sn = 1.0 / 355687428096000.0;
-    sn = fma(sn, a2, -1.0 / 1307674368000.0);
-    sn = fma(sn, a2, 1.0 / 6227020800.0);
-    cs = 1.0 / 20922789888000.0;
-    cs = fma(cs, a2, -1.0 / 87178291200.0);
-    cs = fma(cs, a2, 1.0 / 479001600.0);
-    sn = fma(sn, a2, -1.0 / 39916800.0);
-  } else {
-    sn = -1.0 / 39916800.0;
-    cs = 1.0 / 479001600.0;
-  }
+  double sn = 1.0 / 355687428096000.0;
+  sn = fma(sn, a2, -1.0 / 1307674368000.0);
+  sn = fma(sn, a2, 1.0 / 6227020800.0);
+  double cs = 1.0 / 20922789888000.0;
+  cs = fma(cs, a2, -1.0 / 87178291200.0);
+  cs = fma(cs, a2, 1.0 / 479001600.0);
+  sn = fma(sn, a2, -1.0 / 39916800.0);
   sn = fma(sn, a2, 1.0 / 362880.0);
   cs = fma(cs, a2, -1.0 / 3628800.0);
   sn = fma(sn, a2, -1.0 / 5040.0);
@@ -201,26 +182,16 @@ __device__ __forceinline__ void box_muller(const uint32_t (&o)[4], double& z0, d
   z1 = r * ((n & 2) ? -d : d);        // sin
 }
 
-template <bool FULL, typename Key>
-__device__ __forceinline__ void philox_normal2_of(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, double& z0,
-                                                  double& z1) {
+// Box-Muller pair from one Philox block
+template <typename Key>
+__device__ __forceinline__ void philox_normal2(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, double& z0,
+                                               double& z1) {
   uint32_t o[4];
   if constexpr (sizeof(Key) == sizeof(PhiloxKeys))
     philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), key, o);
   else
     philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), (uint32_t)key, (uint32_t)(key >> 32), o);
-  box_muller<FULL>(o, z0, z1);
-}
-// Box-Muller pair from one Philox block; to about 1e-10 (mid)
-template <typename Key>
-__device__ __forceinline__ void philox_normal2(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, double& z0,
-                                               double& z1) {
-  philox_normal2_of<true>(key, c0, c1, step, z0, z1);
-}
-template <typename Key>
-__device__ __forceinline__ void philox_normal2_mid(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, double& z0,
-                                                   double& z1) {
-  philox_normal2_of<false>(key, c0, c1, step, z0, z1);
+  box_muller(o, z0, z1);
 }
 
 // FP32 Box-Muller pair from the same Philox block, the same normals as
@@ -237,14 +208,7 @@ __device__ __forceinline__ void philox_normal2_mid(const Key& key, uint32_t c0, 
 // t = 2 u2 (mod 2) in [-1, 1), so the fast sine and cosine see |pi t| <= pi,
 // where their absolute error is below 2^-21.4 (t's bits below 2^-32 are of no
 // account beside it).
-template <typename Key>
-__device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, float& z0,
-                                                   float& z1) {
-  uint32_t o[4];
-  if constexpr (sizeof(Key) == sizeof(PhiloxKeys))
-    philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), key, o);
-  else
-    philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), (uint32_t)key, (uint32_t)(key >> 32), o);
+__device__ __forceinline__ void box_muller(const uint32_t (&o)[4], float& z0, float& z1) {
   const uint32_t flip = o[0] >= 0xc0000000u ? 0xffffffffu : 0u;
   // u, or 1 - u where u >= 3/4
   const float q = fmaf((float)(o[0] ^ flip), 0x1p-32f, ((float)((o[1] ^ flip) >> 12) + 0.5f) * 0x1p-52f);
@@ -265,6 +229,16 @@ __device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, 
   __sincosf(3.14159265358979f * t, &sn, &cs);
   z0 = r * cs;
   z1 = r * sn;
+}
+template <typename Key>
+__device__ __forceinline__ void philox_normal2_f32(const Key& key, uint32_t c0, uint32_t c1, uint64_t step, float& z0,
+                                                   float& z1) {
+  uint32_t o[4];
+  if constexpr (sizeof(Key) == sizeof(PhiloxKeys))
+    philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), key, o);
+  else
+    philox4x32_10(c0, c1, (uint32_t)step, (uint32_t)(step >> 32), (uint32_t)key, (uint32_t)(key >> 32), o);
+  box_muller(o, z0, z1);
 }
 
 // ---------------------------------------------------------------- Peskin

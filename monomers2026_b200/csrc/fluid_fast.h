@@ -14,9 +14,9 @@ namespace selm {
 // The other sizes: even with prime factors up to 7, two factors of at most 16
 // of which the plane kernels' first is even and the second at most 14 (two
 // groups of the second are held in registers), up to the largest plane that
-// fits in shared memory (224 in FP32, 160 in FP64).  FP32 normals to 1e-10:
-// measured over these sizes the velocity's error against 64 bits is then that
-// of full FP64 normals (2.1e-7), with the fast ones 2.5e-7 to 3.2e-7.
+// fits in shared memory (224 in FP32, 160 in FP64).  Their FP32 form draws FP64
+// normals: the velocity's error against 64 bits is 2.1e-7 over these sizes,
+// with the fast FP32 ones 2.5e-7 to 3.2e-7.
 #define SELM_EVEN_SIZES_64(X)                                                                                       \
   X(36) X(40) X(42) X(50) X(54) X(56) X(60) X(70) X(72) X(80) X(84) X(90) X(98) X(100) X(108) X(112) X(120) X(126) \
       X(140) X(144) X(160)

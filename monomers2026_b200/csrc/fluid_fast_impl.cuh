@@ -99,7 +99,7 @@ constexpr size_t kZSmemMax = 228 * 1024 / 3 + 1024;  // the largest capped reque
 template <typename T, int N, int N1, int NP> struct FastKernels {
   using Z = ZShape<T, N>;
   using P = PlaneShape<T, N, NP>;
-  static constexpr bool kMid = sizeof(T) == 4 && !Z::kTuned;
+  static constexpr bool kWide64 = sizeof(T) == 4 && !Z::kTuned;
 
   static cudaError_t attrs() {
     cudaError_t e;
@@ -107,11 +107,11 @@ template <typename T, int N, int N1, int NP> struct FastKernels {
       if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::smem))) return e;
     const size_t zmax = smem_z_need<T, N>() > kZSmemMax ? smem_z_need<T, N>() : kZSmemMax;
     if constexpr (Z::kTma) {
-      if ((e = cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true, kMid>,
+      if ((e = cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true, kWide64>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zmax)))
         return e;
     }
-    return cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, false, kMid>,
+    return cudaFuncSetAttribute((const void*)k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, false, kWide64>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zmax);
   }
 
@@ -128,12 +128,12 @@ template <typename T, int N, int N1, int NP> struct FastKernels {
       const size_t zs = smem_z_request(smem_z_need<T, N>(), z_blocks_per_sm);
       if constexpr (Z::kTma) {
         if (zmap) {  // the block's columns by tensor copies (the map covers work)
-          k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true, kMid><<<nb, Z::TPB, zs, st>>>(
+          k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, true, kWide64><<<nb, Z::TPB, zs, st>>>(
               b.work, b.uhat, zg, tb.wz_f, symx, symy, symz, *zmap);
           return cudaGetLastError();
         }
       }
-      k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, false, kMid><<<nb, Z::TPB, zs, st>>>(
+      k_z_update_fast<T, N, N1, Z::WB, Z::TPB, Z::MINB, false, kWide64><<<nb, Z::TPB, zs, st>>>(
           b.work, b.uhat, zg, tb.wz_f, symx, symy, symz, CUtensorMap{});
     }
     return cudaGetLastError();

@@ -91,9 +91,8 @@ __device__ __forceinline__ void mode_unit(const ModeOrder& o, int nz, int u, int
 // the whole per-mode amplitude coef = noise_amp sqrt(lambda_h) (times 1/sqrt 2
 // for a complex draw), which is formed in FP64 and rounded to FP32 once: the
 // noise-variance prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).
-// MID (FP32): the normals to 1e-10 instead (philox_normal2_mid), scaled in FP64
-// and rounded once.
-template <typename T, bool MID>
+// W64 (FP32): the FP64 normals instead, scaled in FP64 and rounded once.
+template <typename T, bool W64>
 __device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int nz, int i, int j, int k, double coef,
                                                 cpx<T> out[3]) {
   const bool selfc = (k == 0 || 2 * k == nz) && (j == 0 || 2 * j == g.ny) && (i == 0 || 2 * i == g.nx);
@@ -106,9 +105,9 @@ __device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, i
       double z0, z1;
       philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
       out[d] = make_double2(z0 * re, z1 * im);
-    } else if constexpr (MID) {
+    } else if constexpr (W64) {
       double z0, z1;
-      philox_normal2_mid(g.rk, q, (uint32_t)d, step, z0, z1);
+      philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
       out[d] = make_float2((float)(z0 * re), (float)(z1 * im));
     } else {
       float z0, z1;
@@ -131,9 +130,9 @@ template <typename T> __device__ __forceinline__ ModeConsts<T> mode_consts(const
 
 // The spectral update of mode (i, j, k), all three components: the
 // transformed forcing at a[c astep] is replaced by the new velocity over N,
-// u_hat (component c at uh[c cplane]) by the new velocity.  MID: the
-// FP32 form's normals to 1e-10 (noise_draw_fast).
-template <typename T, bool MID>
+// u_hat (component c at uh[c cplane]) by the new velocity.  W64: the
+// FP32 form draws FP64 normals (noise_draw_fast).
+template <typename T, bool W64>
 __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>& mc, int nz, const ColSym<T>& col,
                                             const PlaneSym<T>& pz, int k, cpx<T>* __restrict__ uh, long cplane,
                                             cpx<T>* a, int astep) {
@@ -148,12 +147,12 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
     double coef = sqrt(-Lk);
     if (sizeof(T) == 4) coef *= g.noise_amp;
     C Xn[3];
-    noise_draw_fast<T, MID>(g, mc.step, nz, i, j, k, coef, Xn);
+    noise_draw_fast<T, W64>(g, mc.step, nz, i, j, k, coef, Xn);
     if (i == 0 || 2 * i == g.nx) {
       const int jc = (j == 0) ? 0 : ny - j, kc = (k == 0) ? 0 : nz - k;
       if (jc != j || kc != k) {
         C Xc[3];
-        noise_draw_fast<T, MID>(g, mc.step, nz, i, jc, kc, coef, Xc);
+        noise_draw_fast<T, W64>(g, mc.step, nz, i, jc, kc, coef, Xc);
         const T s = (g.noise_mode == 1 || g.qs) ? T(0.7071067811865476) : T(0.5);
 #pragma unroll
         for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<C>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
@@ -269,7 +268,7 @@ template <int WB> __host__ __device__ __forceinline__ int z_blocks(int nxh, int 
 // TMA: the block's columns of work come into shared memory and go back by
 // tensor copies (tmap: work as [plane][component][column], 3-D, box WB x 3
 // x N), instead of the passes' own global loads and stores.
-template <typename T, int N, int N1_, int WB, int TPB, int MINB, bool TMA, bool MID>
+template <typename T, int N, int N1_, int WB, int TPB, int MINB, bool TMA, bool W64>
 __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict__ work, cpx<T>* __restrict__ uhat, ZGeom g,
                                                        const cpx<T>* __restrict__ twz,
                                                        const double* __restrict__ symx,
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(TPB, MINB) k_z_update_fast(cpx<T>* __restrict_
   for (int u = threadIdx.x; u < wn * N; u += blockDim.x) {
     int w, k;
     mode_unit(order, N, u, w, k);
-    mode_update<T, MID>(g, mc, N, get_col(col, w), pz[k], k, uhat + (long)k * plane + col0 + w, (long)N * plane,
+    mode_update<T, W64>(g, mc, N, get_col(col, w), pz[k], k, uhat + (long)k * plane + col0 + w, (long)N * plane,
                         A + dpos<N1, N2>(k) * NL + w, WB);
   }
   __syncthreads();
