@@ -13,6 +13,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "fft_fast.cuh"
 #include "selm_kernels.h"
@@ -91,29 +93,21 @@ __device__ __forceinline__ void mode_unit(const ModeOrder& o, int nz, int u, int
 // the whole per-mode amplitude coef = noise_amp sqrt(lambda_h) (times 1/sqrt 2
 // for a complex draw), which is formed in FP64 and rounded to FP32 once: the
 // noise-variance prefactor stays FP64 (cuda/SELM_Eulerian_Period.cu:141-148).
-// W64 (FP32): the FP64 normals instead, scaled in FP64 and rounded once.
-template <typename T, bool W64>
+// W: the type of the draw; FP64 in the FP32 form takes the FP64 normals, scaled
+// (and averaged, mode_update) in FP64 and rounded once.
+template <typename W>
 __device__ __forceinline__ void noise_draw_fast(const ZGeom& g, uint64_t step, int nz, int i, int j, int k, double coef,
-                                                cpx<T> out[3]) {
+                                                cpx<W> out[3]) {
   const bool selfc = (k == 0 || 2 * k == nz) && (j == 0 || 2 * j == g.ny) && (i == 0 || 2 * i == g.nx);
   const uint32_t q = (uint32_t)(((long)k * g.ny + j) * g.nxh + i);
   const double re = selfc ? coef : coef * 0.7071067811865476, im = selfc ? 0.0 : re;
-  const T ret = (T)re, imt = (T)im;
+  const W rew = (W)re, imw = (W)im;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    if constexpr (sizeof(T) == 8) {
-      double z0, z1;
-      philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
-      out[d] = make_double2(z0 * re, z1 * im);
-    } else if constexpr (W64) {
-      double z0, z1;
-      philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
-      out[d] = make_float2((float)(z0 * re), (float)(z1 * im));
-    } else {
-      float z0, z1;
-      philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
-      out[d] = make_float2(z0 * ret, z1 * imt);
-    }
+    W z0, z1;
+    if constexpr (sizeof(W) == 8) philox_normal2(g.rk, q, (uint32_t)d, step, z0, z1);
+    else philox_normal2_f32(g.rk, q, (uint32_t)d, step, z0, z1);
+    out[d] = fftk::mk<cpx<W>>(z0 * rew, z1 * imw);
   }
 }
 
@@ -146,34 +140,29 @@ __device__ __forceinline__ void mode_update(const ZGeom& g, const ModeConsts<T>&
   if (g.stochastic && !zero) {  // (the zero mode's draw has amplitude 0)
     double coef = sqrt(-Lk);
     if (sizeof(T) == 4) coef *= g.noise_amp;
-    C Xn[3];
-    noise_draw_fast<T, W64>(g, mc.step, nz, i, j, k, coef, Xn);
+    using W = typename std::conditional<W64, double, T>::type;
+    using CW = cpx<W>;
+    CW Xn[3];
+    noise_draw_fast<W>(g, mc.step, nz, i, j, k, coef, Xn);
     if (i == 0 || 2 * i == g.nx) {
       const int jc = (j == 0) ? 0 : ny - j, kc = (k == 0) ? 0 : nz - k;
       if (jc != j || kc != k) {
-        C Xc[3];
-        noise_draw_fast<T, W64>(g, mc.step, nz, i, jc, kc, coef, Xc);
-        const T s = (g.noise_mode == 1 || g.qs) ? T(0.7071067811865476) : T(0.5);
+        CW Xc[3];
+        noise_draw_fast<W>(g, mc.step, nz, i, jc, kc, coef, Xc);
+        const W s = (g.noise_mode == 1 || g.qs) ? W(0.7071067811865476) : W(0.5);
 #pragma unroll
-        for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<C>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
+        for (int c = 0; c < 3; c++) Xn[c] = fftk::mk<CW>((Xn[c].x + Xc[c].x) * s, (Xn[c].y - Xc[c].y) * s);
       } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) Xn[c].y = T(0);
+        for (int c = 0; c < 3; c++) Xn[c].y = W(0);
       }
     }
-    if constexpr (sizeof(T) == 8) {
-      const T amp = (T)g.noise_amp;
+    // FP32: the FP64 prefactor is already in the draw
+    const T amp = sizeof(T) == 8 ? (T)g.noise_amp : T(1);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        X[c].x += amp * Xn[c].x;
-        X[c].y += amp * Xn[c].y;
-      }
-    } else {  // FP32: the FP64 prefactor is already in the draw
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        X[c].x += Xn[c].x;
-        X[c].y += Xn[c].y;
-      }
+    for (int c = 0; c < 3; c++) {
+      X[c].x += amp * (T)Xn[c].x;
+      X[c].y += amp * (T)Xn[c].y;
     }
   }
   C un[3];

@@ -62,3 +62,17 @@ def test_fp32_grids_draw_fp64_normals(probe):
     want = (z[:, :2] * (LD(amp) * 2)).astype(np.float32)  # sqrt(lambda) = 2
     np.testing.assert_array_equal(got[..., 0], want)
     assert not got[..., 1].any()
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+def test_fp32_grids_average_in_fp64(probe, exact):
+    """The Hermitian average of mode (0, 0, k) with the conjugate of (0, 0, -k)
+    on those grids: of 400000 values each the nearest FP32 number (an average
+    of rounded draws is one in about half of them)."""
+    n, k, amp = 10, 3, 0.37
+    got = _mode(probe, n, k, 11, 100000, amp, exact)[:, :2]
+    (zr, zi), _ = normals(_words(probe, n, k, 11, 100000))
+    (cr, ci), _ = normals(_words(probe, n, n - k, 11, 100000))
+    scale = LD(amp) * 2 * np.sin(PI * k / n) * np.sqrt(LD(0.5)) * (np.sqrt(LD(0.5)) if exact else LD(0.5))
+    np.testing.assert_array_equal(got[..., 0], ((zr + cr) * scale)[:, :2].astype(np.float32))
+    np.testing.assert_array_equal(got[..., 1], ((zi - ci) * scale)[:, :2].astype(np.float32))
