@@ -206,8 +206,7 @@ __device__ __forceinline__ void philox_normal2(const Key& key, uint32_t c0, uint
 // the sum): one path for both, where a branch on u took the series and the fast
 // logarithm in every warp.  The angle 2 pi u2 is taken as pi t with the signed
 // t = 2 u2 (mod 2) in [-1, 1), so the fast sine and cosine see |pi t| <= pi,
-// where their absolute error is below 2^-21.4 (t's bits below 2^-32 are of no
-// account beside it).
+// where their absolute error is below 2^-21.4.
 __device__ __forceinline__ void box_muller(const uint32_t (&o)[4], float& z0, float& z1) {
   const uint32_t flip = o[0] >= 0xc0000000u ? 0xffffffffu : 0u;
   // u, or 1 - u where u >= 3/4
@@ -224,7 +223,7 @@ __device__ __forceinline__ void box_muller(const uint32_t (&o)[4], float& z0, fl
   p = fmaf(p, s2, 2.0f);
   // -2 ln u
   const float r = sqrtf(-2.0f * fmaf(fe, 0.693147180559945f, s * p));
-  const float t = fmaf((float)(int32_t)o[2], 0x1p-31f, 0x1p-32f);
+  const float t = fmaf((float)(int32_t)o[2], 0x1p-31f, ((float)(o[3] >> 12) + 0.5f) * 0x1p-51f);
   float sn, cs;
   __sincosf(3.14159265358979f * t, &sn, &cs);
   z0 = r * cs;

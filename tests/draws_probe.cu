@@ -27,6 +27,20 @@ __global__ void k_mode(ZGeom g, int n, int k, uint64_t step0, int steps, float2*
   for (int c = 0; c < 3; c++) out[3 * t + c] = uh[c];
 }
 
+__global__ void k_normals(int fp32, int n, const uint32_t* words, double* z) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const uint32_t o[4] = {words[4 * t], words[4 * t + 1], words[4 * t + 2], words[4 * t + 3]};
+  if (fp32) {
+    float a, b;
+    box_muller(o, a, b);
+    z[2 * t] = a;
+    z[2 * t + 1] = b;
+  } else {
+    box_muller(o, z[2 * t], z[2 * t + 1]);
+  }
+}
+
 // f(device copy of out) and the result back
 template <typename F> int with_output(void* out, size_t bytes, F&& f) {
   void* d = nullptr;
@@ -62,4 +76,18 @@ extern "C" int probe_mode(int n, int k, unsigned long long seed, unsigned long l
   return with_output(out, sizeof(float) * 6 * (size_t)steps, [&](void* d) {
     k_mode<<<(steps + 255) / 256, 256>>>(g, n, k, step0, steps, (float2*)d);
   });
+}
+
+// the pairs of normals of given Philox words [n][4], z [n][2]
+extern "C" int probe_normals(int fp32, int n, const uint32_t* words, double* z) {
+  uint32_t* w = nullptr;
+  cudaError_t e = cudaMalloc(&w, sizeof(uint32_t) * 4 * (size_t)n);
+  if (e != cudaSuccess) return (int)e;
+  e = cudaMemcpy(w, words, sizeof(uint32_t) * 4 * (size_t)n, cudaMemcpyHostToDevice);
+  int rc = (int)e;
+  if (e == cudaSuccess)
+    rc = with_output(z, sizeof(double) * 2 * (size_t)n,
+                     [&](void* d) { k_normals<<<(n + 255) / 256, 256>>>(fp32, n, w, (double*)d); });
+  cudaFree(w);
+  return rc;
 }

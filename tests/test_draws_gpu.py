@@ -76,3 +76,24 @@ def test_fp32_grids_average_in_fp64(probe, exact):
     scale = LD(amp) * 2 * np.sin(PI * k / n) * np.sqrt(LD(0.5)) * (np.sqrt(LD(0.5)) if exact else LD(0.5))
     np.testing.assert_array_equal(got[..., 0], ((zr + cr) * scale)[:, :2].astype(np.float32))
     np.testing.assert_array_equal(got[..., 1], ((zi - ci) * scale)[:, :2].astype(np.float32))
+
+
+def _normals(probe, fp32, words):
+    words = np.ascontiguousarray(words, np.uint32)
+    out = np.zeros((len(words), 2))
+    assert probe.probe_normals(fp32, len(words), words.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p)) == 0
+    return out
+
+
+def test_fp32_angle_takes_all_bits_of_its_uniform(probe):
+    """The angle's uniform has 52 bits, 20 of them in the fourth word: where the
+    third leaves FP32 room for them (angles below 2^-14 turns) some draws
+    change with the fourth word, to no more than the rounding of r sin."""
+    words = np.random.default_rng(3).integers(0, 2**32, (200000, 4), np.uint64).astype(np.uint32)
+    words[:, 2] >>= 14
+    z = []
+    for w3 in (0, 0xFFFFFFFF):
+        words[:, 3] = w3
+        z.append(_normals(probe, 1, words))
+    assert (z[0] != z[1]).any()
+    assert np.abs(z[0] - z[1]).max() < 9 * 2.0**-21
