@@ -97,3 +97,40 @@ def test_fp32_angle_takes_all_bits_of_its_uniform(probe):
         z.append(_normals(probe, 1, words))
     assert (z[0] != z[1]).any()
     assert np.abs(z[0] - z[1]).max() < 9 * 2.0**-21
+
+
+def _edge_words():
+    """Both sides of u1 = 3/4 (the FP32 form's switch), 1/2, 1/sqrt 2 and
+    1/(2 sqrt 2) (the FP64 form's), u1 and u2 next to 0 and 1, quarter and
+    eighth turns, and whole words of zeros and ones below them."""
+    hi = [0, 1, 2, 0x1FFFFFFF, 0x20000000, 0x3FFFFFFF, 0x40000000, 0x5A827999, 0x5A82799A, 0x5FFFFFFF, 0x60000000,
+          0x7FFFFFFF, 0x80000000, 0x9FFFFFFF, 0xA0000000, 0xB504F333, 0xB504F334, 0xBFFFFFFF, 0xC0000000, 0xDFFFFFFF,
+          0xE0000000, 0xFFFFFFFE, 0xFFFFFFFF]
+    lo = [0, 0xFFF, 0x1000, 0x80000000, 0xFFFFF000, 0xFFFFFFFF]
+    return np.stack(np.meshgrid(hi, lo, hi, lo, indexing="ij"), -1).reshape(-1, 4).astype(np.uint32)
+
+
+def _random_words(where):
+    words = np.random.default_rng(5).integers(0, 2**32, (500000, 4), np.uint64).astype(np.uint32)
+    if where == "u1 near 0":
+        words[:, 0] >>= 18
+    elif where == "u1 near 1":
+        words[:, 0] = ~(words[:, 0] >> 18)
+    elif where == "u2 near 0":
+        words[:, 2] >>= 18
+    return words
+
+
+@pytest.mark.parametrize("where", ["edges", "anywhere", "u1 near 0", "u1 near 1", "u2 near 0"])
+def test_normals_match_extended_precision(probe, where):
+    """FP64: relative error within 4 2^-52 (half an ulp from the logarithm, one
+    each from the root, the angle and the sine, half from the product).  FP32:
+    within 11 2^-23 of the radius: 2^-21.2 for the fast sine and cosine (3.5),
+    pi 2^-23 for the rounding of their argument, and 4 for the radius (its
+    fast quotient's 2 ulp, the sums, the root, the product)."""
+    words = _edge_words() if where == "edges" else _random_words(where)
+    want, r = normals(words)
+    want = np.stack(want, 1)
+    z64, z32 = (_normals(probe, fp32, words) for fp32 in (0, 1))
+    assert (np.abs(z64 - want) <= 4 * LD(2) ** -52 * np.abs(want)).all()
+    assert (np.abs(z32 - want) <= 11 * LD(2) ** -23 * r[:, None]).all()
