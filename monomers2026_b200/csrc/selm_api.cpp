@@ -36,6 +36,7 @@ unsigned long long launches_total() { return g_launches.load(); }
 extern "C" unsigned long long selm_kernel_launches(void) { return g_launches.load(); }
 
 static void stage_sim_created();
+static void stage_reserve(int M);
 static void stage_sim_destroyed();
 
 int selm_fail(int code, const std::string& msg) {
@@ -556,6 +557,7 @@ static int set_particles_host(selm_sim* s, int M, const double* x, const double*
     }
     if ((rc = alloc_slots(s, s->tiles, s->tslots, M))) return rc;
     CU(cudaMemsetAsync(s->f, 0, sizeof(double) * 3 * M, s->st));
+    stage_reserve(M);
     step_graphs_invalidate(s);
   }
   if (M == 0) return SELM_OK;
@@ -1136,41 +1138,28 @@ extern "C" int selm_destroy(selm_sim* s) {
 // for 1000 monomers, of which 48 replicas of an ensemble paid 48), while three
 // copies into one page-locked buffer are queued together and waited for once.
 // Above kStageMonomers the copy out of the buffer costs what it saves.  The
-// buffers are shared by the process' simulations: a call takes one (or makes
-// one) and gives it back, at most kStageKept are kept, and the last
-// simulation's destruction frees them.
+// buffers are shared by the process' simulations and made with the monomers of
+// the first kStageKept of them, not in a read-back (page-locking takes locks of
+// the driver and waits for work of other threads); a call takes one and gives
+// it back, one that finds none free copies directly, and the last simulation's
+// destruction frees them.
 namespace {
 constexpr int kStageMonomers = 8192, kStageKept = 8;
 constexpr size_t kStageBytes = sizeof(double) * 9 * kStageMonomers;
 std::mutex g_stage_mu;
 double* g_stage_free[kStageKept];
-int g_stage_nfree = 0, g_stage_sims = 0;
+int g_stage_nfree = 0, g_stage_made = 0, g_stage_sims = 0;
 
 struct StageBuffer {
   double* p = nullptr;
   StageBuffer() {
-    {
-      std::lock_guard<std::mutex> lk(g_stage_mu);
-      if (g_stage_nfree > 0) {
-        p = g_stage_free[--g_stage_nfree];
-        return;
-      }
-    }
-    if (cudaHostAlloc((void**)&p, kStageBytes, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (g_stage_nfree > 0) p = g_stage_free[--g_stage_nfree];
   }
   ~StageBuffer() {
     if (!p) return;
-    {
-      std::lock_guard<std::mutex> lk(g_stage_mu);
-      if (g_stage_sims > 0 && g_stage_nfree < kStageKept) {
-        g_stage_free[g_stage_nfree++] = p;
-        return;
-      }
-    }
-    cudaFreeHost(p);
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    g_stage_free[g_stage_nfree++] = p;
   }
   StageBuffer(const StageBuffer&) = delete;
   StageBuffer& operator=(const StageBuffer&) = delete;
@@ -1188,13 +1177,28 @@ static void stage_sim_created() {
   std::lock_guard<std::mutex> lk(g_stage_mu);
   g_stage_sims++;
 }
+// a buffer per simulation whose read-backs take one, up to kStageKept
+static void stage_reserve(int M) {
+  if (M > kStageMonomers) return;
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (g_stage_made >= std::min(g_stage_sims, kStageKept)) return;
+    g_stage_made++;
+  }
+  double* p = nullptr;
+  const bool ok = cudaHostAlloc((void**)&p, kStageBytes, cudaHostAllocPortable) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  if (ok) g_stage_free[g_stage_nfree++] = p;
+  else g_stage_made--;
+}
 static void stage_sim_destroyed() {
   double* gone[kStageKept];
   int n = 0;
   {
     std::lock_guard<std::mutex> lk(g_stage_mu);
     if (--g_stage_sims == 0)
-      while (g_stage_nfree > 0) gone[n++] = g_stage_free[--g_stage_nfree];
+      for (; g_stage_nfree > 0; g_stage_made--) gone[n++] = g_stage_free[--g_stage_nfree];
   }
   while (n > 0) cudaFreeHost(gone[--n]);
 }
