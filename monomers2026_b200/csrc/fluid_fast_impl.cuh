@@ -39,7 +39,9 @@ template <int N> constexpr int plane_balanced() {
 }
 
 // Shape of a z-kernel block: WB columns, TPB threads, at least MINB blocks
-// per SM (register bound).
+// per SM (register bound).  FP32: three, 80 registers a thread; left alone
+// 96^3 and 48^3 took 84, which is two blocks: nothing alone (25.0 us at 96^3), but
+// 48 members at 32^3 to 96^3, which share the SMs, 1.11 -> 1.17 ms a step.
 // The 128^3 FP32 kernel takes 20 columns in blocks held to three per SM's
 // registers: its 416 blocks then all fit at once, where 16 columns left a
 // second wave of 76 blocks (measured, when the kernel took 64 us, against 78
@@ -57,7 +59,7 @@ template <typename T, int N> struct ZShape {
   static constexpr bool kWide = sizeof(T) == 4 && N == kZTmaSize;
   static constexpr bool kTma = kWide;
   static constexpr int TPB = 256;
-  static constexpr int MINB = sizeof(T) == 8 ? 2 : (kWide || !kTuned ? 3 : 1);
+  static constexpr int MINB = sizeof(T) == 8 ? 2 : 3;
   static constexpr int columns() {
     if (kTuned) return sizeof(T) == 8 ? 8 : (kWide ? kZTmaColumns : 16);
     constexpr long ncol = (long)N * (N / 2 + 1);
