@@ -350,8 +350,6 @@ int engine_allocate_grid(selm_sim* s) {
     if ((rc = dalloc(s, &s->u64[1], 3 * N))) return rc;
     if ((rc = dalloc(s, &s->fg64, 3 * N))) return rc;
     if ((rc = dalloc(s, &s->p64, N))) return rc;
-    // half spectra: the forcing's 3 components, the pressure
-    if ((rc = dalloc(s, &s->work64, 8 * N2))) return rc;
     if ((rc = dalloc(s, &s->partial, 3 * kSumParts))) return rc;
     if ((rc = dalloc(s, &s->sym64, 2 * s->nx))) return rc;
     if ((rc = dalloc(s, &s->step64, 1))) return rc;
@@ -370,6 +368,10 @@ int engine_allocate_grid(selm_sim* s) {
         CU(any_attrs());
       }
     }
+    // half spectra: the forcing's 3 components and, where the captured step draws the
+    // next forcing beside the pressure solve, the pressure; else that one shares the space
+    s->work64_parts = (s->plan64.fast || s->plan64.any) ? 4 : 3;
+    if ((rc = dalloc(s, &s->work64, 2 * s->work64_parts * N2))) return rc;
     CU(cudaMemsetAsync(s->u64[0], 0, sizeof(double) * 3 * N, s->st));
     CU(cudaMemsetAsync(s->u64[1], 0, sizeof(double) * 3 * N, s->st));
     CU(cudaMemsetAsync(s->fg64, 0, sizeof(double) * 3 * N, s->st));
@@ -886,7 +888,7 @@ static PlainBufs plain_bufs(selm_sim* s, double* u_new) {
   b.p = s->p64;
   b.f = s->fg64;
   b.nwork = (double2*)s->work64;
-  b.work = b.nwork + 3 * s->N2;
+  b.work = s->work64_parts == 4 ? b.nwork + 3 * s->N2 : b.nwork;
   b.sym = s->sym64;
   b.dx = s->dx;
   b.noise.seed = s->prm.seed;

@@ -57,6 +57,7 @@ struct selm_sim {
   // plain-form grid (Eulerian::d_u[2], d_f, d_p, cuda/SELM_Eulerian.cuh:12-20)
   double* u64[2] = {nullptr, nullptr};
   double *fg64 = nullptr, *p64 = nullptr, *work64 = nullptr, *partial = nullptr;
+  int work64_parts = 0;         // half spectra in work64
   double* sym64 = nullptr;      // (cos - 1, sin) of 2 pi t / n
   uint64_t* step64 = nullptr;   // device step counter (the step being taken)
   selm::AnyPlan* any64 = nullptr;  // run-time factor kernels' plan, where plan64.any points at it
