@@ -430,7 +430,6 @@ template <typename T> struct MonBlock {
   int tiles[kMonMax][3][3];  // per axis: the tiles of the union stencil, -1: none (home mode: [axis][0] the home tile)
   int home[kMonMax][3];      // home mode: per axis 2 (cell in tile) + (frac < 1/2)
 };
-template <typename T> constexpr size_t mon_smem() { return sizeof(MonBlock<T>); }
 
 // tiles of one axis that the cells c0 .. c0 + 4 (wrapped) reach: up to three
 // distinct ones (a partial last tile can add a third)

@@ -591,11 +591,9 @@ static ZGeom zgeom_of(selm_sim* s, const FusedGeom& g) {
   zg.rho = g.rho;
   zg.dt = g.dt;
   zg.noise_amp = g.noise_amp;
-  zg.idx2 = 1.0 / (g.dx * g.dx);
   zg.qs = (g.integrator == SELM_INTEGRATOR_QUASI_STEADY);
   zg.stochastic = g.stochastic;
   zg.noise_mode = g.noise_mode;
-  zg.seed = g.seed;
   zg.step = g.step;
   zg.rk = philox_keys(g.seed);
   zg.err = s->err;

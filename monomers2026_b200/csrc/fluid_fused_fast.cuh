@@ -247,13 +247,9 @@ __device__ __forceinline__ void zbar_store(const CUtensorMap* map, const void* s
 }
 constexpr long kZbarPolls = 1L << 22;
 
-// Column blocks of the z kernel: block b takes the WB consecutive columns
-// b*WB .. b*WB+WB-1 of the flattened (y, x) half-spectrum plane (column
-// index j*nxh + i, also its offset within a z plane), the last block fewer.
-template <int WB> __host__ __device__ __forceinline__ int z_blocks(int nxh, int ny) {
-  return (nxh * ny + WB - 1) / WB;
-}
-
+// Block b of the z kernel takes the WB consecutive columns b*WB .. b*WB+WB-1 of
+// the flattened (y, x) half-spectrum plane (column index j*nxh + i, also its
+// offset within a z plane), the last block fewer.
 // TMA: the block's columns of work come into shared memory and go back by
 // tensor copies (tmap: work as [plane][component][column], 3-D, box WB x 3
 // x N), instead of the passes' own global loads and stores.

@@ -891,7 +891,6 @@ static PlainBufs plain_bufs(selm_sim* s, double* u_new) {
   b.work = s->work64_parts == 4 ? b.nwork + 3 * s->N2 : b.nwork;
   b.sym = s->sym64;
   b.dx = s->dx;
-  b.noise.seed = s->prm.seed;
   b.noise.rk = philox_keys(s->prm.seed);
   b.noise.step = s->step64;
   b.noise.scale = sqrt(2 * s->prm.KB * s->prm.T * s->prm.dt * s->prm.mu / s->N);  // cuda/SELM_Eulerian_Period.cu:141

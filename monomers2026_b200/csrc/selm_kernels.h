@@ -49,7 +49,6 @@ template <typename T> struct FftTables {
 // The thermal forcing's draw: amplitude per mode scale sqrt(lambda_h), the step
 // after the one the device counter holds.
 struct NoiseArgs {
-  uint64_t seed;
   PhiloxKeys rk;
   const uint64_t* step;
   double scale, dxsq;
@@ -95,12 +94,10 @@ cudaError_t fft3_c2r(cpx<T>* in, T* out, int nx, int ny, int nz, int ncomp, T sc
 struct ZGeom {
   int ny, nxh, nx;
   double dx, mu, rho, dt, noise_amp;
-  double idx2;  // 1/dx^2
   int qs;       // quasi-steady: u_hat = P (F_hat + noise) / (mu lambda_h), no state
   int stochastic, noise_mode;
-  uint64_t seed;
   const uint64_t* step;
-  PhiloxKeys rk;  // round keys of seed
+  PhiloxKeys rk;  // round keys of the seed
   // a decomposed instance's block of columns: work and uhat hold the columns
   // c0 .. c0 + ncol - 1 of the flattened (y, x) half spectrum, ncol apart
   // from one z plane to the next (ncol == 0: all ny * nxh columns)

@@ -67,11 +67,10 @@ extern "C" int probe_mode(int n, int k, unsigned long long seed, unsigned long l
   ZGeom g{};
   g.nx = g.ny = n;
   g.nxh = n / 2 + 1;
-  g.dx = g.rho = g.idx2 = 1.0;
+  g.dx = g.rho = 1.0;
   g.noise_amp = amp;
   g.stochastic = 1;
   g.noise_mode = exact;
-  g.seed = seed;
   g.rk = philox_keys(seed);
   return with_output(out, sizeof(float) * 6 * (size_t)steps, [&](void* d) {
     k_mode<<<(steps + 255) / 256, 256>>>(g, n, k, step0, steps, (float2*)d);
