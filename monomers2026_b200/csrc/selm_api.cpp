@@ -1042,7 +1042,9 @@ static bool stream_is_captured(cudaStream_t st) {
 // timing, a caller's own capture, or the axis passes of the sizes without
 // spectral kernels.
 static int plain_step(selm_sim* s) {
-  const bool graph = !s->cb && !s->prof && (s->plan64.fast || s->plan64.any) && !stream_is_captured(s->st);
+  const bool theirs = stream_is_captured(s->st);
+  if (theirs) s->recorded = true;
+  const bool graph = !s->cb && !s->prof && (s->plan64.fast || s->plan64.any) && !theirs;
   if (graph) {
     const int q = s->cu + 2 * s->cx;
     if (!s->pexec[q]) {
@@ -1051,7 +1053,7 @@ static int plain_step(selm_sim* s) {
     }
     count_launches((unsigned)s->pkernels[q]);
     CU(cudaGraphLaunch(s->pexec[q], s->st));
-    s->ready_early = s->pready[q];
+    s->ready_early = s->pready[q] && !s->recorded;
   } else {
     const int rc = plain_body(s, false);
     if (rc) return rc;

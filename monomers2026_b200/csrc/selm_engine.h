@@ -37,6 +37,7 @@ struct selm_sim {
   cudaEvent_t ev_xv = nullptr, ev_ready = nullptr;
   cudaStream_t st_copy = nullptr;
   bool ready_early = false;
+  bool recorded = false;  // the caller has recorded steps of the plain form: replays, unseen here, write it too
   std::vector<void*> allocs;       // cudaMalloc'd (freed with cudaFree)
   std::vector<void*> pool_allocs;  // from the library's stream-ordered pool (sim_alloc)
   unsigned long long dev_bytes = 0;  // device bytes allocated for this simulation
