@@ -501,6 +501,11 @@ static int set_particles_staged(selm_sim* s, int M, const double* x, const doubl
   if (!s->ev_committed) CU(cudaEventCreateWithFlags(&s->ev_committed, cudaEventDisableTiming));
   const double L = s->hi - s->lo;
   cudaStream_t cs = s->st_copy;
+  if (!s->stage_ordered) {  // the buffers come into being, zeroed, on the simulation's stream
+    CU(cudaEventRecord(s->ev_staged, s->st));
+    CU(cudaStreamWaitEvent(cs, s->ev_staged, 0));
+    s->stage_ordered = true;
+  }
   CU(cudaStreamWaitEvent(cs, s->ev_committed, 0));  // the last commit has read the staging buffers
   CU(cudaMemcpyAsync(s->xin, x, sizeof(double) * n, cudaMemcpyHostToDevice, cs));
   if (v) CU(cudaMemcpyAsync(s->vin, v, sizeof(double) * n, cudaMemcpyHostToDevice, cs));

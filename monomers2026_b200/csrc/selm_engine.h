@@ -53,6 +53,7 @@ struct selm_sim {
   double *xin = nullptr, *vin = nullptr;
   unsigned long long* stage_cnt = nullptr;   // device: bad, outside
   unsigned long long* hstage_cnt = nullptr;  // pinned host copy
+  bool stage_ordered = false;                // the copy stream has waited for their allocation
   cudaEvent_t ev_staged = nullptr;     // staged and checked (copy stream)
   cudaEvent_t ev_committed = nullptr;  // committed (simulation stream): staging free again
   // plain-form grid (Eulerian::d_u[2], d_f, d_p, cuda/SELM_Eulerian.cuh:12-20)
