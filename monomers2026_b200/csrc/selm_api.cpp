@@ -138,12 +138,25 @@ static bool fft_size_ok(int n) {
   return n == 1;
 }
 
+// cos and sin of 2 pi t / n in extended precision, the angle reduced to an
+// eighth of a turn by its integers: rounded once, the tables are the nearest
+// numbers.  (From an angle in doubles the entries were off by up to 1e-15.)
+static void unit_root(long t, long n, long double* c, long double* s) {
+  t %= n;
+  const long quarter = 4 * t / n, r = 4 * t - quarter * n;
+  const bool far = 2 * r > n;
+  const long double x = 1.570796326794896619231321691639751442L * (far ? n - r : r) / n;
+  const long double a = far ? sinl(x) : cosl(x), b = far ? cosl(x) : sinl(x);
+  *c = quarter == 0 ? a : quarter == 1 ? -b : quarter == 2 ? -a : b;
+  *s = quarter == 0 ? b : quarter == 1 ? a : quarter == 2 ? -b : -a;
+}
 template <typename C> static std::vector<C> twiddles(int n, int sign) {
   std::vector<C> w(n);
   for (int t = 0; t < n; t++) {
-    const double a = 2.0 * M_PI * (double)t / (double)n;
-    w[t].x = (decltype(C::x))cos(a);
-    w[t].y = (decltype(C::x))(sign * sin(a));
+    long double c, s;
+    unit_root(t, n, &c, &s);
+    w[t].x = (decltype(C::x))c;
+    w[t].y = (decltype(C::x))(sign * s);
   }
   return w;
 }
@@ -330,9 +343,11 @@ extern "C" int selm_slab_layout(const selm_sim* s, int* z0, int* nzl, long long*
 std::vector<double> symbol_table(int n) {
   std::vector<double> h(2 * (size_t)n);
   for (int t = 0; t < n; t++) {
-    const double sh = sin(M_PI * t / n);
-    h[2 * t] = -2.0 * sh * sh;
-    h[2 * t + 1] = sin(2.0 * M_PI * t / n);
+    long double c, sh, sn;
+    unit_root(t, 2 * n, &c, &sh);
+    unit_root(t, n, &c, &sn);
+    h[2 * t] = (double)(-2.0L * sh * sh);
+    h[2 * t + 1] = (double)sn;
   }
   return h;
 }
