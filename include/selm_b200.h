@@ -140,10 +140,13 @@ int selm_destroy(selm_sim* s);
 
 /* ---- state access (the reference's public pointers, copied) ---- */
 /* Positions, velocities and forces after the last step (any may be NULL).
- * Returns once they are in host memory.  Right after a step of a fused form
- * with the device force field, that is as soon as the step has written them:
+ * Returns once they are in host memory.  Right after a step with the device
+ * force field, in every form, that is as soon as the step has written them:
  * the rest of that step (spread and fluid solve) may still run on the device
- * (selm_synchronize waits for it); every later call is ordered after it. */
+ * (selm_synchronize waits for it, as does work queued on the simulation's
+ * stream); every later call is ordered after it.  After steps that the caller
+ * has recorded into a graph (plain form), read-backs follow everything queued
+ * on the stream. */
 int selm_get_particles(selm_sim* s, double* x, double* v, double* f);
 /* Page-lock host arrays the caller owns (e.g. LAMMPS' atom->x, atom->v,
  * atom->f after each reallocation) so that the per-step copies above run as
