@@ -45,7 +45,7 @@ template <int N> constexpr int plane_balanced() {
 // The 128^3 FP32 kernel takes 20 columns in blocks held to three per SM's
 // registers: its 416 blocks then all fit at once, where 16 columns left a
 // second wave of 76 blocks (measured, when the kernel took 64 us, against 78
-// with 19 columns; 47.6 us now, bound by issue and dependent arithmetic, its 102
+// with 19 columns; 48.0 us now, bound by issue and dependent arithmetic, its 102
 // MB take 16; 20 makes the block's columns a whole number of 16-byte units,
 // which its tensor copies need: kTma).  FP64 at 128^3, 83 us for 204 MB that
 // take 31, has the same bound with two blocks of 128 registers a thread: 10
@@ -53,7 +53,7 @@ template <int N> constexpr int plane_balanced() {
 // of 4 (32-byte runs) up to 24 (FP32) or 12 (FP64) with the least of: columns
 // on the fullest SM, as iterations of the update over the SM's threads, plus
 // half an iteration of latency for each of a block's, in every wave; from 8
-// columns on where those fill the chip once (192^3 FP32: 201 us with the model's 4, 183).
+// columns on where those fill the chip once (192^3 FP32, with shorter normals: 201 us with the model's 4, 183).
 template <typename T, int N> struct ZShape {
   static constexpr bool kTuned = tuned_size<T, N>();
   static constexpr bool kWide = sizeof(T) == 4 && N == kZTmaSize;

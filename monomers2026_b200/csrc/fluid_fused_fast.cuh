@@ -60,7 +60,8 @@ __device__ __forceinline__ PlaneSym<T> plane_sym(const ZGeom& g, int k, const do
 // and the next row's i = 0).  These modes draw twice (the Hermitian average); in
 // the columns' own order every warp of a block that holds them, a third of the
 // blocks at 128^3, went through the second draw for a few lanes: 128^3 z
-// kernel 57.8 -> 47.6 us FP32, 87.8 -> 82.9 FP64; 100^3 FP32 45.4 -> 35.3.
+// kernel 57.8 -> 47.6 us FP32, 87.8 -> 82.9 FP64; 100^3 FP32 45.4 -> 35.3 (48.0
+// and 37.8 since, with the draws' full precision).
 struct ModeOrder {
   int n, first, edges;  // columns before the edge ones, the first of those, how many
   unsigned mn, me;      // ceil(2^32 / d) of the two groups' sizes d (0: d <= 1)
